@@ -94,7 +94,7 @@ class KVCacheContext:
         self.cu_q = None              # python list of cumulative q lengths
         self.layer_offset = 0
         self.cu_q_dev = None          # int32 [B+1]: cu_q on the device (ragged caches, prefill steps)
-        self.prefill_work = {}        # work lists of the ragged prefill kernel, made when a layer needs them
+        self.prefill_work = {}        # work lists of the prefill kernels, made when a layer needs them
         self.q_lens_host = self.context_lens_host = ()
         self.n_long_rows = self.n_single_rows = 0     # sequences with several new rows / with one
 
@@ -127,6 +127,7 @@ class KVCacheContext:
         self.context_lens = torch.as_tensor(context_lens, dtype=torch.int32, device=device).contiguous()
         q = [int(x) for x in q_seq_lens]
         self.q_seq_lens = torch.as_tensor(q, dtype=torch.int32, device=device)
+        self.prefill_work = {}
         cu = [0]
         for n in q:
             cu.append(cu[-1] + n)
@@ -137,7 +138,6 @@ class KVCacheContext:
             self.q_lens_host, self.context_lens_host = q, [int(x) for x in context_lens]
             self.n_long_rows, self.n_single_rows = sum(n > 1 for n in q), sum(n == 1 for n in q)
             self.cu_q_dev = torch.tensor(cu, dtype=torch.int32).to(device)
-            self.prefill_work = {}
         # sequences without new tokens in this step (finished prompts of a chunked prefill, idle serving slots) have
         # no row of their own: one entry per sequence that has tokens
         self.last_token_index = torch.as_tensor([c - 1 for c, n in zip(cu[1:], q) if n > 0], dtype=torch.int64,
@@ -214,6 +214,135 @@ def set_paged_decode_kernel(kind: str) -> None:
     _DECODE_KERNEL = kind
 
 
+_TILE = 128              # query rows of a tile of the prefill kernel
+# Mean key tiles per query tile up to which a launch's CTAs walk over several tiles each (their loads then run under the softmax of
+# the tile before); longer tiles differ too much in length for that and get a CTA each.
+_PERSISTENT_UP_TO = 8.0
+
+
+class _PrefillPlan:
+    """What the prefill kernels need to know about a step: per query tile ``(sequence, first row of q, rows, position of the first
+    row)``, longest first, for the sequences whose keys are all new (``fresh``) and for those with cached ones (``past``); the first
+    row of every sequence in q, and in a gathered copy of all cached rows that a step with history sees. ``ok`` False: a step that
+    these kernels do not take (a sequence longer than its block table, rows that are not there)."""
+
+    def __init__(self, cache, rows: int):
+        self.key = (cache.context_lens, cache.cu_q, rows, _version(cache.context_lens))
+        lens, cu = cache.context_lens.tolist(), cache.cu_q
+        B = len(lens)
+        reach = cache.block_tables.shape[1] * cache.block_size
+        news = [cu[b + 1] - cu[b] for b in range(B)] if len(cu) == B + 1 else []
+        self.rows = cu[-1]
+        self.ok = 0 < self.rows <= rows and len(news) == B and cu[0] == 0 and all(0 <= n <= m <= reach for n, m in zip(news, lens) if n)
+        if not self.ok:
+            return
+        self.aligned = all(n == m and n % _TILE == 0 for n, m in zip(news, lens) if n)
+        tiles = {False: [], True: []}
+        gather = {False: [0], True: [0]}       # of the sequences with history / of all that have new rows
+        for b, (n, m) in enumerate(zip(news, lens)):
+            tiles[n < m] += [(b, cu[b] + r, min(_TILE, n - r), m - n + r) for r in range(0, n, _TILE)]
+            gather[False].append(gather[False][-1] + (m if 0 < n < m else 0))
+            gather[True].append(gather[True][-1] + (m if n else 0))
+        keys = lambda t: (t[3] + t[2] - 1) // _TILE + 1
+        flat, spans = [], []
+        for items in (tiles[False], tiles[True], tiles[False] + tiles[True]):
+            items = sorted(items, key=keys, reverse=True)
+            spans.append((len(flat), len(items), sum(map(keys, items)) <= _PERSISTENT_UP_TO * len(items)))
+            flat += [x for t in items for x in t]
+        at = len(flat)
+        flat += list(cu) + gather[False] + gather[True]
+        dev = torch.tensor(flat, dtype=torch.int32).to(cache.block_tables.device)
+        self.fresh, self.past, self.all = ((dev[a:a + 4 * n], n, p) for a, n, p in spans)
+        self.cu, self.past_rows, self.all_rows = (dev[at + i * (B + 1):at + (i + 1) * (B + 1)] for i in range(3))
+        self.n_past_rows, self.n_all_rows, self.longest = gather[False][-1], gather[True][-1], max(lens)
+
+
+def _prefill_plan(cache, rows: int) -> _PrefillPlan:
+    """The step's plan, shared by its layers: kept until the step's metadata are replaced."""
+    plan = cache.prefill_work.get("plan") if cache.is_prefill else None
+    if plan is None or plan.key[0] is not cache.context_lens or plan.key[1] is not cache.cu_q \
+            or plan.key[2:] != (rows, _version(cache.context_lens)):
+        plan = _PrefillPlan(cache, rows)
+        if cache.is_prefill:
+            cache.prefill_work["plan"] = plan
+    return plan
+
+
+def _version(t: torch.Tensor) -> int:
+    """Counts changes in place (tensors made in inference mode keep no count)."""
+    return 0 if t.is_inference() else t._version
+
+
+def _needs_graph(*tensors) -> bool:
+    """Whether a derivative is wanted: the kernels of this module have none."""
+    return (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)) or torch.autograd.forward_ad._current_level >= 0
+
+
+def _rows_ok(t: torch.Tensor) -> bool:
+    """``[T, heads, dim]`` whose heads lie side by side and whose rows start on 16 bytes."""
+    return (t.dtype == torch.bfloat16 and t.stride(2) == 1 and t.stride(1) == t.shape[2] and t.stride(0) % 8 == 0
+            and t.stride(0) >= t.shape[1] * t.shape[2] and t.data_ptr() % 16 == 0)
+
+
+def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
+    """Prefill attention of a step's sequences: those without history attend over their own rows of ``k`` / ``v``, the others over
+    the cache (an int8 cache, or one of other block sizes than the kernel's, through a copy of the rows they see) with weights that are not
+    rounded. None where the kernel does not take the call."""
+    T, nq, hd = q.shape
+    nkv = k.shape[1]
+    if not (q.is_cuda and q.dtype == torch.bfloat16 and hd in (64, 128) and v.shape == k.shape and k.shape[2] == hd and k.shape[0] == T
+            and T and nkv and nq % nkv == 0 and Fn.get_attention_backend() == "auto") or _needs_graph(q, k, v):
+        return None
+    plan = _prefill_plan(cache, T)
+    if not plan.ok or (plan.fresh[1] and not (_rows_ok(k) and _rows_ok(v))):
+        return None
+    kc, vc = cache.key_cache[layer], cache.value_cache[layer]
+    ksc, vsc = _layer_scales(cache, layer)
+    if plan.past[1] and (kc.dtype != (torch.bfloat16 if ksc is None else torch.int8) or not kc.is_contiguous() or not vc.is_contiguous()
+                         or plan.n_past_rows >= 1 << 31):
+        return None
+    if q.stride(2) != 1 or q.stride(1) % 8 or q.stride(0) % 8 or q.stride(1) < hd or q.stride(0) < hd or q.data_ptr() % 16:
+        q = q.contiguous()
+    lib, st, stream = _lib.get_lib(), _lib.status_word(q.device).data_ptr(), _lib.stream_ptr()
+    out = torch.empty((plan.rows, nq * hd), dtype=q.dtype, device=q.device)
+
+    def launch(work, keys, values, ld_k, ld_v, key_rows, key_row, exact):
+        rc = lib.mfb_ragged_prefill_tc(
+            q.data_ptr(), q.stride(0), q.stride(1), keys, values, ld_k, ld_v, work[0].data_ptr(), work[1], cache.block_tables.data_ptr(),
+            cache.block_tables.shape[1], cache.block_size, key_rows, _lib.ptr(key_row), out.data_ptr(), out.stride(0), T, nq, nkv, hd,
+            hd, int(exact), int(work[2]), float(scale), st, stream)
+        _lib.check(rc, "mfb_ragged_prefill_tc")
+        _lib.count_launch()
+
+    if plan.fresh[1]:
+        launch(plan.fresh, k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), T, plan.cu, False)
+    if plan.past[1]:
+        row = nkv * hd
+        if ksc is None and lib.mfb_ragged_prefill_tc_supported(nq, nkv, hd, hd, cache.block_size):
+            launch(plan.past, kc.data_ptr(), vc.data_ptr(), row, row, kc.shape[0] * cache.block_size, None, True)
+        else:
+            copies = torch.empty((2, plan.n_past_rows, row), dtype=q.dtype, device=q.device)
+            _gather_rows(cache, copies[0], kc, ksc, plan.past_rows, plan.longest)
+            _gather_rows(cache, copies[1], vc, vsc, plan.past_rows, plan.longest)
+            launch(plan.past, copies[0].data_ptr(), copies[1].data_ptr(), row, row, plan.n_past_rows, plan.past_rows, True)
+    return out
+
+
+def _gather_rows(cache, out, rows, scales, cu, longest: int):
+    """Cached rows of every sequence, one after the other (``cu [B + 1]``), de-quantised where ``scales`` are given."""
+    lib, tables = _lib.get_lib(), cache.block_tables
+    B, max_blocks = tables.shape
+    heads, dim = rows.shape[2:]
+    if scales is None:
+        rc = lib.mfb_gather_cache(rows.data_ptr(), tables.data_ptr(), cu.data_ptr(), out.data_ptr(), B, longest, cache.block_size,
+                                  max_blocks, heads * dim, _lib.stream_ptr())
+    else:
+        rc = lib.mfb_gather_cache_int8(rows.data_ptr(), scales.data_ptr(), tables.data_ptr(), cu.data_ptr(), out.data_ptr(), B, longest,
+                                       cache.block_size, max_blocks, heads, dim, _lib.stream_ptr())
+    _lib.check(rc, "mfb_gather_cache")
+    _lib.count_launch()
+
+
 def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
     """q: [T, nq, hd]; k/v: [T, nkv, hd] of the new tokens. Returns [T, nq*hd]."""
     cache: KVCacheContext = meta.cache
@@ -266,7 +395,11 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
             o = Fn.attention_reference(q[b:b + 1].unsqueeze(0), kk.unsqueeze(0), vv.unsqueeze(0), causal=False, scale=scale)
             out[b] = o[0, 0]
         return out.view(T, nq * hd)
-    # prefill (optionally with history, e.g. chunked prefill): per-sequence causal attention
+    # prefill (optionally with history, e.g. chunked prefill): causal attention of all sequences in one or two launches
+    out = _ragged_prefill(q, k, v, cache, layer, scale)
+    if out is not None:
+        return out
+    # other types, sizes and layouts: sequence by sequence
     outs = []
     lens = cache.context_lens.tolist()
     for b in range(B):
@@ -322,6 +455,50 @@ def mla_decode_attention(q_cat: torch.Tensor, latent_cache: torch.Tensor, block_
     return out
 
 
+_EXPANDED_BYTES = 2 << 30        # of expanded keys and values at a time; more heads than that take turns
+
+
+def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
+    """Multi-latent attention of a step's new rows (any lengths, with or without history) over keys and values expanded from the
+    cached latents once per call. Expanded numbers are kept as the sum of two bf16 numbers and the softmax weights likewise, so that
+    nothing between query and result is rounded to 16 bits. None where the kernel does not take the call."""
+    T, nh, nope = q_nope.shape
+    rope_d, vd, rank = attn.rope_d, attn.vd, attn.kv_rank
+    w, rows = attn.linear_kvb.weight, cache.key_cache[layer]
+    if not (q_nope.is_cuda and q_nope.dtype == q_pe.dtype == rows.dtype == w.dtype == torch.bfloat16 and (nope, rope_d, vd) == (128, 64, 128)
+            and rank % 8 == 0 and T and w.is_contiguous() and rows.is_contiguous() and Fn.get_gemm_backend() == "tcgen05") or _needs_graph(q_nope, q_pe, w):
+        return None
+    plan = _prefill_plan(cache, T)
+    n = plan.n_all_rows if plan.ok else 0
+    if not plan.ok or n >= 1 << 31:
+        return None
+    q_pe = q_pe.reshape(T, nh, rope_d)
+    if q_nope.stride(2) != 1 or q_nope.stride(1) % 8 or q_nope.stride(0) % 8 or q_nope.stride(1) < nope or q_nope.stride(0) < nope \
+            or q_nope.data_ptr() % 16:
+        q_nope = q_nope.contiguous()
+    q_pe = q_pe.contiguous()
+    lib, dev = _lib.get_lib(), q_nope.device
+    latent = torch.empty((n, rank + rope_d), dtype=torch.bfloat16, device=dev)
+    _gather_rows(cache, latent, rows, None, plan.all_rows, plan.longest)
+    out = torch.empty((plan.rows, nh * vd), dtype=torch.bfloat16, device=dev)
+    w = w.view(nh, nope + vd, rank)
+    step = max(1, min(nh, _EXPANDED_BYTES // (n * 256 * 8)))
+    for h in range(0, nh, step):
+        heads = min(step, nh - h)
+        kv = Fn.gemm(latent[:, :rank], w[h:h + heads].view(-1, rank), out_dtype=torch.float32)
+        parts = torch.empty((2,) + kv.shape, dtype=torch.bfloat16, device=dev)
+        rc = lib.mfb_split_f32(kv.data_ptr(), parts[0].data_ptr(), parts[1].data_ptr(), kv.numel(), _lib.stream_ptr())
+        _lib.check(rc, "mfb_split_f32")
+        rc = lib.mfb_latent_prefill_tc(
+            q_nope.data_ptr() + 2 * h * q_nope.stride(1), q_nope.stride(0), q_nope.stride(1), q_pe.data_ptr() + 2 * h * rope_d,
+            q_pe.stride(0), rope_d, parts[0].data_ptr(), parts[1].data_ptr(), latent.data_ptr() + 2 * rank, rank + rope_d, n,
+            plan.all_rows.data_ptr(), plan.all[0].data_ptr(), plan.all[1], out.data_ptr() + 2 * h * vd, out.stride(0), T, heads,
+            float(attn.scale), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+        _lib.check(rc, "mfb_latent_prefill_tc")
+        _lib.count_launch(2)
+    return out
+
+
 def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
     """Multi-latent attention with a latent cache ``[kv_lora ‖ k_pe]``.
 
@@ -366,6 +543,9 @@ def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
             o = native.mla_forward(qf[a:e].unsqueeze(0), k[a:e].unsqueeze(0), v[a:e].unsqueeze(0), True, attn.scale)
             outs.append(o.reshape(e - a, nh * vd))
         return torch.cat(outs, dim=0)
+    out = _latent_prefill(attn, q_nope, q_pe, cache, layer)
+    if out is not None:
+        return out
     outs = []
     for b in range(B):
         a, e = cache.cu_q[b], cache.cu_q[b + 1]

@@ -144,6 +144,10 @@ def _declare(lib):
     sig("mfb_paged_prefill_tc_supported", [I, I, I, I, I])
     sig("mfb_paged_prefill_tc_wide_supported", [I, I, I, I, I])
     sig("mfb_paged_prefill_tc", [P, P, P, P, I, I, P, P, P] + [I] * 11 + [L, L, F, F, L, F, P, P])
+    sig("mfb_split_f32", [P, P, P, L, P])
+    sig("mfb_ragged_prefill_tc_supported", [I, I, I, I, I])
+    sig("mfb_ragged_prefill_tc", [P, L, L, P, P, L, L, P, I, P, I, I, L, P, P, L] + [I] * 7 + [F, P, P])
+    sig("mfb_latent_prefill_tc", [P, L, L, P, L, L, P, P, P, L, L, P, P, I, P, L, I, I, F, P, P])
     sig("mfb_paged_attention_any", [P] * 8 + [I] * 11 + [F, F, L, F, I, P])
     sig("mfb_residual_streams", [P, I, P, L, P, P, P, P, P, P, I, I, I, F, I, P])
     sig("mfb_embed_stream", [P, P, P, P, P, I, I, I, F, I, P])

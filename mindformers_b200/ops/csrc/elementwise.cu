@@ -237,6 +237,25 @@ static inline int ew_grid(long long work_items, int threads) {
   return (int)blocks;
 }
 
+// hi + lo = x to 16 bits of fraction. Bound by memory: 8 bytes moved per number; eight numbers per thread so that every access
+// is 16 bytes wide.
+__global__ void split_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
+                                 long long vecs) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
+    float f[8];
+    *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(x)[2 * i];
+    *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(x)[2 * i + 1];
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      h[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
+      l[j] = pack_bf16x2(f[2 * j] - __uint_as_float(h[j] << 16), f[2 * j + 1] - __uint_as_float(h[j] & 0xffff0000u));
+    }
+    reinterpret_cast<uint4*>(hi)[i] = make_uint4(h[0], h[1], h[2], h[3]);
+    reinterpret_cast<uint4*>(lo)[i] = make_uint4(l[0], l[1], l[2], l[3]);
+  }
+}
+
 }  // namespace mfb
 
 extern "C" {
@@ -312,6 +331,16 @@ int mfb_add_bf16(const void* a, const void* b, void* out, long long n, cudaStrea
   if (n <= 0) return 0;
   add_bf16_kernel<<<ew_grid(n / 8 + 1, 256), 256, 0, stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
                                                                (__nv_bfloat16*)out, n);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// x [n] fp32 as the sum of two bf16 arrays; n a multiple of 8, every address on 16 bytes.
+int mfb_split_f32(const float* x, void* hi, void* lo, long long n, cudaStream_t stream) {
+  if (n < 0 || n % 8) { mfb_host::set_error("split_f32: %lld numbers", n); return 1; }
+  if (n == 0) return 0;
+  long long blocks = (n / 8 + 255) / 256;
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  split_f32_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

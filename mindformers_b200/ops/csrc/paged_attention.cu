@@ -274,7 +274,7 @@ __global__ void gather_cache_kernel(const __nv_bfloat16* __restrict__ cache, con
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)n * vecs;
        i += (long long)gridDim.x * blockDim.x) {
     const int tok = (int)(i / vecs), c = (int)(i - (long long)tok * vecs);
-    const int blk = block_tables[(size_t)b * max_blocks + tok / block_size];
+    const int blk = max(block_tables[(size_t)b * max_blocks + tok / block_size], 0);   // none: any block, as in the decode kernels
     const uint4 v = *reinterpret_cast<const uint4*>(cache + ((size_t)blk * block_size + tok % block_size) * row_elems + c * 8);
     *reinterpret_cast<uint4*>(out + (size_t)(start + tok) * row_elems + c * 8) = v;
   }
@@ -290,7 +290,7 @@ __global__ void gather_cache_int8_kernel(const int8_t* __restrict__ cache, const
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (long long)n * heads; w += warps) {
     const int tok = (int)(w / heads), h = (int)(w - (long long)tok * heads);
-    const int blk = block_tables[(size_t)b * max_blocks + tok / block_size];
+    const int blk = max(block_tables[(size_t)b * max_blocks + tok / block_size], 0);   // none: any block, as in the decode kernels
     const size_t slot = (size_t)blk * block_size + tok % block_size;
     const float sc = scale[slot * heads + h];
     const int8_t* src = cache + (slot * heads + h) * hd;

@@ -53,6 +53,8 @@ struct Args {
   float cap_poly[5];           // capped score (log2 units) = s * polynomial in s^2, for |s| * cap_scale <= kPolyReach
   long long ld_out;
   float out_scale;
+  const int* key_row;        // [B] row of K and V at which a sequence's keys start (they lie one after the other), or null: paged
+  int zero_tail;             // rows of V past a sequence's last key count as zero, whatever they hold
   int* status;
 };
 
@@ -114,19 +116,37 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
 constexpr float kPolyReach = 0.6f;
 constexpr float kTanhRatio[5] = {0.999999926f, -0.33332302f, 0.133100644f, -0.0520966534f, 0.0154687513f};
 
+// How much of a product's operands the tensor cores see.
+//   kBf16     P rounded to bf16.
+//   kSplitP   P as the sum of two bf16 numbers (16 bits of its fraction): the second lies in the columns of S that the first
+//             leaves free, and P V is two products. What the weights lose is then far below the rounding of the result, as with
+//             weights kept in 32 bits: 1.5 times the products of kBf16, for callers whose weights may not be rounded.
+//   kLatent   keys and values that are themselves 32-bit products (expanded latents) come as sums of two bf16 numbers too; the
+//             last 64 columns of Q and K, the rotated part that all heads share, come through maps of their own.
+//   kRows     kBf16 for ragged rows.
+// All but kBf16 take keys and values that lie one after the other (key_row) as well as pages, and honour zero_tail.
+// What the split costs and what it replaces: 4 portions of up to 512 rows behind 5000 cached tokens (32 / 8 heads of 128, two layers)
+// take 0.64 ms with kSplitP, 12.0 ms as 32-bit products and a softmax over whole score matrices, both 0.0017 off the 64-bit result
+// (the rounding of the result); 3000 rows of 16 latent heads behind 1200 tokens 0.75 ms against 4.9 ms, projections included.
+enum Parts { kBf16 = 0, kSplitP = 1, kLatent = 2, kRows = 3 };
+
 // HQ: padded query / key size (64, 128 or 192), HV: padded value size (64 or 128); CAP: scores are soft-capped
-template <int HQ, int HV, bool CAP>
+template <int HQ, int HV, bool CAP, int PARTS>
 __global__ void __launch_bounds__(kThreads, HQ > 128 ? 1 : 2)
 paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                        const __grid_constant__ CUtensorMap tmV, const Args args) {
+                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ2,
+                        const __grid_constant__ CUtensorMap tmK2, const Args args) {
+  constexpr bool SPLIT = PARTS == kSplitP || PARTS == kLatent, ROWS = PARTS != kBf16;
   constexpr int QB = HQ / 64, VB = HV / 64;          // 64-column sub-tiles
-  constexpr int kQBytes = QB * kSubBytes, kVBytes = VB * kSubBytes;
+  constexpr int KB = PARTS == kLatent ? 2 * QB - 1 : QB;              // kLatent: head columns, shared columns, rest of the head columns
+  constexpr int VT = PARTS == kLatent ? 2 * VB : VB;
+  constexpr int kQBytes = QB * kSubBytes, kKBytes = KB * kSubBytes, kVBytes = VT * kSubBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + kQBytes;
-  uint8_t* sV = sK + kQBytes;
+  uint8_t* sV = sK + kKBytes;
   uint8_t* sOut = sV + kVBytes;               // 2 KB per softmax warp
   uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + 4 * 2048);
   uint64_t* q_full = bars;
@@ -168,6 +188,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
+    if (PARTS == kLatent) {
+      tma_prefetch_desc(&tmQ2);
+      tma_prefetch_desc(&tmK2);
+    }
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_holder), 256);
@@ -177,7 +201,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + kTile;   // P lives in the first 64 columns of S
+  // P lives in the first 64 columns of S, its second part in the other 64
+  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + kTile;
   if (warp == 0) {
     // ------------------------------ TMA producer (the whole warp, one lane issues) ------------------------------
     const bool leader = elect_one();
@@ -195,17 +220,45 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       const Tile t = tile_of(item);
       const int* table = args.block_tables + static_cast<size_t>(t.b) * args.max_blocks;
       const int kv_head = t.head / args.group, end = t.pos0 + t.rows;
-      const int kcol = kv_head * args.D, vcol = (args.vheads > 1 ? t.vsel : kv_head) * args.DV;
-      int page = tile_page(table, bs, t.lo * kTile, end);
+      // kLatent: a head's key columns, then its value columns
+      const int kcol = PARTS == kLatent ? kv_head * (HQ - 64 + HV) : kv_head * args.D;
+      const int vcol = PARTS == kLatent ? kcol + HQ - 64 : (args.vheads > 1 ? t.vsel : kv_head) * args.DV;
+      const int key0 = ROWS && args.key_row ? args.key_row[t.b] : 0;
+      int page = ROWS && args.key_row ? 0 : tile_page(table, bs, t.lo * kTile, end);
       claim(q_empty, (n & 1) ^ 1, q_full, kQBytes);
       if (!ok) break;
       if (leader)
-        for (int c = 0; c < QB; ++c) tma_load_3d(smem_u32(sQ) + c * kSubBytes, &tmQ, smem_u32(q_full), c * 64, t.head, t.q0);
+        for (int c = 0; c < QB; ++c) {
+          const bool shared = PARTS == kLatent && c == QB - 1;
+          tma_load_3d(smem_u32(sQ) + c * kSubBytes, shared ? &tmQ2 : &tmQ, smem_u32(q_full), shared ? 0 : c * 64, t.head, t.q0);
+        }
       __syncwarp();
       for (int j = t.lo; j < t.n_kv; ++j, ++it) {
         const uint32_t ph = it & 1;
-        claim(k_empty, ph ^ 1, k_full, kQBytes);
+        claim(k_empty, ph ^ 1, k_full, kKBytes);
         if (!ok) break;
+        if (ROWS && args.key_row) {
+          // one box of 128 rows per sub-tile, from any row on
+          const int r = key0 + j * kTile;
+          if constexpr (PARTS == kLatent) {
+            for (int c = 0; c < QB - 1; ++c) {
+              tma_load_2d_warp(leader, smem_u32(sK) + c * kSubBytes, &tmK, smem_u32(k_full), kcol + c * 64, r);
+              tma_load_2d_warp(leader, smem_u32(sK) + (QB + c) * kSubBytes, &tmV, smem_u32(k_full), kcol + c * 64, r);
+            }
+            tma_load_2d_warp(leader, smem_u32(sK) + (QB - 1) * kSubBytes, &tmK2, smem_u32(k_full), 0, r);
+          } else {
+            for (int c = 0; c < QB; ++c)
+              tma_load_2d_warp(leader, smem_u32(sK) + c * kSubBytes, &tmK, smem_u32(k_full), kcol + c * 64, r);
+          }
+          claim(v_empty, ph ^ 1, v_full, kVBytes);
+          if (!ok) break;
+          for (int c = 0; c < VB; ++c) {
+            tma_load_2d_warp(leader, smem_u32(sV) + c * kSubBytes, PARTS == kLatent ? &tmK : &tmV, smem_u32(v_full), vcol + c * 64, r);
+            if constexpr (PARTS == kLatent)
+              tma_load_2d_warp(leader, smem_u32(sV) + (VB + c) * kSubBytes, &tmV, smem_u32(v_full), vcol + c * 64, r);
+          }
+          continue;
+        }
         tma_load_pages(leader, smem_u32(sK), kSubBytes, &tmK, smem_u32(k_full), page, bs, kcol, QB);
         const int next = j + 1 < t.n_kv ? tile_page(table, bs, (j + 1) * kTile, end) : 0;
         claim(v_empty, ph ^ 1, v_full, kVBytes);
@@ -237,6 +290,16 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 #pragma unroll
       for (int k = 0; k < kTile / 16; ++k)           // bf16 pairs: 8 columns of P per 16 keys
         umma_f16_ts_warp(leader, tmem_O, tmem_S + k * 8, v_desc + ((k * 16 * 128) >> 4), IDESC_PV, (!first_key || k > 0) ? 1u : 0u);
+      if constexpr (SPLIT) {
+#pragma unroll
+        for (int k = 0; k < kTile / 16; ++k)
+          umma_f16_ts_warp(leader, tmem_O, tmem_S + 64 + k * 8, v_desc + ((k * 16 * 128) >> 4), IDESC_PV, 1u);
+      }
+      if constexpr (PARTS == kLatent) {
+#pragma unroll
+        for (int k = 0; k < kTile / 16; ++k)
+          umma_f16_ts_warp(leader, tmem_O, tmem_S + k * 8, v_desc + ((VB * kSubBytes + k * 16 * 128) >> 4), IDESC_PV, 1u);
+      }
       umma_commit_warp(leader, smem_u32(pv_done));
       umma_commit_warp(leader, smem_u32(v_empty));
     };
@@ -254,6 +317,14 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           constexpr int kSubUnits = kSubBytes >> 4;
           const int off = (k >> 2) * kSubUnits + (k & 3) * 2;
           umma_f16_ss_warp(leader, tmem_S, q_desc + off, k_desc + off, IDESC_QK, k > 0 ? 1u : 0u);
+        }
+        if constexpr (PARTS == kLatent) {
+#pragma unroll
+          for (int k = 0; k < (HQ - 64) / 16; ++k) {
+            constexpr int kSubUnits = kSubBytes >> 4;
+            const int off = (k >> 2) * kSubUnits + (k & 3) * 2;
+            umma_f16_ss_warp(leader, tmem_S, q_desc + off, k_desc + QB * kSubUnits + off, IDESC_QK, 1u);
+          }
         }
         umma_commit_warp(leader, smem_u32(s_full));
         umma_commit_warp(leader, smem_u32(k_empty));
@@ -350,6 +421,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           uint64_t rs2[4] = {0, 0, 0, 0};
           // exp2 of the scaled, shifted scores two at a time; P goes back as bf16 pairs, 64 score columns (32 packed
           // registers) per store, into the first 64 columns of this tile's S buffer
+          uint32_t rest[SPLIT ? 32 : 1];       // second part of P: stored once the scores it overwrites are read
+          (void)rest;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             // pass 2: 64 scores at a time; the second half is read before the first half's P overwrites columns 0..31
@@ -358,6 +431,15 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 #pragma unroll
               for (int i = 0; i < 32; ++i) zero[i] = 0u;
               tmem_st_32x32b_x32(s_tmem + h * 32, zero);
+              if constexpr (SPLIT) {
+                if (h == 0) {
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) rest[i] = 0u;
+                } else {
+                  tmem_st_32x32b_x32(s_tmem + 64, rest);
+                  tmem_st_32x32b_x32(s_tmem + 96, zero);
+                }
+              }
               continue;
             }
             uint32_t sr[64];
@@ -367,6 +449,9 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
               tmem_ld_32x32b_x32(s_tmem + h * 64, ra);
               tmem_ld_32x32b_x32(s_tmem + h * 64 + 32, rb);
               tmem_ld_wait();
+            }
+            if constexpr (SPLIT) {
+              if (h == 1) tmem_st_32x32b_x32(s_tmem + 64, rest);
             }
             float* s = reinterpret_cast<float*>(sr);
             if constexpr (CAP) {
@@ -411,8 +496,13 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
               const float e0 = ex2(t0), e1 = ex2(t1);
               rs2[i & 3] = add2(rs2[i & 3], pack2(e0, e1));
               pk[i] = pack_bf16x2(e0, e1);
+              if constexpr (SPLIT)
+                rest[i] = pack_bf16x2(e0 - __uint_as_float(pk[i] << 16), e1 - __uint_as_float(pk[i] & 0xffff0000u));
             }
             tmem_st_32x32b_x32(s_tmem + h * 32, pk);
+            if constexpr (SPLIT) {
+              if (h == 1) tmem_st_32x32b_x32(s_tmem + 96, rest);
+            }
           }
           float r0, r1, r2, r3;
           unpack2(add2(rs2[0], rs2[1]), r0, r1);
@@ -421,6 +511,19 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         };
         if (lo_max > 0 || hi_min < kTile - 1) softmax_tile(std::true_type{});
         else softmax_tile(std::false_type{});
+        if (ROWS && args.zero_tail && j == n_kv - 1 && t.pos0 + t.rows < n_kv * kTile) {
+          // rows past the last key belong to another sequence or to nobody: their weights are zero, but zero times an
+          // infinity there would not be. One row per thread; the product waits for p_ready below.
+          ok = mbar_wait(smem_u32(v_full), it & 1, abort_flag, args.status, kStatusWaitTimeoutEpilogue);
+          if (!ok) break;
+          if (j * kTile + row >= t.pos0 + t.rows) {
+#pragma unroll
+            for (int c = 0; c < VT; ++c)
+#pragma unroll
+              for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(sV + c * kSubBytes + row * 128 + q * 16) = make_uint4(0, 0, 0, 0);
+          }
+          fence_proxy_async_smem();
+        }
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(smem_u32(p_ready));
@@ -805,13 +908,14 @@ int launch_values(const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMa
   return 0;
 }
 
-// three-dimensional map of q [T, Hq, D]: box of 128 tokens x 1 head x 64 columns; columns past D read as zero
-int make_q_map(CUtensorMap* out, const void* q, uint64_t T, uint64_t Hq, uint64_t D) {
+// three-dimensional map of q [T, Hq, D] with rows ld and heads ld_head elements apart: box of 128 tokens x 1 head x 64 columns;
+// columns past D read as zero
+int make_q_map(CUtensorMap* out, const void* q, uint64_t T, uint64_t Hq, uint64_t D, uint64_t ld, uint64_t ld_head) {
   mfb_host::EncodeTiledFn enc = mfb_host::get_encode_tiled();
   if (!enc) { mfb_host::set_error("cuTensorMapEncodeTiled entry point not available"); return 1; }
-  if ((reinterpret_cast<uintptr_t>(q) & 15) || (D * 2) % 16) { mfb_host::set_error("paged_prefill_tc: q not aligned"); return 2; }
+  if ((reinterpret_cast<uintptr_t>(q) & 15) || D % 8 || ld % 8 || ld_head % 8) { mfb_host::set_error("paged_prefill_tc: q not aligned"); return 2; }
   cuuint64_t gdim[3] = {D, Hq, T};
-  cuuint64_t gstride[2] = {D * 2, Hq * D * 2};
+  cuuint64_t gstride[2] = {ld_head * 2, ld * 2};
   cuuint32_t box[3] = {64, 1, kTile};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), gdim, gstride, box, estr,
@@ -821,12 +925,14 @@ int make_q_map(CUtensorMap* out, const void* q, uint64_t T, uint64_t Hq, uint64_
   return 0;
 }
 
-template <int HQ, int HV, bool CAP>
-int launch(const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMap& tV, const Args& a, int max_ctas, cudaStream_t stream) {
-  constexpr int QBYTES = HQ / 64 * kSubBytes, VBYTES = HV / 64 * kSubBytes;
-  constexpr int SMEM = 2 * QBYTES + VBYTES + 4 * 2048 + 9 * 8 + 16 + 1024;
+template <int HQ, int HV, bool CAP, int PARTS>
+int launch(const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMap& tV, const CUtensorMap& tQ2, const CUtensorMap& tK2,
+           const Args& a, int max_ctas, cudaStream_t stream) {
+  constexpr int QBYTES = HQ / 64 * kSubBytes, VBYTES = HV / 64 * (PARTS == kLatent ? 2 : 1) * kSubBytes;
+  constexpr int KBYTES = PARTS == kLatent ? 2 * QBYTES - kSubBytes : QBYTES;
+  constexpr int SMEM = QBYTES + KBYTES + VBYTES + 4 * 2048 + 9 * 8 + 16 + 1024;
   static_assert((HQ > 128 ? 1 : 2) * SMEM <= 232448, "shared memory budget exceeded");
-  auto kern = paged_prefill_tc_kernel<HQ, HV, CAP>;
+  auto kern = paged_prefill_tc_kernel<HQ, HV, CAP, PARTS>;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) {
@@ -836,7 +942,7 @@ int launch(const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMap& tV, 
     attr_set = true;
   }
   const int grid = a.n_items < max_ctas ? a.n_items : max_ctas;
-  kern<<<grid, kThreads, SMEM, stream>>>(tQ, tK, tV, a);
+  kern<<<grid, kThreads, SMEM, stream>>>(tQ, tK, tV, tQ2, tK2, a);
   if (cudaGetLastError() != cudaSuccess) { mfb_host::set_error("paged_prefill_tc: launch failed"); return 11; }
   return 0;
 }
@@ -890,7 +996,7 @@ int mfb_paged_prefill_tc(const void* q, const void* key_cache, const void* value
   const uint64_t rows = (uint64_t)num_blocks * block_size;
   if ((rc = mfb_host::make_tmap_2d(&tK, key_cache, 2, BF, rows, (uint64_t)Hkv * D, (uint64_t)ld_k, block_size, 64))) return 30 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tV, value_cache, 2, BF, rows, (uint64_t)Hkv * DV, (uint64_t)ld_v, block_size, 64))) return 40 + rc;
-  if ((rc = ppt::make_q_map(&tQ, q, T, Hq, D))) return 20 + rc;
+  if ((rc = ppt::make_q_map(&tQ, q, T, Hq, D, (uint64_t)Hq * D, D))) return 20 + rc;
   ppt::Args a;
   a.work = reinterpret_cast<const int4*>(work); a.vheads = all_values ? Hkv : 1; a.n_items = n_work * Hq * a.vheads;
   a.block_tables = block_tables; a.sink = sink;
@@ -901,7 +1007,7 @@ int mfb_paged_prefill_tc(const void* q, const void* key_cache, const void* value
   a.cap_scale = softcap > 0.f ? scale / softcap : 0.f;
   float power = a.scale_log2;
   for (int k = 0; k < 5; ++k, power *= a.cap_scale * a.cap_scale) a.cap_poly[k] = ppt::kTanhRatio[k] * power;
-  a.ld_out = ld_out; a.out_scale = out_scale;
+  a.ld_out = ld_out; a.out_scale = out_scale; a.key_row = nullptr; a.zero_tail = 0;
   if (a.vheads > 1 && !sink && !(softcap > 0.f)) {
     if (D > 64) return DV > 64 ? ppt::launch_values<128, 128>(tQ, tK, tV, a, n_work, Hkv, stream)
                                : ppt::launch_values<128, 64>(tQ, tK, tV, a, n_work, Hkv, stream);
@@ -910,10 +1016,11 @@ int mfb_paged_prefill_tc(const void* q, const void* key_cache, const void* value
   }
   const int max_ctas = persistent ? (D > 128 ? 1 : 2) * 148 : a.n_items;
 #define MFB_PPT(HQ_, HV_) \
-  return softcap > 0.f ? ppt::launch<HQ_, HV_, true>(tQ, tK, tV, a, max_ctas, stream) : ppt::launch<HQ_, HV_, false>(tQ, tK, tV, a, max_ctas, stream)
+  return softcap > 0.f ? ppt::launch<HQ_, HV_, true, ppt::kBf16>(tQ, tK, tV, tQ, tK, a, max_ctas, stream) \
+                       : ppt::launch<HQ_, HV_, false, ppt::kBf16>(tQ, tK, tV, tQ, tK, a, max_ctas, stream)
   if (D > 128)
-    return DV > 64 ? ppt::launch<192, 128, false>(tQ, tK, tV, a, max_ctas, stream)
-                   : ppt::launch<192, 64, false>(tQ, tK, tV, a, max_ctas, stream);
+    return DV > 64 ? ppt::launch<192, 128, false, ppt::kBf16>(tQ, tK, tV, tQ, tK, a, max_ctas, stream)
+                   : ppt::launch<192, 64, false, ppt::kBf16>(tQ, tK, tV, tQ, tK, a, max_ctas, stream);
   if (D > 64) {
     if (DV > 64) MFB_PPT(128, 128);
     MFB_PPT(128, 64);
@@ -921,6 +1028,81 @@ int mfb_paged_prefill_tc(const void* q, const void* key_cache, const void* value
   if (DV > 64) MFB_PPT(64, 128);
   MFB_PPT(64, 64);
 #undef MFB_PPT
+}
+
+// 1 when mfb_ragged_prefill_tc serves these shapes (bf16). Heads fill the 64-column boxes whole, so that no box holds another head's
+// numbers, which may not be finite; block_size 0: keys that lie one after the other only.
+int mfb_ragged_prefill_tc_supported(int Hq, int Hkv, int D, int DV, int block_size) {
+  return (D == 64 || D == 128) && DV == D && mfb_paged_prefill_tc_supported(Hq, Hkv, D, DV, block_size ? block_size : 128);
+}
+
+// Prefill of a ragged batch of ordinary grouped-query attention (causal, no window, sink or cap), q [T, Hq, D] with rows ld_q and heads
+// ld_head elements apart. Keys and values of sequence b: the pages of block_tables in caches [num_blocks, block_size, Hkv, D | DV]
+// (key_row null), or rows key_row[b] .. of k / v [key_rows, Hkv, D | DV]. Whatever lies past a sequence's last key has no effect.
+// exact_weights: the softmax weights are not rounded to 16 bits. Other arguments as above.
+int mfb_ragged_prefill_tc(const void* q, long long ld_q, long long ld_head, const void* k, const void* v, long long ld_k, long long ld_v,
+                          const int* work, int n_work, const int* block_tables, int max_blocks, int block_size, long long key_rows,
+                          const int* key_row, void* out, long long ld_out, int T, int Hq, int Hkv, int D, int DV, int exact_weights,
+                          int persistent, float scale, int* status, cudaStream_t stream) {
+  if (!mfb_ragged_prefill_tc_supported(Hq, Hkv, D, DV, key_row ? 128 : block_size) || key_rows < 1 || T < 1 ||
+      key_rows > 0x7fffffffLL) {
+    mfb_host::set_error("ragged_prefill_tc: unsupported Hq=%d Hkv=%d D=%d DV=%d block_size=%d", Hq, Hkv, D, DV, block_size);
+    return 1;
+  }
+  if (n_work <= 0) return 0;
+  if (ld_k < (long long)Hkv * D || ld_v < (long long)Hkv * DV || ld_out % 8 || (reinterpret_cast<uintptr_t>(out) & 15)) {
+    mfb_host::set_error("ragged_prefill_tc: row pitches %lld, %lld, %lld", ld_k, ld_v, ld_out);
+    return 1;
+  }
+  CUtensorMap tQ, tK, tV;
+  int rc;
+  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const int box = key_row ? ppt::kTile : block_size;
+  if ((rc = mfb_host::make_tmap_2d(&tK, k, 2, BF, key_rows, (uint64_t)Hkv * D, (uint64_t)ld_k, box, 64))) return 30 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tV, v, 2, BF, key_rows, (uint64_t)Hkv * DV, (uint64_t)ld_v, box, 64))) return 40 + rc;
+  if ((rc = ppt::make_q_map(&tQ, q, T, Hq, D, ld_q, ld_head))) return 20 + rc;
+  ppt::Args a = {};
+  a.work = reinterpret_cast<const int4*>(work); a.vheads = 1; a.n_items = n_work * Hq;
+  a.block_tables = block_tables; a.out = reinterpret_cast<__nv_bfloat16*>(out);
+  a.num_q_heads = Hq; a.group = Hq / Hkv; a.D = D; a.DV = DV; a.block_size = block_size; a.max_blocks = max_blocks;
+  a.scale_log2 = scale * 1.4426950408889634f; a.status = status;
+  a.ld_out = ld_out; a.out_scale = 1.f; a.key_row = key_row; a.zero_tail = 1;
+  const int max_ctas = persistent ? 2 * 148 : a.n_items;
+  const bool wide = D > 64;
+  if (exact_weights)
+    return wide ? ppt::launch<128, 128, false, ppt::kSplitP>(tQ, tK, tV, tQ, tK, a, max_ctas, stream)
+                : ppt::launch<64, 64, false, ppt::kSplitP>(tQ, tK, tV, tQ, tK, a, max_ctas, stream);
+  return wide ? ppt::launch<128, 128, false, ppt::kRows>(tQ, tK, tV, tQ, tK, a, max_ctas, stream)
+              : ppt::launch<64, 64, false, ppt::kRows>(tQ, tK, tV, tQ, tK, a, max_ctas, stream);
+}
+
+// Prefill of multi-latent attention, 128 + 64 numbers per query and key and 128 per value. q_nope [T, H, 128] and q_pe [T, H, 64] with
+// rows ld_q / ld_qp and heads hd_q / hd_qp elements apart; kv_hi + kv_lo [key_rows, H, 128 + 128] the expanded keys and values as sums of
+// two bf16 numbers, pe [key_rows, 64] (rows ld_pe apart) the rotated key part. Sequence b's keys are the rows key_row[b] .. . The
+// weights are not rounded to 16 bits.
+int mfb_latent_prefill_tc(const void* q_nope, long long ld_q, long long hd_q, const void* q_pe, long long ld_qp, long long hd_qp,
+                          const void* kv_hi, const void* kv_lo, const void* pe, long long ld_pe, long long key_rows, const int* key_row,
+                          const int* work, int n_work, void* out, long long ld_out, int T, int H, float scale, int* status, cudaStream_t stream) {
+  if (H < 1 || T < 1 || key_rows < 1 || key_rows > 0x7fffffffLL || !key_row || ld_out % 8 || (reinterpret_cast<uintptr_t>(out) & 15)) {
+    mfb_host::set_error("latent_prefill_tc: T=%d H=%d rows=%lld", T, H, key_rows);
+    return 1;
+  }
+  if (n_work <= 0) return 0;
+  CUtensorMap tQ, tQ2, tK, tV, tK2;
+  int rc;
+  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  if ((rc = ppt::make_q_map(&tQ, q_nope, T, H, 128, ld_q, hd_q))) return 20 + rc;
+  if ((rc = ppt::make_q_map(&tQ2, q_pe, T, H, 64, ld_qp, hd_qp))) return 25 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tK, kv_hi, 2, BF, key_rows, (uint64_t)H * 256, (uint64_t)H * 256, ppt::kTile, 64))) return 30 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tV, kv_lo, 2, BF, key_rows, (uint64_t)H * 256, (uint64_t)H * 256, ppt::kTile, 64))) return 40 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tK2, pe, 2, BF, key_rows, 64, (uint64_t)ld_pe, ppt::kTile, 64))) return 50 + rc;
+  ppt::Args a = {};
+  a.work = reinterpret_cast<const int4*>(work); a.vheads = 1; a.n_items = n_work * H;
+  a.out = reinterpret_cast<__nv_bfloat16*>(out);
+  a.num_q_heads = H; a.group = 1; a.D = 192; a.DV = 128; a.block_size = 128;
+  a.scale_log2 = scale * 1.4426950408889634f; a.status = status;
+  a.ld_out = ld_out; a.out_scale = 1.f; a.key_row = key_row; a.zero_tail = 1;
+  return ppt::launch<192, 128, false, ppt::kLatent>(tQ, tK, tV, tQ2, tK2, a, a.n_items, stream);
 }
 
 }  // extern "C"

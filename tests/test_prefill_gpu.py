@@ -1,0 +1,138 @@
+"""Prefill attention of ragged batches on the tensor cores, against 64-bit PyTorch."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _attend(q, k, v, scale):
+    """Causal attention of the last rows of a sequence in 64 bits: q [n, H, D], k / v [L, G, D]."""
+    n, H, _ = q.shape
+    L, G, _ = k.shape
+    k, v = (t.double().repeat_interleave(H // G, 1) for t in (k, v))
+    s = torch.einsum("qhd,khd->hqk", q.double(), k) * scale
+    hide = torch.arange(L, device=DEV)[None] > torch.arange(L - n, L, device=DEV)[:, None]
+    return torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(hide, float("-inf")), -1), v).flatten(1)
+
+
+def _tables(lens, block):
+    need = [-(-n // block) for n in lens]
+    order = torch.randperm(sum(need)).to(torch.int32)
+    tables = torch.full((len(lens), max(need) + 1), -1, dtype=torch.int32)
+    at = 0
+    for b, n in enumerate(need):
+        tables[b, :n] = order[at:at + n]
+        at += n
+    return tables, sum(need)
+
+
+def _slots(tables, block, lens, news):
+    out = []
+    for b, (n, m) in enumerate(zip(lens, news)):
+        pos = torch.arange(n - m, n)
+        out.append(tables[b, pos // block].long() * block + pos % block)
+    return torch.cat(out)
+
+
+def _cached(rows, tables, b, n, block):
+    return rows[tables[b, :-(-n // block)].long().to(DEV)].flatten(0, 1)[:n]
+
+
+# lengths at the edges of the 128-row tiles, sequences without new rows and with one, histories of all kinds in one batch
+NEWS = [[1, 127, 0, 300], [128, 129, 1, 64], [257, 5]]
+PAST = [[0, 0, 0, 0], [700, 129, 64, 0], [128, 1]]
+
+
+@pytest.mark.parametrize("step", range(3))
+@pytest.mark.parametrize("heads,kv,dim", [(8, 2, 128), (7, 1, 128), (4, 4, 64)])
+@pytest.mark.parametrize("block,int8", [(16, False), (128, False), (64, True), (24, False)])
+def test_ragged_prefill(step, heads, kv, dim, block, int8):
+    from mindformers_b200.inference import paged_attention as pa
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(step)
+    news, past = NEWS[step], PAST[step]
+    lens = [n + p for n, p in zip(news, past)]
+    tables, blocks = _tables(lens, block)
+    ctx = pa.KVCacheContext(1, blocks, block, kv, dim, torch.bfloat16, DEV, kv_cache_dtype="int8" if int8 else None)
+    T = sum(news)
+    qkv = torch.randn(T, heads + 2 * kv, dim, device=DEV).to(torch.bfloat16)
+    q, k, v = qkv[:, :heads], qkv[:, heads:heads + kv], qkv[:, heads + kv:]
+    hist = torch.randn(2, sum(lens), kv, dim, device=DEV).to(torch.bfloat16)
+    step_meta = dict(block_tables=tables.numpy(), context_lens=lens, device=DEV)
+    if not int8:                       # what earlier users of the pages left behind has no effect
+        ctx.key_cache[0].fill_(float("nan"))
+        ctx.value_cache[0].fill_(float("inf"))
+    ctx.set_step(is_prefill=True, slot_mapping=_slots(tables, block, lens, lens).numpy(), q_seq_lens=lens, **step_meta)
+    pa._write_cache(ctx, 0, hist[0], hist[1])
+    ctx.set_step(is_prefill=True, slot_mapping=_slots(tables, block, lens, news).numpy(), q_seq_lens=news, **step_meta)
+    meta = types.SimpleNamespace(cache=ctx)
+    before = _lib.launch_count()
+    with torch.no_grad():
+        got = pa.paged_attention_forward(q, k, v, meta, 1, dim ** -0.5)
+        again = pa.paged_attention_forward(q, k, v, meta, 1, dim ** -0.5)
+    assert _lib.launch_count() > before + 2 and got.shape == (T, heads * dim)
+    assert torch.equal(got, again)
+    at = 0
+    for b, (n, m) in enumerate(zip(news, lens)):
+        rows = slice(at, at + n)
+        at += n
+        if not n:
+            continue
+        if n == m:
+            kk, vv = k[rows], v[rows]
+        else:
+            sc = pa._layer_scales(ctx, 0)
+            kk, vv = (pa._gather(c[0], tables[b].to(DEV), m, block, s, torch.bfloat16)
+                      for c, s in zip((ctx.key_cache, ctx.value_cache), sc))
+        want = _attend(q[rows], kk, vv, dim ** -0.5)
+        err = (got[rows].double() - want).norm() / want.norm()
+        # rounding of the result alone: 2^-9 at most, its mean square over a binade 2^-9 / sqrt(3) / 1.44; the weights of
+        # sequences without history are rounded too
+        assert err < (1.9e-3 if n < m else 4e-3), (b, float(err))
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("step", range(3))
+@pytest.mark.parametrize("heads,block,share", [(16, 128, 1 << 30), (3, 16, 1 << 30), (5, 64, 1)])
+def test_latent_prefill(step, heads, block, share, monkeypatch):
+    """``share``: bytes of expanded keys and values at a time (1: head by head)."""
+    from mindformers_b200.inference import paged_attention as pa
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(step)
+    monkeypatch.setattr(pa, "_EXPANDED_BYTES", share)
+    news, past = NEWS[step], PAST[step]
+    lens = [n + p for n, p in zip(news, past)]
+    tables, blocks = _tables(lens, block)
+    ctx = pa.KVCacheContext(1, blocks, block, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
+    ctx.key_cache[0].fill_(float("nan"))
+    w = (torch.randn(heads * 256, 512, device=DEV) * 512 ** -0.5).to(torch.bfloat16)
+    attn = types.SimpleNamespace(nh=heads, nope=128, rope_d=64, vd=128, kv_rank=512, layer_number=1, scale=192 ** -0.5,
+                                 linear_kvb=types.SimpleNamespace(weight=w))
+    T = sum(news)
+    q = torch.randn(T, heads, 192, device=DEV).to(torch.bfloat16)
+    lat = torch.randn(sum(lens), 576, device=DEV).to(torch.bfloat16)
+    step_meta = dict(block_tables=tables.numpy(), context_lens=lens, device=DEV)
+    ctx.set_step(is_prefill=True, slot_mapping=_slots(tables, block, lens, lens).numpy(), q_seq_lens=lens, **step_meta)
+    pa._write_cache(ctx, 0, lat.unsqueeze(1), None)
+    ctx.set_step(is_prefill=True, slot_mapping=_slots(tables, block, lens, news).numpy(), q_seq_lens=news, **step_meta)
+    new = torch.randn(T, 576, device=DEV).to(torch.bfloat16)
+    q_pe = q[..., 128:].clone()
+    with torch.no_grad():
+        got = pa.mla_paged_attention_forward(attn, q[..., :128], q_pe, new[:, :512], new[:, 512:], types.SimpleNamespace(cache=ctx))
+    assert got.shape == (T, heads * 128)
+    at = 0
+    for b, (n, m) in enumerate(zip(news, lens)):
+        rows = slice(at, at + n)
+        at += n
+        if not n:
+            continue
+        lt = _cached(ctx.key_cache[0][:, :, 0], tables, b, m, block).double()
+        kv = (lt[:, :512] @ w.double().t()).view(m, heads, 256)
+        keys = torch.cat((kv[..., :128], lt[:, None, 512:].expand(m, heads, 64)), -1)
+        want = _attend(q[rows], keys, kv[..., 128:], attn.scale)
+        err = (got[rows].double() - want).norm() / want.norm()
+        assert err < 1.9e-3, (b, float(err))         # rounding of the result alone
+    assert _lib.read_status() == 0
