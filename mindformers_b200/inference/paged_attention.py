@@ -15,10 +15,38 @@ import os
 import math
 from typing import List, Optional
 
+import numpy as np
 import torch
 
 from ..ops import _lib
 from ..ops import functional as Fn
+
+
+def _version(t: torch.Tensor) -> int:
+    """Counts changes in place (tensors made in inference mode keep no count)."""
+    return 0 if t.is_inference() else t._version
+
+
+def _to_device(arrays, device):
+    """int32 arrays as device tensors, each on 16 bytes, through one pinned buffer and one copy in stream order."""
+    at, spans = 0, []
+    for a in arrays:
+        spans.append((at, a.size, a.shape))
+        at += -(-a.size // 4) * 4
+    host = torch.empty(max(at, 1), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
+    flat = host.numpy()
+    for a, (start, n, _) in zip(arrays, spans):
+        flat[start:start + n] = a.reshape(-1)
+    dev = host.to(device, non_blocking=True)       # the pinned buffer is not handed out again before the copy is done
+    return [dev[start:start + n].view(shape) for start, n, shape in spans]
+
+
+def _host_lens(cache) -> list:
+    """The step's context lengths on the host: those ``set_step`` was given, unless the device tensor was replaced or changed since."""
+    known = getattr(cache, "host_lens", None)
+    if known is not None and known[0] is cache.context_lens and known[1] == _version(cache.context_lens):
+        return known[2]
+    return cache.context_lens.tolist()
 
 
 class KVCacheContext:
@@ -93,6 +121,7 @@ class KVCacheContext:
         self.last_token_index = None  # int64 [B] row of the last new token of each sequence
         self.cu_q = None              # python list of cumulative q lengths
         self.layer_offset = 0
+        self.host_lens = None         # what set_step was given: (context_lens, its version, the lengths)
         self.cu_q_dev = None          # int32 [B+1]: cu_q on the device (ragged caches, prefill steps)
         self.prefill_work = {}        # work lists of the prefill kernels, made when a layer needs them
         self.q_lens_host = self.context_lens_host = ()
@@ -122,26 +151,35 @@ class KVCacheContext:
 
     def set_step(self, *, is_prefill, block_tables, slot_mapping, context_lens, q_seq_lens, device):
         self.is_prefill = is_prefill
-        self.block_tables = torch.as_tensor(block_tables, dtype=torch.int32, device=device).contiguous()
-        self.slot_mapping = torch.as_tensor(slot_mapping, dtype=torch.int32, device=device).contiguous()
-        self.context_lens = torch.as_tensor(context_lens, dtype=torch.int32, device=device).contiguous()
         q = [int(x) for x in q_seq_lens]
-        self.q_seq_lens = torch.as_tensor(q, dtype=torch.int32, device=device)
-        self.prefill_work = {}
         cu = [0]
         for n in q:
             cu.append(cu[-1] + n)
         self.cu_q = cu
+        self.prefill_work = {}
+        # sequences without new tokens in this step (finished prompts of a chunked prefill, idle serving slots) have
+        # no row of their own: one entry per sequence that has tokens
+        last = [c - 1 for c, n in zip(cu[1:], q) if n > 0]
+        given = (block_tables, slot_mapping, context_lens)
+        self.host_lens = None
+        if torch.device(device).type != "cuda" or any(isinstance(x, torch.Tensor) and x.is_cuda for x in given):
+            self.block_tables, self.slot_mapping, self.context_lens = (
+                torch.as_tensor(x, dtype=torch.int32, device=device).contiguous() for x in given)
+            self.q_seq_lens = torch.as_tensor(q, dtype=torch.int32, device=device)
+            self.last_token_index = torch.as_tensor(last, dtype=torch.int64, device=device)
+        else:
+            # one copy, in the order of the current stream, that the host does not wait for
+            given = [np.asarray(x).astype(np.int32) for x in given] + [np.asarray(q, np.int32)]
+            self.block_tables, self.slot_mapping, self.context_lens, self.q_seq_lens, index = _to_device(
+                given + [np.asarray(last, np.int64).view(np.int32)], device)
+            self.last_token_index = index.view(torch.int64)
+            self.host_lens = (self.context_lens, _version(self.context_lens), given[2].tolist())
         if self.carry is not None and is_prefill:
             self.carry_before.copy_(self.carry)
         if self.ragged and is_prefill:
             self.q_lens_host, self.context_lens_host = q, [int(x) for x in context_lens]
             self.n_long_rows, self.n_single_rows = sum(n > 1 for n in q), sum(n == 1 for n in q)
             self.cu_q_dev = torch.tensor(cu, dtype=torch.int32).to(device)
-        # sequences without new tokens in this step (finished prompts of a chunked prefill, idle serving slots) have
-        # no row of their own: one entry per sequence that has tokens
-        self.last_token_index = torch.as_tensor([c - 1 for c, n in zip(cu[1:], q) if n > 0], dtype=torch.int64,
-                                                device=device)
 
 
 def _write_cache(cache: KVCacheContext, layer: int, k: torch.Tensor, v: Optional[torch.Tensor]):
@@ -228,7 +266,7 @@ class _PrefillPlan:
 
     def __init__(self, cache, rows: int):
         self.key = (cache.context_lens, cache.cu_q, rows, _version(cache.context_lens))
-        lens, cu = cache.context_lens.tolist(), cache.cu_q
+        lens, cu = _host_lens(cache), cache.cu_q
         B = len(lens)
         reach = cache.block_tables.shape[1] * cache.block_size
         news = [cu[b + 1] - cu[b] for b in range(B)] if len(cu) == B + 1 else []
@@ -251,7 +289,7 @@ class _PrefillPlan:
             flat += [x for t in items for x in t]
         at = len(flat)
         flat += list(cu) + gather[False] + gather[True]
-        dev = torch.tensor(flat, dtype=torch.int32).to(cache.block_tables.device)
+        dev, = _to_device([np.asarray(flat, np.int32)], cache.block_tables.device)
         self.fresh, self.past, self.all = ((dev[a:a + 4 * n], n, p) for a, n, p in spans)
         self.cu, self.past_rows, self.all_rows = (dev[at + i * (B + 1):at + (i + 1) * (B + 1)] for i in range(3))
         self.n_past_rows, self.n_all_rows, self.longest = gather[False][-1], gather[True][-1], max(lens)
@@ -268,14 +306,53 @@ def _prefill_plan(cache, rows: int) -> _PrefillPlan:
     return plan
 
 
-def _version(t: torch.Tensor) -> int:
-    """Counts changes in place (tensors made in inference mode keep no count)."""
-    return 0 if t.is_inference() else t._version
-
-
 def _needs_graph(*tensors) -> bool:
     """Whether a derivative is wanted: the kernels of this module have none."""
     return (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)) or torch.autograd.forward_ad._current_level >= 0
+
+
+def _strided(q: torch.Tensor) -> torch.Tensor:
+    """``[T, heads, dim]`` that a tensor map can describe: itself, or a copy."""
+    ok = q.stride(2) == 1 and q.stride(1) >= q.shape[2] and q.stride(0) >= q.shape[2] and q.stride(1) % 8 == 0 and q.stride(0) % 8 == 0 \
+        and q.data_ptr() % 16 == 0
+    return q if ok else q.clone(memory_format=torch.contiguous_format)
+
+
+def _decode_scratch(cache, need: int, device) -> torch.Tensor:
+    """The partial results of decode steps (one buffer per cache)."""
+    scratch = getattr(cache, "_decode_scratch", None)
+    if scratch is None or scratch.numel() * 4 < need:
+        scratch = cache._decode_scratch = torch.empty((need + 3) // 4, dtype=torch.float32, device=device)
+    return scratch
+
+
+def _decode_step(q, k, v, cache, layer: int, scale: float):
+    """One new row per sequence: into the cache and attention over it in one call (bf16 cache of head dim 128: ``paged_decode_tc.cu``, int8
+    cache: ``paged_decode_int8.cu``). None where those kernels do not take the call; nothing was written then."""
+    B, nq, hd = q.shape
+    kc, lens = cache.key_cache[layer], cache.context_lens
+    ksc, vsc = _layer_scales(cache, layer)
+    if not q.is_cuda or not (q.dtype == k.dtype == v.dtype == torch.bfloat16) or B != lens.shape[0] or k.shape != v.shape \
+            or k.shape[0] != B or k.shape[2] != hd or kc.dtype != (torch.bfloat16 if ksc is None else torch.int8):
+        return None
+    out = torch.empty((B, nq * hd), dtype=torch.bfloat16, device=q.device)
+    tables = cache.block_tables
+    need = 0
+    for _ in range(2):
+        scratch = _decode_scratch(cache, need, q.device)
+        rc = _lib.get_lib().mfb_paged_decode_step(
+            q.data_ptr(), *q.stride(), k.data_ptr(), *k.stride(), v.data_ptr(), *v.stride(), kc.data_ptr(),
+            cache.value_cache[layer].data_ptr(), _lib.ptr(ksc), _lib.ptr(vsc), cache.slot_mapping.data_ptr(), tables.data_ptr(),
+            lens.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel() * 4, B, nq, k.shape[1], hd, kc.shape[0],
+            cache.block_size, tables.shape[1], scale, _lib.status_word(q.device).data_ptr(), _lib.stream_ptr())
+        if rc <= 0:
+            break
+        need = rc
+    if rc == -1:
+        return None
+    _lib.check(rc, "mfb_paged_decode_step")
+    _lib.count_launch(3)
+    return out
 
 
 def _rows_ok(t: torch.Tensor) -> bool:
@@ -301,8 +378,7 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
     if plan.past[1] and (kc.dtype != (torch.bfloat16 if ksc is None else torch.int8) or not kc.is_contiguous() or not vc.is_contiguous()
                          or plan.n_past_rows >= 1 << 31):
         return None
-    if q.stride(2) != 1 or q.stride(1) % 8 or q.stride(0) % 8 or q.stride(1) < hd or q.stride(0) < hd or q.data_ptr() % 16:
-        q = q.contiguous()
+    q = _strided(q)
     lib, st, stream = _lib.get_lib(), _lib.status_word(q.device).data_ptr(), _lib.stream_ptr()
     out = torch.empty((plan.rows, nq * hd), dtype=q.dtype, device=q.device)
 
@@ -347,6 +423,10 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
     """q: [T, nq, hd]; k/v: [T, nkv, hd] of the new tokens. Returns [T, nq*hd]."""
     cache: KVCacheContext = meta.cache
     layer = layer_number - 1 - cache.layer_offset
+    if not cache.is_prefill and _DECODE_KERNEL == "tensor_core":
+        out = _decode_step(q, k, v, cache, layer, scale)
+        if out is not None:
+            return out
     _write_cache(cache, layer, k, v)
     T, nq, hd = q.shape
     nkv = k.shape[1]
@@ -354,36 +434,17 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
     if not cache.is_prefill and T == B:
         out = torch.empty((T, nq, hd), dtype=q.dtype, device=q.device)
         if q.is_cuda and q.dtype == torch.bfloat16 and hd in (64, 128) and nq // nkv <= 16:
-            qc = q.contiguous()
             lib = _lib.get_lib()
             max_blocks = cache.block_tables.shape[1]
             ksc, vsc = _layer_scales(cache, layer)
-            if ksc is None and _DECODE_KERNEL == "tensor_core" \
-                    and lib.mfb_paged_decode_tc_supported(nq, nkv, hd, cache.block_size):
-                # bf16 cache, head dim 128: Q K^T and P V on the tensor cores, K / V tiles streamed by TMA
-                splits = lib.mfb_paged_decode_tc_splits(B, nkv, max_blocks * cache.block_size)
-                need = lib.mfb_paged_decode_scratch_bytes(B, nq, hd, splits)
-                scratch = getattr(cache, "_decode_scratch", None)
-                if scratch is None or scratch.numel() * 4 < need:
-                    scratch = cache._decode_scratch = torch.empty((need + 3) // 4, dtype=torch.float32, device=q.device)
-                kc = cache.key_cache[layer]
-                rc = lib.mfb_paged_decode_attention_tc(
-                    qc.data_ptr(), kc.data_ptr(), cache.value_cache[layer].data_ptr(), cache.block_tables.data_ptr(),
-                    cache.context_lens.data_ptr(), out.data_ptr(), scratch.data_ptr(), splits, B, nq, nkv, kc.shape[0],
-                    cache.block_size, max_blocks, float(scale), _lib.status_word(q.device).data_ptr(), _lib.stream_ptr())
-                _lib.check(rc, "mfb_paged_decode_attention_tc")
-                _lib.count_launch(2)
-                return out.view(T, nq * hd)
+            qc = q.contiguous()
             splits = lib.mfb_paged_decode_splits(B, nkv, cache.block_size, max_blocks)
-            need = lib.mfb_paged_decode_scratch_bytes(B, nq, hd, splits)
-            scratch = getattr(cache, "_decode_scratch", None)
-            if scratch is None or scratch.numel() * 4 < need:
-                scratch = cache._decode_scratch = torch.empty((need + 3) // 4, dtype=torch.float32, device=q.device)
             rc = lib.mfb_paged_decode_attention_ex(
                 qc.data_ptr(), cache.key_cache[layer].data_ptr(), cache.value_cache[layer].data_ptr(),
                 _lib.ptr(ksc), _lib.ptr(vsc),
-                cache.block_tables.data_ptr(), cache.context_lens.data_ptr(), out.data_ptr(), scratch.data_ptr(), splits,
-                B, nq, nkv, hd, cache.block_size, max_blocks, float(scale), _lib.stream_ptr())
+                cache.block_tables.data_ptr(), cache.context_lens.data_ptr(), out.data_ptr(),
+                _decode_scratch(cache, lib.mfb_paged_decode_scratch_bytes(B, nq, hd, splits), q.device).data_ptr(), splits, B, nq, nkv, hd,
+                cache.block_size, max_blocks, float(scale), _lib.stream_ptr())
             _lib.check(rc, "mfb_paged_decode_attention_ex")
             _lib.count_launch(2)
             return out.view(T, nq * hd)
@@ -473,10 +534,7 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
     if not plan.ok or n >= 1 << 31:
         return None
     q_pe = q_pe.reshape(T, nh, rope_d)
-    if q_nope.stride(2) != 1 or q_nope.stride(1) % 8 or q_nope.stride(0) % 8 or q_nope.stride(1) < nope or q_nope.stride(0) < nope \
-            or q_nope.data_ptr() % 16:
-        q_nope = q_nope.contiguous()
-    q_pe = q_pe.contiguous()
+    q_nope, q_pe = _strided(q_nope), q_pe.contiguous()
     lib, dev = _lib.get_lib(), q_nope.device
     latent = torch.empty((n, rank + rope_d), dtype=torch.bfloat16, device=dev)
     _gather_rows(cache, latent, rows, None, plan.all_rows, plan.longest)
@@ -523,7 +581,7 @@ def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
         o_lat = mla_decode_attention(q_cat, cache.key_cache[layer], cache.block_tables, cache.context_lens,
                                      cache.block_size, attn.scale, cache)
         return torch.einsum("bhr,hvr->bhv", o_lat, w_uv).reshape(B, nh * vd)
-    lens = cache.context_lens.tolist()
+    lens = _host_lens(cache)
     q_lens = [cache.cu_q[b + 1] - cache.cu_q[b] for b in range(B)]
     if (cache.is_prefill and q_nope.is_cuda and q_nope.dtype == torch.bfloat16 and nope == 128 and rope_d == 64
             and vd == 128 and all(ql == n and ql % 128 == 0 and ql > 0 for ql, n in zip(q_lens, lens))):

@@ -141,6 +141,11 @@ def _declare(lib):
     sig("mfb_quant_act_int8", [P, L, P, L, P, P, L, I, P])
     sig("mfb_paged_decode_tc_supported_ex", [I, I, I, I, I])
     sig("mfb_paged_decode_attention_tc_ex", [P] * 9 + [I] * 13 + [F, F, L, F, P, P])
+    sig("mfb_paged_decode_attention_tc_q", [P, L, L] + [P] * 8 + [I] * 13 + [F, F, L, F, P, P])
+    sig("mfb_paged_decode_step", [P, L, L, L, P, L, L, L, P, L, L, L] + [P] * 9 + [L] + [I] * 7 + [F, P, P], L)
+    sig("mfb_paged_decode_int8_supported", [I, I, I, I])
+    sig("mfb_paged_decode_int8_splits", [I, I, I])
+    sig("mfb_paged_decode_attention_int8", [P, L, L] + [P] * 8 + [I] * 7 + [F, P])
     sig("mfb_paged_prefill_tc_supported", [I, I, I, I, I])
     sig("mfb_paged_prefill_tc_wide_supported", [I, I, I, I, I])
     sig("mfb_paged_prefill_tc", [P, P, P, P, I, I, P, P, P] + [I] * 11 + [L, L, F, F, L, F, P, P])

@@ -248,19 +248,42 @@ __global__ void paged_combine_kernel(const float* __restrict__ part_acc, const f
     row = cu_q[b];
     if (cu_q[b + 1] - cu_q[b] != 1) return;
   }
-  const int d = threadIdx.x;
-  if (d >= hd) return;
+  const int d = threadIdx.x, lane = d & 31;
+  // Bound by latency: the (max, sum) pairs of up to 32 splits are one load per lane, their weights come by shuffle, and the partial
+  // rows of splits that hold anything are read four at a time. A loop of dependent loads over all splits took 7.6 us for
+  // one sequence of 700 tokens in a table of 8192, of which most splits are empty.
   const float sk = sink ? sink[h] * 1.4426950408889634f : -INFINITY;
+  const float* ml = part_ml + bh * splits * 2;
   float mx = sk;
-  for (int s2 = 0; s2 < splits; ++s2) mx = fmaxf(mx, part_ml[(bh * splits + s2) * 2]);
-  float num = 0.f, den = sink ? exp2f(sk - mx) : 0.f;
-  for (int s2 = 0; s2 < splits; ++s2) {
-    const float ms = part_ml[(bh * splits + s2) * 2];
-    const float w = ms == -INFINITY ? 0.f : exp2f(ms - mx);
-    num += w * part_acc[(bh * splits + s2) * hd + d];
-    den += w * part_ml[(bh * splits + s2) * 2 + 1];
+  for (int s0 = 0; s0 < splits; s0 += 32)
+    if (s0 + lane < splits) mx = fmaxf(mx, ml[(s0 + lane) * 2]);
+  mx = warp_max(mx);
+  float num = 0.f, den = 0.f;
+  for (int s0 = 0; s0 < splits; s0 += 32) {
+    float w = 0.f;
+    if (s0 + lane < splits) {
+      const float ms = ml[(s0 + lane) * 2];
+      w = ms == -INFINITY ? 0.f : exp2f(ms - mx);
+      den += w * ml[(s0 + lane) * 2 + 1];
+    }
+    uint32_t used = __ballot_sync(0xffffffffu, w != 0.f);
+    const float* acc = part_acc + (bh * splits + s0) * hd + (d < hd ? d : 0);
+    while (used) {
+      float f[4], x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int at = used ? __ffs(used) - 1 : 0;
+        const float g = __shfl_sync(0xffffffffu, w, at);
+        f[i] = used ? g : 0.f;
+        x[i] = used ? acc[static_cast<size_t>(at) * hd] : 0.f;
+        used &= used - 1;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) num += f[i] * x[i];
+    }
   }
-  out[row * ld_out + (size_t)h * hd + d] = __float2bfloat16(den > 0.f ? out_scale * num / den : 0.f);
+  den = warp_sum(den) + (sink ? exp2f(sk - mx) : 0.f);
+  if (d < hd) out[row * ld_out + (size_t)h * hd + d] = __float2bfloat16(den > 0.f ? out_scale * num / den : 0.f);
 }
 
 // out[t, :] = cache[slot(t), :] gathered through the block table: token i of sequence b for i < lens[b],

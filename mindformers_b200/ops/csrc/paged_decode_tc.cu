@@ -151,7 +151,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const uint32_t qb = smem_u32(q_full);
       mbar_expect_tx(qb, k_halves * (kHeads * 128));
       for (int c = 0; c < k_halves; ++c)
-        tma_load_2d(smem_u32(sQ) + c * (kHeads * 128), &tmQ, qb, c * 64, q_row * args.num_q_heads + head0);
+        tma_load_3d(smem_u32(sQ) + c * (kHeads * 128), &tmQ, qb, c * 64, head0, q_row);
       const int bs = args.block_size;
       const int pages = kTile / bs;               // pages per tile (block_size divides 128)
       const int* table = args.block_tables + static_cast<size_t>(b) * args.max_blocks;
@@ -374,6 +374,22 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   }
 }
 
+// three-dimensional map of q [rows, Hq, D] with rows ld and heads ld_head elements apart: box of one row x 16 heads x 64 columns
+int make_q_map(CUtensorMap* out, const void* q, uint64_t rows, uint64_t Hq, uint64_t D, uint64_t ld, uint64_t ld_head) {
+  mfb_host::EncodeTiledFn enc = mfb_host::get_encode_tiled();
+  if (!enc) { mfb_host::set_error("cuTensorMapEncodeTiled entry point not available"); return 1; }
+  if ((reinterpret_cast<uintptr_t>(q) & 15) || ld % 8 || ld_head % 8) { mfb_host::set_error("paged_decode_tc: q not aligned"); return 2; }
+  cuuint64_t gdim[3] = {D, Hq, rows};
+  cuuint64_t gstride[2] = {ld_head * 2, ld * 2};
+  cuuint32_t box[3] = {64, kHeads, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), gdim, gstride, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { mfb_host::set_error("paged_decode_tc: tensor map of q failed (%d)", (int)r); return 3; }
+  return 0;
+}
+
 }  // namespace pdt
 }  // namespace mfb
 
@@ -418,7 +434,8 @@ int mfb_paged_decode_tc_splits(int B, int Hkv, int max_len) {
 // with one row are computed and written. chunk > 0: keys of the query's own chunk of positions only; window > 0: the last
 // `window` keys only. sink: [Hq] fp32 or null, adds exp(sink) to the softmax denominator. softcap > 0: scores become softcap *
 // tanh(score / softcap). Rows of out lie ld_out elements apart; the result is multiplied by out_scale.
-int mfb_paged_decode_attention_tc_ex(const void* q, const void* key_cache, const void* value_cache, const int* block_tables,
+// Rows and heads of q may lie ld_q and ld_head elements apart (slices of a fused projection).
+int mfb_paged_decode_attention_tc_q(const void* q, long long ld_q, long long ld_head, const void* key_cache, const void* value_cache, const int* block_tables,
                                      const int* context_lens, const int* cu_q, const float* sink, void* out, void* scratch,
                                      int splits, int rows, int B, int Hq, int Hkv, int D, int DV, int num_blocks,
                                      int block_size, int max_blocks, int chunk, int window, int all_values, float scale,
@@ -434,7 +451,7 @@ int mfb_paged_decode_attention_tc_ex(const void* q, const void* key_cache, const
   int rc;
   const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const uint64_t slots = (uint64_t)num_blocks * block_size, kp = (uint64_t)Hkv * D, vp = (uint64_t)Hkv * DV;
-  if ((rc = mfb_host::make_tmap_2d(&tQ, q, 2, BF, (uint64_t)rows * Hq, D, D, pdt::kHeads, 64))) return 20 + rc;
+  if ((rc = pdt::make_q_map(&tQ, q, rows, Hq, D, ld_q, ld_head))) return 20 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tK, key_cache, 2, BF, slots, kp, kp, block_size, 64))) return 30 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tV, value_cache, 2, BF, slots, vp, vp, block_size, 64))) return 40 + rc;
   pdt::Args a;
@@ -461,6 +478,17 @@ int mfb_paged_decode_attention_tc_ex(const void* q, const void* key_cache, const
   if (cudaGetLastError() != cudaSuccess) { mfb_host::set_error("paged_decode_tc: launch failed"); return 11; }
   return mfb_paged_combine_ex(a.part_acc, a.part_ml, out, splits, B * Hq * a.vheads, DV, Hq * a.vheads, cu_q, sink, ld_out,
       out_scale, stream);
+}
+
+// The same for a contiguous q.
+int mfb_paged_decode_attention_tc_ex(const void* q, const void* key_cache, const void* value_cache, const int* block_tables,
+                                     const int* context_lens, const int* cu_q, const float* sink, void* out, void* scratch,
+                                     int splits, int rows, int B, int Hq, int Hkv, int D, int DV, int num_blocks,
+                                     int block_size, int max_blocks, int chunk, int window, int all_values, float scale,
+                                     float softcap, long long ld_out, float out_scale, int* status, cudaStream_t stream) {
+  return mfb_paged_decode_attention_tc_q(q, (long long)Hq * D, D, key_cache, value_cache, block_tables, context_lens, cu_q, sink, out,
+                                         scratch, splits, rows, B, Hq, Hkv, D, DV, num_blocks, block_size, max_blocks, chunk, window,
+                                         all_values, scale, softcap, ld_out, out_scale, status, stream);
 }
 
 // q [B, Hq, 128], caches [num_blocks, block_size, Hkv, 128], out [B, Hq, 128]: one row per sequence, no chunks, no sink.

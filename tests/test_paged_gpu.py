@@ -1,4 +1,4 @@
-"""Prefill attention of ragged batches on the tensor cores, against 64-bit PyTorch."""
+"""Attention over the paged cache on the tensor cores (ragged prefill, decode over int8 rows), against 64-bit PyTorch."""
 import types
 
 import pytest
@@ -89,9 +89,9 @@ def test_ragged_prefill(step, heads, kv, dim, block, int8):
                       for c, s in zip((ctx.key_cache, ctx.value_cache), sc))
         want = _attend(q[rows], kk, vv, dim ** -0.5)
         err = (got[rows].double() - want).norm() / want.norm()
-        # rounding of the result alone: 2^-9 at most, its mean square over a binade 2^-9 / sqrt(3) / 1.44; the weights of
-        # sequences without history are rounded too
-        assert err < (1.9e-3 if n < m else 4e-3), (b, float(err))
+        # rounding of the result alone: at most 2^-9 = 1.95e-3 of every number; the weights of sequences without history
+        # are rounded too
+        assert err < (2e-3 if n < m else 4e-3), (b, float(err))
     assert _lib.read_status() == 0
 
 
@@ -134,5 +134,44 @@ def test_latent_prefill(step, heads, block, share, monkeypatch):
         keys = torch.cat((kv[..., :128], lt[:, None, 512:].expand(m, heads, 64)), -1)
         want = _attend(q[rows], keys, kv[..., 128:], attn.scale)
         err = (got[rows].double() - want).norm() / want.norm()
-        assert err < 1.9e-3, (b, float(err))         # rounding of the result alone
+        assert err < 2e-3, (b, float(err))         # rounding of the result alone
+    assert _lib.read_status() == 0
+
+
+# context lengths at the edges of a warp's 16 tokens and a round's 64, one of many splits, an idle row without blocks
+@pytest.mark.parametrize("heads,kv,dim", [(8, 8, 128), (14, 2, 128), (8, 1, 64), (9, 1, 128), (32, 2, 64), (16, 1, 128)])
+@pytest.mark.parametrize("block,cache", [(16, "int8"), (48, "int8"), (128, "int8"), (24, "int8"), (16, "bf16"), (128, "bf16")])
+def test_decode(heads, kv, dim, block, cache):
+    from mindformers_b200.inference import paged_attention as pa
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(heads)
+    lens = [1, 15, 16, 17, 64, 65, 1000, 3, 5000]
+    idle, B, int8 = 7, len(lens), cache == "int8"
+    tables, blocks = _tables(lens, block)
+    ctx = pa.KVCacheContext(1, blocks, block, kv, dim, torch.bfloat16, DEV, kv_cache_dtype="int8" if int8 else None)
+    if int8:                           # scales of rows that nobody wrote
+        ctx.key_scale[0].fill_(float("nan"))
+        ctx.value_scale[0].fill_(float("inf"))
+    step = dict(block_tables=tables.numpy(), context_lens=lens, device=DEV)
+    ctx.set_step(is_prefill=True, slot_mapping=_slots(tables, block, lens, lens).numpy(), q_seq_lens=lens, **step)
+    rows = torch.randn(2, sum(lens), kv, dim, device=DEV).to(torch.bfloat16) * torch.rand(sum(lens), 1, 1, device=DEV).to(torch.bfloat16)
+    pa._write_cache(ctx, 0, rows[0], rows[1])
+    slots = _slots(tables, block, lens, [1] * B)
+    slots[idle], tables[idle] = -1, -1
+    ctx.set_step(is_prefill=False, slot_mapping=slots.numpy(), q_seq_lens=[1] * B, **step)
+    qkv = torch.randn(B, heads + 2 * kv, dim, device=DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        got = pa.paged_attention_forward(qkv[:, :heads], qkv[:, heads:heads + kv], qkv[:, heads + kv:], types.SimpleNamespace(cache=ctx), 1,
+                                         dim ** -0.5)
+    for b, n in enumerate(lens):
+        if b == idle:
+            assert not got[b].any()
+            continue
+        k, v = (_cached(c[0], tables, b, n, block).double() for c in (ctx.key_cache, ctx.value_cache))
+        if int8:
+            k, v = (x * _cached(s[0], tables, b, n, block).double().unsqueeze(-1) for x, s in ((k, ctx.key_scale), (v, ctx.value_scale)))
+        want = _attend(qkv[b:b + 1, :heads], k, v, dim ** -0.5)[0]
+        err = (got[b].double() - want).norm() / want.norm()
+        # rounding of the result alone; the bf16 cache's kernel rounds the weights as well
+        assert err < (2e-3 if int8 or dim == 64 else 4e-3), (b, float(err))
     assert _lib.read_status() == 0
