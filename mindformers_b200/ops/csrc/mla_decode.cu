@@ -350,26 +350,47 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 // out[b, h, :] = sum_s 2^(m_s - M) o_s / sum_s 2^(m_s - M) l_s
+// Bound by latency: the (max, sum) pairs of up to 32 splits are one load per lane, and the rows of splits that hold anything are read two
+// at a time.
 __global__ void __launch_bounds__(128)
 mla_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out,
                    int splits, int num_heads) {
-  const int h = blockIdx.x, b = blockIdx.y;
+  const int h = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31;
+  const size_t first = static_cast<size_t>(b) * splits * num_heads + h;
+  const float2* ml = reinterpret_cast<const float2*>(part_ml);
   float M = -INFINITY;
-  for (int s = 0; s < splits; ++s) {
-    const float* ml = part_ml + ((static_cast<size_t>(b) * splits + s) * num_heads + h) * 2;
-    if (ml[1] > 0.f) M = fmaxf(M, ml[0]);
-  }
+  for (int s0 = 0; s0 < splits; s0 += 32)
+    if (s0 + lane < splits) {
+      const float2 v = ml[first + static_cast<size_t>(s0 + lane) * num_heads];
+      if (v.y > 0.f) M = fmaxf(M, v.x);
+    }
+  M = warp_max(M);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   float L = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const size_t idx = (static_cast<size_t>(b) * splits + s) * num_heads + h;
-    const float l = part_ml[idx * 2 + 1];
-    if (!(l > 0.f)) continue;
-    const float w = exp2f(part_ml[idx * 2] - M);
-    L += w * l;
-    const float4 v = reinterpret_cast<const float4*>(part_o + idx * kMlaRank)[threadIdx.x];
-    acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z; acc[3] += w * v.w;
+  for (int s0 = 0; s0 < splits; s0 += 32) {
+    float w = 0.f;
+    bool holds = false;
+    if (s0 + lane < splits) {
+      const float2 v = ml[first + static_cast<size_t>(s0 + lane) * num_heads];
+      holds = v.y > 0.f;
+      w = holds ? exp2f(v.x - M) : 0.f;
+      if (holds) L += w * v.y;
+    }
+    uint32_t used = __ballot_sync(0xffffffffu, holds);
+    while (used) {
+      const int a = __ffs(used) - 1;
+      used &= used - 1;
+      const bool two = used != 0;
+      const int c = two ? __ffs(used) - 1 : a;
+      used &= used - 1;
+      const float wa = __shfl_sync(0xffffffffu, w, a), wc = __shfl_sync(0xffffffffu, w, c);
+      const float4 x = reinterpret_cast<const float4*>(part_o + (first + static_cast<size_t>(s0 + a) * num_heads) * kMlaRank)[threadIdx.x];
+      const float4 y = reinterpret_cast<const float4*>(part_o + (first + static_cast<size_t>(s0 + c) * num_heads) * kMlaRank)[threadIdx.x];
+      acc[0] += wa * x.x; acc[1] += wa * x.y; acc[2] += wa * x.z; acc[3] += wa * x.w;
+      if (two) { acc[0] += wc * y.x; acc[1] += wc * y.y; acc[2] += wc * y.z; acc[3] += wc * y.w; }
+    }
   }
+  L = warp_sum(L);
   const float inv = L > 0.f ? 1.f / L : 0.f;
   __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(out + (static_cast<size_t>(b) * num_heads + h) * kMlaRank) + threadIdx.x * 2;
   dst[0] = __floats2bfloat162_rn(acc[0] * inv, acc[1] * inv);
@@ -388,12 +409,21 @@ int mfb_mla_cluster_splits(int B, int num_heads, int max_len);
 int mfb_mla_decode_cluster_launch(const void* q, const void* cache, const int* block_tables, const int* context_lens,
                                   float* part_o, float* part_ml, int splits, int B, int num_heads, int num_blocks,
                                   int block_size, int max_blocks, float scale, int* status, cudaStream_t stream);
+int mfb_mla_decode_heads_splits(int B, int num_heads, int max_len);
+int mfb_mla_decode_heads_launch(const void* q, const void* cache, const int* block_tables, const int* context_lens, float* part_o,
+                                float* part_ml, int splits, int B, int num_heads, int num_blocks, int block_size, int max_blocks,
+                                float scale, int* status, cudaStream_t stream);
+// More than one chunk of 16 heads: heads on the rows (mla_decode_heads.cu), which reads a tile 1.4 times for all of them where this file's
+// kernel reads it twice per chunk: 32 heads, 32 x 2304 / 8 x 4000 / 64 x 1500 tokens 42 / 34 / 56 us against 58 / 38 / 68 us, 128 heads 56 / 36 /
+// 72 us against 146 / 87 / 190 us. With one chunk the scores are not worth computing twice: 16 heads 42 / 30 / 52 us against 44 / 34 / 48 us.
+static bool heads_on_rows(int num_heads) { return num_heads > kMlaHeads; }
 void mfb_mla_decode_set_variant(int v) { g_mla_variant = v == 1 ? 1 : 0; }
 int mfb_mla_decode_get_variant() { return g_mla_variant; }
 
 // Number of sequence splits that fills the GPU for a batch of B sequences of up to max_len tokens.
 int mfb_mla_decode_splits(int B, int num_heads, int max_len) {
   if (g_mla_variant == 1) return mfb_mla_cluster_splits(B, num_heads, max_len);
+  if (heads_on_rows(num_heads)) return mfb_mla_decode_heads_splits(B, num_heads, max_len);
   // cost of a choice = waves of CTAs over the 2 x 148 resident CTAs x (tiles per CTA + about one tile of fixed work per CTA)
   const int chunks = (num_heads + kMlaHeads - 1) / kMlaHeads;
   const int tiles = (max_len + kMlaTile - 1) / kMlaTile;
@@ -422,25 +452,28 @@ int mfb_mla_decode_attention(const void* q, const void* cache, const int* block_
     mfb_host::set_error("mla_decode: unsupported B=%d heads=%d splits=%d block_size=%d", B, num_heads, splits, block_size);
     return 1;
   }
-  CUtensorMap tQ, tC;
   int rc;
-  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  if ((rc = mfb_host::make_tmap_2d(&tQ, q, 2, BF, (uint64_t)B * num_heads, kMlaDim, kMlaDim, kMlaHeads, 64))) return 20 + rc;
-  if ((rc = mfb_host::make_tmap_2d(&tC, cache, 2, BF, (uint64_t)num_blocks * block_size, kMlaDim, kMlaDim, block_size, 64))) return 30 + rc;
   MlaArgs a;
   a.block_tables = block_tables; a.context_lens = context_lens; a.max_blocks = max_blocks; a.block_size = block_size;
   a.num_heads = num_heads; a.splits = splits; a.scale_log2 = scale * 1.4426950408889634f;
   a.part_o = reinterpret_cast<float*>(scratch);
   a.part_ml = a.part_o + static_cast<size_t>(B) * splits * num_heads * kMlaRank;
   a.status = status;
-  if (g_mla_variant == 1) {
-    rc = mfb_mla_decode_cluster_launch(q, cache, block_tables, context_lens, a.part_o, a.part_ml, splits, B, num_heads,
-                                       num_blocks, block_size, max_blocks, scale, status, stream);
+  if (g_mla_variant == 1 || heads_on_rows(num_heads)) {
+    rc = g_mla_variant == 1
+             ? mfb_mla_decode_cluster_launch(q, cache, block_tables, context_lens, a.part_o, a.part_ml, splits, B, num_heads, num_blocks,
+                                             block_size, max_blocks, scale, status, stream)
+             : mfb_mla_decode_heads_launch(q, cache, block_tables, context_lens, a.part_o, a.part_ml, splits, B, num_heads, num_blocks,
+                                           block_size, max_blocks, scale, status, stream);
     if (rc) return rc;
     mla_combine_kernel<<<dim3(num_heads, B), 128, 0, stream>>>(a.part_o, a.part_ml, reinterpret_cast<__nv_bfloat16*>(out),
                                                                 splits, num_heads);
     return cudaGetLastError() == cudaSuccess ? 0 : 12;
   }
+  CUtensorMap tQ, tC;
+  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  if ((rc = mfb_host::make_tmap_2d(&tQ, q, 2, BF, (uint64_t)B * num_heads, kMlaDim, kMlaDim, kMlaHeads, 64))) return 20 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tC, cache, 2, BF, (uint64_t)num_blocks * block_size, kMlaDim, kMlaDim, block_size, 64))) return 30 + rc;
   constexpr int SMEM = kMlaSlots * kMlaUnit + kMlaPBytes + kMlaQBytes + 4 * kMlaHeads * 4 + 18 * 8 + 16 + 1024;
   static bool attr_set = false;
   if (!attr_set) {

@@ -175,3 +175,23 @@ def test_decode(heads, kv, dim, block, cache):
         # rounding of the result alone; the bf16 cache's kernel rounds the weights as well
         assert err < (2e-3 if int8 or dim == 64 else 4e-3), (b, float(err))
     assert _lib.read_status() == 0
+
+
+# heads on the rows of the products: chunks of 32, 64 and 128 rows with and without a remainder; splits with one tile, several and none
+@pytest.mark.parametrize("heads", [17, 32, 40, 64, 100, 128, 130])
+@pytest.mark.parametrize("block", [16, 64, 128])
+def test_latent_decode_heads_on_rows(heads, block):
+    from mindformers_b200.inference import paged_attention as pa
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(heads)
+    lens = [1, 127, 128, 129, 700, 3000]
+    tables, blocks = _tables(lens, block)
+    cache = torch.randn(blocks, block, 1, 576, device=DEV).to(torch.bfloat16)
+    q = torch.randn(len(lens), heads, 576, device=DEV).to(torch.bfloat16)
+    got = pa.mla_decode_attention(q, cache, tables.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), block, 192 ** -0.5)
+    for b, n in enumerate(lens):
+        lat = _cached(cache[:, :, 0], tables, b, n, block).double()
+        want = torch.softmax(q[b].double() @ lat.t() * 192 ** -0.5, -1) @ lat[:, :512]
+        err = (got[b].double() - want).norm() / want.norm()
+        assert err < 4e-3, (b, float(err))           # the weights and the result are rounded, 2^-9 at most each
+    assert _lib.read_status() == 0
