@@ -55,6 +55,9 @@ def _declare(lib):
     sig("mfb_rmsnorm_fwd", [P, P, P, P, P, P, I, I, F, P])
     sig("mfb_rmsnorm_bwd_parts", [I])
     sig("mfb_rmsnorm_bwd", [P, P, P, P, P, P, P, P, I, P, I, I, P])
+    sig("mfb_qk_norm_fwd", [P] * 5 + [I] * 4 + [F, F, P])
+    sig("mfb_qk_norm_bwd_scratch", [I], L)
+    sig("mfb_qk_norm_bwd", [P] * 8 + [I, I, P] + [I] * 4 + [P])
     sig("mfb_headnorm_fwd", [P, P, P, I, I, I, L, F, P])
     sig("mfb_swiglu_fwd", [P, P, L, I, P])
     sig("mfb_swiglu_bwd", [P, P, P, L, I, P])

@@ -19,6 +19,7 @@
 namespace mfb {
 
 constexpr int kNormThreads = 256;
+constexpr int kNarrowH = 1024;   // rows up to here belong to part of a warp, or to one
 constexpr int kMaxVec = 4;  // 4 x 8 bf16 per thread => H <= 8192 stays in registers
 
 __device__ __forceinline__ float block_sum(float v, float* red) {
@@ -365,8 +366,10 @@ colsum_partials_kernel(const float* __restrict__ partial, int parts, int H,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  if (c < H)
+  if (c < H) {
+#pragma unroll 8
     for (int p = warp; p < parts; p += 8) s += partial[(size_t)p * H + c];
+  }
   sm[warp][lane] = s;
   __syncthreads();
   if (warp == 0 && c < H) {
@@ -376,6 +379,238 @@ colsum_partials_kernel(const float* __restrict__ partial, int parts, int H,
     if (dw_f32) dw_f32[c] = accumulate ? dw_f32[c] + t : t;
     if (dw_bf16) dw_bf16[c] = __float2bfloat16(accumulate ? __bfloat162float(dw_bf16[c]) + t : t);
   }
+}
+
+// ---- narrow rows: LPR lanes of a warp per row, NV 16-byte vectors per lane (H <= LPR * NV * 8 <= 1024) ----
+// Heads (128 numbers) and latents (512) would leave most of a 256-thread CTA idle and cost two block barriers per row: 65536 rows of 128
+// numbers took 66 us forward and 130 + 22 us backward (dx, dw) that way, against 12 and 18 us for their bytes. A row's sums are three
+// to five shuffles here and there is no barrier until the end.
+__device__ __forceinline__ float lanes_sum(float v, int lpr) {
+  for (int o = lpr >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <bool HAS_RES, int LPR, int NV>
+__global__ void __launch_bounds__(256)
+rmsnorm_narrow_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* __restrict__ w,
+                          __nv_bfloat16* __restrict__ y, __nv_bfloat16* h_out, float* __restrict__ rstd_out, int T, int H, float eps) {
+  const int nvec = H / 8, lane = threadIdx.x % LPR;
+  const long long step = (long long)gridDim.x * (256 / LPR);
+  bf16x8 wv[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (lane + i * LPR < nvec) wv[i] = reinterpret_cast<const bf16x8*>(w)[lane + i * LPR];
+  // the lanes of a warp leave together: rows past the end compute nothing
+  for (long long r0 = (long long)blockIdx.x * (256 / LPR) + threadIdx.x / 32 * (32 / LPR); r0 < T; r0 += step) {
+    const long long row = r0 + (threadIdx.x % 32) / LPR;
+    bf16x8 a[NV];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = lane + i * LPR;
+      if (row < T && v < nvec) {
+        a[i] = reinterpret_cast<const bf16x8*>(x + row * H)[v];
+        if (HAS_RES) {
+          const bf16x8 b = reinterpret_cast<const bf16x8*>(res + row * H)[v];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 fa = __bfloat1622float2(a[i].v[j]), fb = __bfloat1622float2(b.v[j]);
+            a[i].v[j] = __floats2bfloat162_rn(fa.x + fb.x, fa.y + fb.y);
+          }
+          reinterpret_cast<bf16x8*>(h_out + row * H)[v] = a[i];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(a[i].v[j]);
+          ss += f.x * f.x + f.y * f.y;
+        }
+      }
+    }
+    const float rstd = rsqrtf(lanes_sum(ss, LPR) / (float)H + eps);
+    if (row < T && lane == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = lane + i * LPR;
+      if (row < T && v < nvec) {
+        bf16x8 o;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(a[i].v[j]), fw = __bfloat1622float2(wv[i].v[j]);
+          o.v[j] = __floats2bfloat162_rn(f.x * rstd * fw.x, f.y * rstd * fw.y);
+        }
+        reinterpret_cast<bf16x8*>(y + row * H)[v] = o;
+      }
+    }
+  }
+}
+
+// One row of the backward pass held by LPR lanes: dx from dy, h (and dres), the row's terms of dw into acc.
+template <bool HAS_DRES, int LPR, int NV>
+__device__ __forceinline__ void narrow_bwd_row(bool valid, const __nv_bfloat16* dy, const __nv_bfloat16* h, const __nv_bfloat16* dres,
+                                               __nv_bfloat16* dx, float r, const bf16x8 (&wv)[NV], float (&acc)[NV][8], int lane,
+                                               int nvec, int H) {
+  bf16x8 d[NV], a[NV];
+  float dot = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = lane + i * LPR;
+    if (valid && v < nvec) {
+      d[i] = reinterpret_cast<const bf16x8*>(dy)[v];
+      a[i] = reinterpret_cast<const bf16x8*>(h)[v];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 fd = __bfloat1622float2(d[i].v[j]), fh = __bfloat1622float2(a[i].v[j]), fw = __bfloat1622float2(wv[i].v[j]);
+        dot += fd.x * fw.x * fh.x + fd.y * fw.y * fh.y;
+        acc[i][2 * j] += fd.x * fh.x * r;
+        acc[i][2 * j + 1] += fd.y * fh.y * r;
+      }
+    }
+  }
+  const float c = lanes_sum(dot, LPR) * r * r * r / (float)H;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = lane + i * LPR;
+    if (valid && v < nvec) {
+      bf16x8 o, e;
+      if (HAS_DRES) e = reinterpret_cast<const bf16x8*>(dres)[v];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 fd = __bfloat1622float2(d[i].v[j]), fh = __bfloat1622float2(a[i].v[j]), fw = __bfloat1622float2(wv[i].v[j]);
+        float a0 = fd.x * fw.x * r - fh.x * c, a1 = fd.y * fw.y * r - fh.y * c;
+        if (HAS_DRES) {
+          const float2 f = __bfloat1622float2(e.v[j]);
+          a0 += f.x;
+          a1 += f.y;
+        }
+        o.v[j] = __floats2bfloat162_rn(a0, a1);
+      }
+      reinterpret_cast<bf16x8*>(dx)[v] = o;
+    }
+  }
+}
+// the CTA's sums of acc, in a fixed order, into one row of partial sums
+template <int LPR, int NV>
+__device__ __forceinline__ void narrow_dw_row(const float (&acc)[NV][8], float* __restrict__ out, int lane, int nvec, int H) {
+  constexpr int kSlots = 256 / LPR;
+  __shared__ float sm[kSlots][LPR * 8 + 1];
+  const int slot = threadIdx.x / LPR;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm[slot][lane * 8 + j] = acc[i][j];
+    __syncthreads();
+    for (int c = threadIdx.x; c < LPR * 8; c += 256) {
+      const int col = i * LPR * 8 + c;
+      if (col < H) {
+        float t = 0.f;
+#pragma unroll 4
+        for (int q = 0; q < kSlots; ++q) t += sm[q][c];
+        out[col] = t;
+      }
+    }
+  }
+}
+template <bool HAS_DRES, int LPR, int NV>
+__global__ void __launch_bounds__(256)
+rmsnorm_narrow_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ w,
+                          const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                          float* __restrict__ dw_partial, int T, int H) {
+  const int nvec = H / 8, lane = threadIdx.x % LPR;
+  const long long step = (long long)gridDim.x * (256 / LPR);
+  bf16x8 wv[NV];
+  float acc[NV][8];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    if (lane + i * LPR < nvec) wv[i] = reinterpret_cast<const bf16x8*>(w)[lane + i * LPR];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  }
+#pragma unroll 2
+  for (long long r0 = (long long)blockIdx.x * (256 / LPR) + threadIdx.x / 32 * (32 / LPR); r0 < T; r0 += step) {
+    const long long row = r0 + (threadIdx.x % 32) / LPR;
+    const bool valid = row < T;
+    narrow_bwd_row<HAS_DRES, LPR, NV>(valid, dy + row * H, h + row * H, HAS_DRES ? dres + row * H : nullptr, dx + row * H,
+                                      valid ? rstd[row] : 0.f, wv, acc, lane, nvec, H);
+  }
+  narrow_dw_row<LPR, NV>(acc, dw_partial + (size_t)blockIdx.x * H, lane, nvec, H);
+}
+
+// ---- the query and key heads of a packed [T, nq + 2 nkv, hd] buffer, each kind with its own weight; value heads are copied ----
+// One pass over the buffer in place of a copy of each slice, a norm of each and a concatenation: 2048 tokens of 32 + 2 x 8 heads of 128
+// took 62 us more than this forward and 270 us more backward.
+template <int LPR>
+__global__ void __launch_bounds__(256)
+qk_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
+                   __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int T, int nq, int nkv, int hd, float eps_q, float eps_k) {
+  const int nvec = hd / 8, lane = threadIdx.x % LPR, heads = nq + 2 * nkv;
+  const long long rows = (long long)T * heads, step = (long long)gridDim.x * (256 / LPR);
+  const bool in = lane < nvec;
+  bf16x8 q, k;
+  if (in) {
+    q = reinterpret_cast<const bf16x8*>(wq)[lane];
+    k = reinterpret_cast<const bf16x8*>(wk)[lane];
+  }
+  for (long long r0 = (long long)blockIdx.x * (256 / LPR) + threadIdx.x / 32 * (32 / LPR); r0 < rows; r0 += step) {
+    const long long row = r0 + (threadIdx.x % 32) / LPR;
+    const bool valid = row < rows && in;
+    const long long t = row / heads;
+    const int head = (int)(row - t * heads);
+    bf16x8 a;
+    float ss = 0.f;
+    if (valid) {
+      a = reinterpret_cast<const bf16x8*>(x + row * hd)[lane];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(a.v[j]);
+        ss += f.x * f.x + f.y * f.y;
+      }
+    }
+    const float rstd = rsqrtf(lanes_sum(ss, LPR) / (float)hd + (head < nq ? eps_q : eps_k));
+    if (valid) {
+      bf16x8 o = a;
+      if (head < nq + nkv) {
+        if (lane == 0) rstd_out[t * (nq + nkv) + head] = rstd;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(a.v[j]), fw = __bfloat1622float2(head < nq ? q.v[j] : k.v[j]);
+          o.v[j] = __floats2bfloat162_rn(f.x * rstd * fw.x, f.y * rstd * fw.y);
+        }
+      }
+      reinterpret_cast<bf16x8*>(y + row * hd)[lane] = o;
+    }
+  }
+}
+// CTAs 0 .. ctas_q - 1 take the query rows, the next ctas_k the key rows, each with a row of partial sums of its weight's gradient, the
+// others copy the value rows.
+template <int LPR>
+__global__ void __launch_bounds__(256)
+qk_norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wq,
+                   const __nv_bfloat16* __restrict__ wk, const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
+                   float* __restrict__ dw_partial, int T, int nq, int nkv, int hd, int ctas_q, int ctas_k) {
+  const int nvec = hd / 8, lane = threadIdx.x % LPR, heads = nq + 2 * nkv, bid = blockIdx.x;
+  const int kind = bid < ctas_q ? 0 : bid < ctas_q + ctas_k ? 1 : 2;
+  const int first = kind == 0 ? 0 : kind == 1 ? ctas_q : ctas_q + ctas_k;
+  const int ctas = kind == 0 ? ctas_q : kind == 1 ? ctas_k : gridDim.x - ctas_q - ctas_k;
+  const int n = kind == 0 ? nq : nkv, head0 = kind == 0 ? 0 : kind == 1 ? nq : nq + nkv;
+  const long long rows = (long long)T * n, step = (long long)ctas * (256 / LPR);
+  bf16x8 wv[1];
+  float acc[1][8] = {};
+  if (kind < 2 && lane < nvec) wv[0] = reinterpret_cast<const bf16x8*>(kind == 0 ? wq : wk)[lane];
+#pragma unroll 2
+  for (long long r0 = (long long)(bid - first) * (256 / LPR) + threadIdx.x / 32 * (32 / LPR); r0 < rows; r0 += step) {
+    const long long r = r0 + (threadIdx.x % 32) / LPR;
+    const bool valid = r < rows;
+    const long long t = r / n;
+    const int head = head0 + (int)(r - t * n);
+    const long long at = (t * heads + head) * hd;
+    if (kind == 2) {
+      if (valid && lane < nvec) reinterpret_cast<bf16x8*>(dx + at)[lane] = reinterpret_cast<const bf16x8*>(dy + at)[lane];
+    } else {
+      narrow_bwd_row<false, LPR, 1>(valid, dy + at, x + at, nullptr, dx + at, valid ? rstd[t * (nq + nkv) + head] : 0.f, wv, acc, lane,
+                                    nvec, hd);
+    }
+  }
+  if (kind < 2) narrow_dw_row<LPR, 1>(acc, dw_partial + (size_t)bid * hd, lane, nvec, hd);
 }
 
 // ---- warp-per-row variant for per-head q/k norm: rows are (token, head) with strides ----
@@ -426,6 +661,21 @@ int mfb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void
     mfb_host::set_error("rmsnorm: H=%d above %d is not supported", H, kNormThreads * kMaxVec * 8);
     return 1;
   }
+  if (H <= kNarrowH) {
+    const int per = H <= 64 ? 32 : H <= 128 ? 16 : 8;            // rows of a CTA
+    const int need = (T + per - 1) / per, grid = need < 148 * 8 ? need : 148 * 8;
+#define MFB_RMS_NARROW(RES, LPR, NV)                                                                       \
+  rmsnorm_narrow_fwd_kernel<RES, LPR, NV><<<grid, 256, 0, stream>>>(                                       \
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, T, H, eps)
+#define MFB_RMS_NARROW_H(RES)                                                                              \
+  if (H <= 64) MFB_RMS_NARROW(RES, 8, 1); else if (H <= 128) MFB_RMS_NARROW(RES, 16, 1);                   \
+  else if (H <= 256) MFB_RMS_NARROW(RES, 32, 1); else if (H <= 512) MFB_RMS_NARROW(RES, 32, 2);            \
+  else MFB_RMS_NARROW(RES, 32, 4)
+    if (res) { MFB_RMS_NARROW_H(true); } else { MFB_RMS_NARROW_H(false); }
+#undef MFB_RMS_NARROW_H
+#undef MFB_RMS_NARROW
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  }
   const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;      // vectors per thread: 1..4
   const int cap = 148 * (nv <= 2 ? 8 : 4);
   const int grid = T < cap ? T : cap;
@@ -460,6 +710,22 @@ int mfb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* r
     return 1;
   }
   if (T <= 0) return 0;
+  if (H <= kNarrowH) {
+    const int per = H <= 64 ? 32 : H <= 128 ? 16 : 8;
+    const int need = (T + per - 1) / per, most = mfb_rmsnorm_bwd_parts(T), parts = need < most ? need : most;
+#define MFB_RMS_NARROW(DRES, LPR, NV)                                                                      \
+  rmsnorm_narrow_bwd_kernel<DRES, LPR, NV><<<parts, 256, 0, stream>>>(                                     \
+      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, T, H)
+#define MFB_RMS_NARROW_H(DRES)                                                                             \
+  if (H <= 64) MFB_RMS_NARROW(DRES, 8, 1); else if (H <= 128) MFB_RMS_NARROW(DRES, 16, 1);                 \
+  else if (H <= 256) MFB_RMS_NARROW(DRES, 32, 1); else if (H <= 512) MFB_RMS_NARROW(DRES, 32, 2);          \
+  else MFB_RMS_NARROW(DRES, 32, 4)
+    if (dres) { MFB_RMS_NARROW_H(true); } else { MFB_RMS_NARROW_H(false); }
+#undef MFB_RMS_NARROW_H
+#undef MFB_RMS_NARROW
+    colsum_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(scratch, parts, H, dw_f32, (__nv_bfloat16*)dw_bf16, accumulate);
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  }
   const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;
   const int cap = 148 * (nv <= 2 ? 6 : 3);
   const int grid = T < cap ? T : cap;
@@ -488,6 +754,50 @@ int mfb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* r
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, rstd, scratch, T, H, rows_per_split);
   colsum_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(scratch, parts, H, dw_f32,
                                                            (__nv_bfloat16*)dw_bf16, accumulate);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// packed [T, nq + 2 nkv, hd] -> the same with every query head normalised and times wq, every key head and wk, value heads as they are;
+// rstd [T, nq + nkv]. hd a multiple of 8 up to 256; every address on 16 bytes.
+int mfb_qk_norm_fwd(const void* x, const void* wq, const void* wk, void* y, float* rstd, int T, int nq, int nkv, int hd, float eps_q,
+                    float eps_k, cudaStream_t stream) {
+  if (hd % 8 || hd < 8 || hd > 256 || nq < 1 || nkv < 1) { mfb_host::set_error("qk_norm: hd=%d nq=%d nkv=%d", hd, nq, nkv); return 1; }
+  if (T <= 0) return 0;
+  const int per = hd <= 64 ? 32 : hd <= 128 ? 16 : 8;
+  const long long need = ((long long)T * (nq + 2 * nkv) + per - 1) / per;
+  const unsigned grid = (unsigned)(need < 148 * 8 ? need : 148 * 8);
+#define MFB_QK(LPR)                                                                                                     \
+  qk_norm_fwd_kernel<LPR><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, \
+                                                    (__nv_bfloat16*)y, rstd, T, nq, nkv, hd, eps_q, eps_k)
+  if (hd <= 64) MFB_QK(8); else if (hd <= 128) MFB_QK(16); else MFB_QK(32);
+#undef MFB_QK
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// Floats of scratch that mfb_qk_norm_bwd needs.
+long long mfb_qk_norm_bwd_scratch(int hd) { return 148LL * 6 * hd; }
+
+// Gradients of the above: dx like x, dwq / dwk [hd] fp32 (accumulate: added to).
+int mfb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk, const float* rstd, void* dx, float* dwq, float* dwk,
+                    int acc_q, int acc_k, float* scratch, int T, int nq, int nkv, int hd, cudaStream_t stream) {
+  if (hd % 8 || hd < 8 || hd > 256 || nq < 1 || nkv < 1) { mfb_host::set_error("qk_norm_bwd: hd=%d nq=%d nkv=%d", hd, nq, nkv); return 1; }
+  if (T <= 0) return 0;
+  // up to six CTAs per SM, shared out by rows: a value row costs about half
+  const int per = hd <= 64 ? 32 : hd <= 128 ? 16 : 8;
+  auto share = [&](int heads, double part) {
+    const long long need = ((long long)T * heads + per - 1) / per;
+    const long long most = (long long)(148 * 6 * part);
+    return (int)(need < most ? need : most < 1 ? 1 : most);
+  };
+  const double all = nq + 1.5 * nkv;
+  const int cq = share(nq, nq / all), ck = share(nkv, nkv / all), cv = share(nkv, 0.5 * nkv / all);
+#define MFB_QK(LPR)                                                                                                     \
+  qk_norm_bwd_kernel<LPR><<<cq + ck + cv, 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, \
+                                                            (const __nv_bfloat16*)wk, rstd, (__nv_bfloat16*)dx, scratch, T, nq, nkv, hd, cq, ck)
+  if (hd <= 64) MFB_QK(8); else if (hd <= 128) MFB_QK(16); else MFB_QK(32);
+#undef MFB_QK
+  colsum_partials_kernel<<<(hd + 31) / 32, 256, 0, stream>>>(scratch, cq, hd, dwq, nullptr, acc_q);
+  colsum_partials_kernel<<<(hd + 31) / 32, 256, 0, stream>>>(scratch + (size_t)cq * hd, ck, hd, dwk, nullptr, acc_k);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -406,6 +406,7 @@ class _RMSNormFn(torch.autograd.Function):
         _lib.check(rc, "mfb_rmsnorm_fwd")
         _lib.count_launch()
         ctx.save_for_backward(h, w, rstd)
+        ctx.set_materialize_grads(False)         # an unused residual stream costs no zeros
         ctx.has_res = residual is not None
         ctx.shape = shape
         return y.reshape(shape), h.reshape(shape)
@@ -414,7 +415,7 @@ class _RMSNormFn(torch.autograd.Function):
     def backward(ctx, dy, dh):
         h, w, rstd = ctx.saved_tensors
         T, H = h.shape
-        dy2 = dy.reshape(T, H)
+        dy2 = torch.zeros_like(h) if dy is None else dy.reshape(T, H)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dres = None
@@ -440,6 +441,59 @@ class _RMSNormFn(torch.autograd.Function):
             dw = dw.to(w.dtype)
         dx = dx.reshape(ctx.shape)
         return dx, (dx if ctx.has_res else None), dw, None
+
+
+class _QKNormFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, packed, wq, wk, nq, nkv, eps_q, eps_k):
+        T, _, hd = packed.shape
+        out = torch.empty_like(packed)
+        rstd = torch.empty((T, nq + nkv), dtype=torch.float32, device=packed.device)
+        rc = _lib.get_lib().mfb_qk_norm_fwd(packed.data_ptr(), wq.data_ptr(), wk.data_ptr(), out.data_ptr(), rstd.data_ptr(), T, nq, nkv,
+                                            hd, float(eps_q), float(eps_k), _lib.stream_ptr())
+        _lib.check(rc, "mfb_qk_norm_fwd")
+        _lib.count_launch()
+        ctx.save_for_backward(packed, wq, wk, rstd)
+        ctx.meta = (nq, nkv)
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        packed, wq, wk, rstd = ctx.saved_tensors
+        nq, nkv = ctx.meta
+        T, _, hd = packed.shape
+        dy = dy.contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        lib = _lib.get_lib()
+        dx = torch.empty_like(packed)
+        scratch = _scratch(packed.device, lib.mfb_qk_norm_bwd_scratch(hd))
+        dws, targets = [], []
+        for w in (wq, wk):
+            main_grad = getattr(w, "main_grad", None)
+            dws.append(None if main_grad is not None else torch.empty(hd, dtype=torch.float32, device=dx.device))
+            targets.append(dws[-1] if main_grad is None else main_grad)
+        rc = lib.mfb_qk_norm_bwd(dy.data_ptr(), packed.data_ptr(), wq.data_ptr(), wk.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
+                                 targets[0].data_ptr(), targets[1].data_ptr(), int(dws[0] is None), int(dws[1] is None),
+                                 scratch.data_ptr(), T, nq, nkv, hd, _lib.stream_ptr())
+        _lib.check(rc, "mfb_qk_norm_bwd")
+        _lib.count_launch(3)
+        dwq, dwk = (None if d is None else d.to(w.dtype) for d, w in zip(dws, (wq, wk)))
+        return dx, dwq, dwk, None, None, None, None
+
+
+def qk_norm_supported(packed: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor) -> bool:
+    """Whether ``qk_norm`` takes a packed ``[T, heads, hd]`` buffer and these weights (empty batches stay on the general path)."""
+    hd = packed.shape[-1]
+    return (packed.is_cuda and packed.dtype == wq.dtype == wk.dtype == torch.bfloat16 and packed.dim() == 3 and packed.is_contiguous()
+            and packed.shape[0] > 0 and hd % 8 == 0 and hd <= 256 and wq.shape == wk.shape == (hd,) and wq.is_contiguous()
+            and wk.is_contiguous() and packed.data_ptr() % 16 == wq.data_ptr() % 16 == wk.data_ptr() % 16 == 0)
+
+
+def qk_norm(packed: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, nq: int, nkv: int, eps_q: float, eps_k: float) -> torch.Tensor:
+    """``packed [T, nq + 2 nkv, hd]`` with every query head RMS-normalised and times ``wq``, every key head and ``wk``, and the value heads
+    as they are: one pass in place of two sliced copies, two norms and a concatenation."""
+    return apply_fn(_QKNormFn, packed, wq, wk, nq, nkv, eps_q, eps_k)
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5,

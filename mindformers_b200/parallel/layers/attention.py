@@ -17,6 +17,7 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as _module
 
 from ...ops import functional as Fn
 from .. import parallel_state as ps
@@ -103,6 +104,14 @@ class CoreAttention(nn.Module):
         return o.reshape(T, -1)
 
 
+def _plain_norm(m) -> bool:
+    """An ``RMSNorm`` module that nothing hooks into, so that its arithmetic may run without calling it."""
+    return (type(m) is RMSNorm and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+            and not (_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
+                     or _module._global_backward_pre_hooks))
+
+
 class SelfAttention(nn.Module):
     """GQA self-attention with a fused QKV projection.
 
@@ -160,7 +169,12 @@ class SelfAttention(nn.Module):
     def forward(self, hidden, rotary, meta: AttnMeta):
         qkv, _ = self.linear_qkv(hidden)
         packed, q, k, v = self._split(qkv)
-        if self.q_layernorm is not None:
+        if self.q_layernorm is not None and _plain_norm(self.q_layernorm) and _plain_norm(self.k_layernorm) \
+                and Fn.qk_norm_supported(packed, self.q_layernorm.weight, self.k_layernorm.weight):
+            packed = Fn.qk_norm(packed, self.q_layernorm.weight, self.k_layernorm.weight, self.nq, self.nkv, self.q_layernorm.eps,
+                                self.k_layernorm.eps)
+            q, k, v = packed[:, :self.nq], packed[:, self.nq:self.nq + self.nkv], packed[:, self.nq + self.nkv:]
+        elif self.q_layernorm is not None:
             qn = self.q_layernorm(q)
             kn = self.k_layernorm(k)
             packed = torch.cat((qn, kn, v), dim=1)
