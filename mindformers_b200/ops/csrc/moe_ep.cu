@@ -70,30 +70,41 @@ __device__ bool moe_wait_all(const int* flags, int world, int want, int* status)
 // ---------------------------------------------------------------------------------------------------------------
 // rank of each copy within its expert (stable in copy order) and the per-expert counts
 // ---------------------------------------------------------------------------------------------------------------
+// Every CTA reads all ids, so the reading (from L2) and the barriers of a round bound it: a thread takes four ids per round, which are
+// neighbours, and a round has one barrier. 32768 ids, 128 experts: 33 us with one id per thread and three barriers.
 __global__ void __launch_bounds__(1024)
 moe_rank_kernel(const long long* __restrict__ ids, int n, int* __restrict__ rank_in_e, int* __restrict__ counts) {
   const int e = blockIdx.x;
-  __shared__ int warp_tot[32];
-  __shared__ int running;
-  if (threadIdx.x == 0) running = 0;
-  __syncthreads();
+  __shared__ int warp_tot[2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int base = 0; base < n; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const bool hit = i < n && (int)ids[i] == e;
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) warp_tot[warp] = __popc(m);
-    __syncthreads();
-    int before = 0;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    if (hit) rank_in_e[i] = running + before + __popc(m & ((1u << lane) - 1u));
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int t = 0;
-      for (int w = 0; w < nwarps; ++w) t += warp_tot[w];
-      running += t;
+  int running = 0, turn = 0;
+  for (int base = 0; base < n; base += 4 * blockDim.x, turn ^= 1) {
+    const int i = base + 4 * static_cast<int>(threadIdx.x);
+    bool hit[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) hit[u] = i + u < n && static_cast<int>(ids[i + u]) == e;
+    const int mine = hit[0] + hit[1] + hit[2] + hit[3];
+    int upto = mine;                                   // hits of this lane and those before it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
     }
+    if (lane == 31) warp_tot[turn][warp] = upto;
     __syncthreads();
+    // totals of the other warps; the next round writes the other half of the array
+    const int t = lane < nwarps ? warp_tot[turn][lane] : 0;
+    int before = lane < warp ? t : 0, all = t;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    int rank = running + before + upto - mine;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (hit[u]) rank_in_e[i + u] = rank++;
+    running += all;
   }
   if (threadIdx.x == 0) counts[e] = running;
 }
@@ -121,6 +132,7 @@ moe_plan_kernel(MoePlanArgs a) {
   __shared__ int tot[kMoeMaxExperts];     // copies per global expert over all sources
   __shared__ int mine[kMoeMaxExperts];    // copies from sources before this rank
   __shared__ int seg[kMoeMaxExperts + 1];
+  __shared__ int first[kMoeMaxExperts + 1];   // padded rows of the experts before, over all ranks
   const int e = threadIdx.x;
   int* table_local = a.table_peer[a.rank];
   if (a.world > 1) {
@@ -150,15 +162,26 @@ moe_plan_kernel(MoePlanArgs a) {
   if (e < kMoeMaxRanks)
     a.owner_cap[e] = e >= a.world ? 0 : (a.world > 1 ? moe_ld_acquire_sys(table_local + e * (a.E + 1) + a.E) : a.rows_cap);
   __syncthreads();
-  // padded segment starts per owner rank (every rank computes all of them: they are the senders' bases)
-  if (e < a.world) {
-    int off = 0;
-    for (int le = 0; le < a.E_local; ++le) {
-      const int ge = e * a.E_local + le;
-      seg[ge] = off;
-      off += (tot[ge] + kMoeBlock - 1) / kMoeBlock * kMoeBlock;
+  // padded segment starts per owner rank (every rank computes all of them: they are the senders' bases): a prefix sum over all experts,
+  // counted from the owner's first
+  {
+    const int padded = e < a.E ? (tot[e] + kMoeBlock - 1) / kMoeBlock * kMoeBlock : 0;
+    int upto = padded;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if ((e & 31) >= o) upto += v;
     }
-    if (e == a.rank) {
+    __shared__ int warp_sum_of[kMoeMaxExperts / 32];
+    if ((e & 31) == 31) warp_sum_of[e >> 5] = upto;
+    __syncthreads();
+    for (int w = 0; w < (e >> 5); ++w) upto += warp_sum_of[w];
+    if (e < a.E) first[e + 1] = upto;
+    if (e == 0) first[0] = 0;
+    __syncthreads();
+    if (e < a.E) seg[e] = first[e] - first[e / a.E_local * a.E_local];
+    if (e == 0) {
+      const int off = first[(a.rank + 1) * a.E_local] - first[a.rank * a.E_local];
       seg[a.E] = off;
       // overflow has a word of its own right behind the wait status, so neither can hide the other
       if (off > a.rows_cap && a.status) atomicExch(a.status + 1, 1);
@@ -182,16 +205,14 @@ moe_plan_kernel(MoePlanArgs a) {
     a.group_offsets[a.E_local] = total;
     a.num_blocks[0] = total / kMoeBlock;
   }
-  __syncthreads();
-  for (int b = threadIdx.x; b < a.nblocks_cap; b += blockDim.x) {
-    const int row = b * kMoeBlock;
-    int g = a.E_local - 1;
-    for (int le = 0; le < a.E_local; ++le) {
-      const int ge = a.rank * a.E_local + le;
-      const int end = seg[ge] + (tot[ge] + kMoeBlock - 1) / kMoeBlock * kMoeBlock;
-      if (row < end) { g = le; break; }
-    }
-    a.block_group[b] = g;
+  // every expert names its row blocks; blocks past the last segment go to the last expert
+  const int used = seg[a.E] / kMoeBlock;
+  for (int b = threadIdx.x; b < a.nblocks_cap; b += blockDim.x)
+    if (b >= used) a.block_group[b] = a.E_local - 1;
+  if (e < a.E_local) {
+    const int ge = a.rank * a.E_local + e;
+    const int b0 = seg[ge] / kMoeBlock, b1 = b0 + (tot[ge] + kMoeBlock - 1) / kMoeBlock;
+    for (int b = b0; b < b1 && b < a.nblocks_cap; ++b) a.block_group[b] = e;
   }
 }
 
@@ -263,18 +284,18 @@ moe_scatter_kernel(MoeMoveArgs a, const __nv_bfloat16* __restrict__ x) {
   // padding rows of the local segments start as zero: the weight-gradient GEMM sums over them. Without a plan
   // (inference: rows are independent and padding rows are never gathered) they are left as they are.
   if (a.group_offsets) {
+    // (a segment has less than 128 of them; spread over all warps: with the same few warps clearing every segment's rows the
+    // launch took 108 us for 4096 x 8 rows of 2048 numbers, most of it after the last copy)
     const uint4 z = make_uint4(0, 0, 0, 0);
-    for (int le = 0; le < a.E_local; ++le) {
-      const int first = a.group_offsets[le] + a.seg_fill[le];
-      int last = a.group_offsets[le + 1];
-      if (last > a.rows_cap) last = a.rows_cap;
-      for (long long r = first + gw; r < last; r += nwarps) {
-        uint4* dst = reinterpret_cast<uint4*>(a.buf_peer[a.rank] + r * a.H);
-        for (int v = lane; v < vecs; v += 32) dst[v] = z;
-      }
+    for (long long i = gw; i < (long long)a.E_local * kMoeBlock; i += nwarps) {
+      const int le = (int)(i / kMoeBlock);
+      const long long r = (long long)a.group_offsets[le] + a.seg_fill[le] + i % kMoeBlock;
+      if (r >= a.group_offsets[le + 1] || r >= a.rows_cap) continue;
+      uint4* dst = reinterpret_cast<uint4*>(a.buf_peer[a.rank] + r * a.H);
+      for (int v = lane; v < vecs; v += 32) dst[v] = z;
     }
   }
-  __threadfence_system();
+  if (a.world > 1) __threadfence_system();
 }
 
 struct MoeBarrierArgs {
@@ -308,9 +329,41 @@ moe_gather_kernel(MoeMoveArgs a, __nv_bfloat16* __restrict__ out, const __nv_bfl
   const long long gw = (long long)blockIdx.x * warps_per_cta + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * warps_per_cta;
   const int vecs = a.H >> 3;
-  if (!g) {
-    // forward / inference: one work item = 32 vectors of one token, the k rows are fetched four at a time
-    if (!out) return;
+  if (g) {
+    // one work item = one copy: its row and the token's gradient eight vectors at a time (a warp per token, with a sum over the
+    // warp for every 32 vectors of every copy, took 90 us for 4096 x 8 rows of 2048 numbers)
+    for (long long c = gw; c < (long long)a.T * a.k; c += nwarps) {
+      const long long t = c / a.k;
+      const int row = a.dest_row[c], owner = (int)a.ids[c] / a.E_local;
+      float dot = 0.f;
+      if (row >= 0 && owner >= 0 && owner < a.world) {
+        const uint4* src = reinterpret_cast<const uint4*>(a.buf_peer[owner] + (long long)row * a.H);
+        const uint4* gt = reinterpret_cast<const uint4*>(g + t * a.H);
+        for (int v0 = 0; v0 < vecs; v0 += 256) {
+          uint4 q[8], p[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int v = v0 + u * 32 + lane;
+            if (v < vecs) { q[u] = moe_ld_cg(src + v); p[u] = gt[v]; }
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (v0 + u * 32 + lane < vecs) {
+              const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162*>(&q[u]), *d = reinterpret_cast<const __nv_bfloat162*>(&p[u]);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 f = __bfloat1622float2(h[i]), w = __bfloat1622float2(d[i]);
+                dot += w.x * f.x + w.y * f.y;
+              }
+            }
+        }
+      }
+      dot = warp_sum(dot);
+      if (lane == 0) dots[c] = dot;
+    }
+  }
+  if (out) {
+    // one work item = 32 vectors of one token, the k rows are fetched four at a time
     const int chunks = (vecs + 31) >> 5;
     for (long long item = gw; item < (long long)a.T * chunks; item += nwarps) {
       const long long t = item / chunks;
@@ -357,73 +410,6 @@ moe_gather_kernel(MoeMoveArgs a, __nv_bfloat16* __restrict__ out, const __nv_bfl
         }
       }
       if (v < vecs) {
-        uint4 q;
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) h[i] = __float22bfloat162_rn(make_float2(acc[2 * i], acc[2 * i + 1]));
-        reinterpret_cast<uint4*>(out + t * a.H)[v] = q;
-      }
-    }
-    return;
-  }
-  for (long long t = gw; t < a.T; t += nwarps) {
-    for (int v0 = 0; v0 < vecs; v0 += 32) {
-      const int v = v0 + lane;
-      float acc[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-      float gv[8];
-      if (g && v < vecs) {
-        const uint4 q = reinterpret_cast<const uint4*>(g + t * a.H)[v];
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); gv[2 * i] = f.x; gv[2 * i + 1] = f.y; }
-      }
-      // the k rows of a token sit on up to k peers: four loads in flight before the first is used, since one peer
-      // load takes microseconds to return
-      for (int j0 = 0; j0 < a.k; j0 += 4) {
-        uint4 q4[4];
-        bool have[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          have[u] = false;
-          const int j = j0 + u;
-          if (j < a.k) {
-            const long long c = t * a.k + j;
-            const int row = a.dest_row[c];
-            const int owner = (int)a.ids[c] / a.E_local;
-            if (row >= 0 && owner >= 0 && owner < a.world && v < vecs) {
-              q4[u] = moe_ld_cg(a.buf_peer[owner] + (long long)row * a.H + 8 * v);
-              have[u] = true;
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = j0 + u;
-          if (j >= a.k) break;
-          const long long c = t * a.k + j;
-          float dot = 0.f;
-          if (have[u]) {
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q4[u]);
-            const float w = a.weights ? a.weights[c] : 1.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 f = __bfloat1622float2(h[i]);
-              acc[2 * i] += w * f.x;
-              acc[2 * i + 1] += w * f.y;
-              if (g) dot += gv[2 * i] * f.x + gv[2 * i + 1] * f.y;
-            }
-          }
-          if (g) {
-            dot = warp_sum(dot);
-            if (lane == 0) {
-              if (v0 == 0) dots[c] = dot; else dots[c] += dot;
-            }
-          }
-        }
-      }
-      if (out && v < vecs) {
         uint4 q;
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
 #pragma unroll

@@ -233,10 +233,11 @@ class MoEExchange:
             _lib.count_launch()
 
     def gather(self, st, T, ids, peer_ptrs, weights=None, g=None, own=None, extra=None):
-        """``own [T, H]``: the rows of copies for identity experts; ``extra [T, H]`` (any row pitch) is added to the result."""
-        out = torch.empty(T, self.H, dtype=torch.bfloat16, device=self.dev)
+        """``own [T, H]``: the rows of copies for identity experts; ``extra [T, H]`` (any row pitch) is added to the result. With ``g``
+        the rows' products with it alone: ``(None, dots)``."""
+        out = torch.empty(T, self.H, dtype=torch.bfloat16, device=self.dev) if g is None else None
         dots = torch.empty(T, self.k, dtype=torch.float32, device=self.dev) if g is not None else None
-        rc = self.lib.mfb_moe_gather(self.world, self.rank, T, self.k, self.H, self.E_local, st.rows, out.data_ptr(),
+        rc = self.lib.mfb_moe_gather(self.world, self.rank, T, self.k, self.H, self.E_local, st.rows, _lib.ptr(out),
                                      ids.data_ptr(), st.dest_row.data_ptr(), peer_ptrs, _lib.ptr(weights), _lib.ptr(g),
                                      _lib.ptr(dots), _lib.ptr(own), _lib.ptr(extra), 0 if extra is None else extra.stride(0),
                                      self.status(), _lib.stream_ptr())
