@@ -11,54 +11,81 @@ struct alignas(16) bf16x8 {
 
 __device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
 
-// in: [T, 2F] = [gate | up] ; out: [T, F] = silu(gate) * up
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
-                                  long long T, int F) {
-  const int fv = F / 8;
-  const long long total = T * fv;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / fv;
-    const int c = (int)(i - t * fv);
-    const bf16x8 g = reinterpret_cast<const bf16x8*>(in + t * 2 * F)[c];
-    const bf16x8 u = reinterpret_cast<const bf16x8*>(in + t * 2 * F + F)[c];
-    bf16x8 o;
+// Quotients of vector indexes below 2^31 by a divisor that only the launcher knows: a multiplication and a shift (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994) instead of a 64-bit division per 16 bytes.
+struct FastDiv {
+  uint32_t mul, shift, d;
+  __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
+};
+
+// One vector (eight columns) of a row of [gate | up]: its own function for both, so that all loads of a thread stand before its stores.
+__device__ __forceinline__ bf16x8 swiglu_of(const bf16x8& g, const bf16x8& u) {
+  bf16x8 o;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 fg = __bfloat1622float2(g.v[j]);
-      float2 fu = __bfloat1622float2(u.v[j]);
-      o.v[j] = __floats2bfloat162_rn(silu(fg.x) * fu.x, silu(fg.y) * fu.y);
+  for (int j = 0; j < 4; ++j) {
+    const float2 fg = __bfloat1622float2(g.v[j]), fu = __bfloat1622float2(u.v[j]);
+    o.v[j] = __floats2bfloat162_rn(silu(fg.x) * fu.x, silu(fg.y) * fu.y);
+  }
+  return o;
+}
+__device__ __forceinline__ void swiglu_grad(const bf16x8& g, const bf16x8& u, const bf16x8& d, bf16x8& og, bf16x8& ou) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 fg = __bfloat1622float2(g.v[j]), fu = __bfloat1622float2(u.v[j]), fd = __bfloat1622float2(d.v[j]);
+    const float s0 = 1.f / (1.f + __expf(-fg.x)), s1 = 1.f / (1.f + __expf(-fg.y));
+    og.v[j] = __floats2bfloat162_rn(fd.x * fu.x * s0 * (1.f + fg.x * (1.f - s0)), fd.y * fu.y * s1 * (1.f + fg.y * (1.f - s1)));
+    ou.v[j] = __floats2bfloat162_rn(fd.x * fg.x * s0, fd.y * fg.y * s1);
+  }
+}
+
+// in: [T, 2F] = [gate | up] ; out: [T, F] = silu(gate) * up. Bound by memory: UNROLL vectors per thread, whose loads are all in flight
+// before the first exponential (one at a time, with a 64-bit division each, moved 352 MB in 84 us: 0.64 of the memory's rate).
+template <int UNROLL>
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const bf16x8* __restrict__ in, bf16x8* __restrict__ out, uint32_t total, FastDiv fv) {
+  const uint32_t first = blockIdx.x * (256 * UNROLL) + threadIdx.x;
+  bf16x8 g[UNROLL], u[UNROLL];
+#pragma unroll
+  for (int k = 0; k < UNROLL; ++k) {
+    const uint32_t i = first + k * 256;
+    if (i < total) {
+      const size_t at = static_cast<size_t>(fv(i)) * fv.d + i;         // row r, column c: 2 r F + c
+      g[k] = in[at];
+      u[k] = in[at + fv.d];
     }
-    reinterpret_cast<bf16x8*>(out + t * F)[c] = o;
+  }
+#pragma unroll
+  for (int k = 0; k < UNROLL; ++k) {
+    const uint32_t i = first + k * 256;
+    if (i < total) out[i] = swiglu_of(g[k], u[k]);
   }
 }
 
 // din[T,2F] from dout[T,F] and the saved input.
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dout,
-                                  __nv_bfloat16* __restrict__ din, long long T, int F) {
-  const int fv = F / 8;
-  const long long total = T * fv;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / fv;
-    const int c = (int)(i - t * fv);
-    const bf16x8 g = reinterpret_cast<const bf16x8*>(in + t * 2 * F)[c];
-    const bf16x8 u = reinterpret_cast<const bf16x8*>(in + t * 2 * F + F)[c];
-    const bf16x8 d = reinterpret_cast<const bf16x8*>(dout + t * F)[c];
-    bf16x8 og, ou;
+template <int UNROLL>
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const bf16x8* __restrict__ in, const bf16x8* __restrict__ dout, bf16x8* __restrict__ din, uint32_t total, FastDiv fv) {
+  const uint32_t first = blockIdx.x * (256 * UNROLL) + threadIdx.x;
+  bf16x8 g[UNROLL], u[UNROLL], d[UNROLL];
+  size_t at[UNROLL];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 fg = __bfloat1622float2(g.v[j]);
-      float2 fu = __bfloat1622float2(u.v[j]);
-      float2 fd = __bfloat1622float2(d.v[j]);
-      float s0 = 1.f / (1.f + __expf(-fg.x)), s1 = 1.f / (1.f + __expf(-fg.y));
-      float dg0 = fd.x * fu.x * s0 * (1.f + fg.x * (1.f - s0));
-      float dg1 = fd.y * fu.y * s1 * (1.f + fg.y * (1.f - s1));
-      og.v[j] = __floats2bfloat162_rn(dg0, dg1);
-      ou.v[j] = __floats2bfloat162_rn(fd.x * fg.x * s0, fd.y * fg.y * s1);
+  for (int k = 0; k < UNROLL; ++k) {
+    const uint32_t i = first + k * 256;
+    if (i < total) {
+      at[k] = static_cast<size_t>(fv(i)) * fv.d + i;
+      g[k] = in[at[k]];
+      u[k] = in[at[k] + fv.d];
+      d[k] = dout[i];
     }
-    reinterpret_cast<bf16x8*>(din + t * 2 * F)[c] = og;
-    reinterpret_cast<bf16x8*>(din + t * 2 * F + F)[c] = ou;
+  }
+#pragma unroll
+  for (int k = 0; k < UNROLL; ++k) {
+    if (first + k * 256 < total) {
+      bf16x8 og, ou;
+      swiglu_grad(g[k], u[k], d[k], og, ou);
+      din[at[k]] = og;
+      din[at[k] + fv.d] = ou;
+    }
   }
 }
 
@@ -261,19 +288,38 @@ __global__ void split_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __r
 extern "C" {
 using namespace mfb;
 
+static FastDiv fast_div(uint32_t d) {          // numerators below 2^31
+  FastDiv f;
+  f.d = d;
+  f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = (uint32_t)(((1ull << 32) * ((1ull << f.shift) - d)) / d + 1);
+  return f;
+}
+
+// Rows of a call that keep the vector indexes below 2^31; a larger one is cut.
+static long long swiglu_rows(int F) { const long long n = 0x7fffffffLL / (F / 8) - 256 * 4; return n < 1 ? 1 : n; }
+
 int mfb_swiglu_fwd(const void* in, void* out, long long T, int F, cudaStream_t stream) {
-  if (F % 8) { mfb_host::set_error("swiglu: F=%d must be a multiple of 8", F); return 1; }
-  if (T <= 0) return 0;
-  swiglu_fwd_kernel<<<ew_grid(T * (F / 8), 256), 256, 0, stream>>>((const __nv_bfloat16*)in,
-                                                                   (__nv_bfloat16*)out, T, F);
+  if (F % 8 || F < 8) { mfb_host::set_error("swiglu: F=%d must be a multiple of 8", F); return 1; }
+  const FastDiv fv = fast_div(F / 8);
+  for (long long t = 0; t < T; t += swiglu_rows(F)) {
+    const long long rows = T - t < swiglu_rows(F) ? T - t : swiglu_rows(F);
+    const uint32_t total = (uint32_t)(rows * (F / 8));
+    swiglu_fwd_kernel<4><<<(total + 1023) / 1024, 256, 0, stream>>>((const bf16x8*)in + t * (F / 4), (bf16x8*)out + t * (F / 8), total, fv);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
 int mfb_swiglu_bwd(const void* in, const void* dout, void* din, long long T, int F, cudaStream_t stream) {
-  if (F % 8) { mfb_host::set_error("swiglu: F=%d must be a multiple of 8", F); return 1; }
-  if (T <= 0) return 0;
-  swiglu_bwd_kernel<<<ew_grid(T * (F / 8), 256), 256, 0, stream>>>(
-      (const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, (__nv_bfloat16*)din, T, F);
+  if (F % 8 || F < 8) { mfb_host::set_error("swiglu: F=%d must be a multiple of 8", F); return 1; }
+  const FastDiv fv = fast_div(F / 8);
+  for (long long t = 0; t < T; t += swiglu_rows(F)) {
+    const long long rows = T - t < swiglu_rows(F) ? T - t : swiglu_rows(F);
+    const uint32_t total = (uint32_t)(rows * (F / 8));
+    swiglu_bwd_kernel<2><<<(total + 511) / 512, 256, 0, stream>>>((const bf16x8*)in + t * (F / 4), (const bf16x8*)dout + t * (F / 8),
+                                                                  (bf16x8*)din + t * (F / 4), total, fv);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
