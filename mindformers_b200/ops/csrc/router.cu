@@ -205,6 +205,103 @@ router_bwd_kernel(const float* __restrict__ logits, const long long* __restrict_
   }
 }
 
+// ---- the gate: logits [T, E] fp32 of bf16 rows and fp32 weights -------------------------------------------------------------------
+// A few rows (a decode step): fp32 products on the CUDA cores. Bound by latency, so that the loads of a weight row are spread over four
+// warps, four of them in flight per lane: a CTA has two experts and eight rows, a weight is read once for eight rows. 24 rows, 128 experts,
+// 2048 columns: a conversion of the rows, a library product and its split reduction took 25 us; with a warp per expert 16 us.
+constexpr int kGateRows = 8, kGateParts = 4, kGateExperts = 2;
+__global__ void __launch_bounds__(kGateParts * kGateExperts * 32)
+gate_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ld, const float* __restrict__ w, float* __restrict__ logits, int T, int E,
+                 int H) {
+  __shared__ float part[kGateExperts][kGateParts][kGateRows];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = warp % kGateParts, le = warp / kGateParts;
+  const int e = blockIdx.x * kGateExperts + le, t0 = blockIdx.y * kGateRows;
+  const int n = T - t0 < kGateRows ? T - t0 : kGateRows;
+  const float4* wr = reinterpret_cast<const float4*>(w + (long long)(e < E ? e : 0) * H);
+  float acc[kGateRows] = {};
+#pragma unroll 4
+  for (int v = q * 32 + lane; v < H / 4; v += kGateParts * 32) {
+    const float4 f = __ldg(wr + v);
+#pragma unroll
+    for (int i = 0; i < kGateRows; ++i) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(x + (long long)(t0 + (i < n ? i : 0)) * ld) + v);
+      acc[i] = fmaf(f.x, __uint_as_float(u.x << 16), acc[i]);
+      acc[i] = fmaf(f.y, __uint_as_float(u.x & 0xffff0000u), acc[i]);
+      acc[i] = fmaf(f.z, __uint_as_float(u.y << 16), acc[i]);
+      acc[i] = fmaf(f.w, __uint_as_float(u.y & 0xffff0000u), acc[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kGateRows; ++i) {
+    const float s = warp_sum(acc[i]);
+    if (lane == i) part[le][q][i] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < kGateExperts * kGateRows) {
+    const int k = threadIdx.x / kGateRows, i = threadIdx.x % kGateRows, f = blockIdx.x * kGateExperts + k;
+    if (f < E && i < n) logits[(long long)(t0 + i) * E + f] = (part[k][0][i] + part[k][1][i]) + (part[k][2][i] + part[k][3][i]);
+  }
+}
+
+// Many rows, backward: the products run on the tensor cores with an fp32 operand as the sum of three bf16 numbers, 24 bits, which is all of
+// it. Their accumulators drop what does not fit instead of rounding it, so that a sum over thousands of products is 2e-6 to 4e-6 off where fp32
+// library products are 0.5e-6 off; the weight's gradient is therefore summed over 256 rows at a time (0.24e-6) and the blocks are added
+// here. (The rows' gradient has 6 E products and is rounded to bf16. The logits stay with fp32 products: an error of 2e-6 decides
+// ten times as many ties between experts.) x [R, C] becomes six copies side by side (`across`: [R, 6 C]) or one below the other ([6 R, C]),
+// each a part 0, 1 or 2 as `parts` says.
+struct SplitArgs { int part[6]; };
+__global__ void __launch_bounds__(256)
+split3_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, long long R, int C, int across, SplitArgs a) {
+  const int vecs = C / 8;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < R * vecs; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / vecs;
+    const int c = (int)(i - r * vecs);
+    float f[8];
+    *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(x)[2 * i];
+    *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(x)[2 * i + 1];
+    uint4 p[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      uint32_t h[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        h[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
+        f[2 * j] -= __uint_as_float(h[j] << 16);
+        f[2 * j + 1] -= __uint_as_float(h[j] & 0xffff0000u);
+      }
+      p[k] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const long long at = across ? (r * 6 + k) * vecs + c : (k * R + r) * vecs + c;
+      reinterpret_cast<uint4*>(out)[at] = a.part[k] == 0 ? p[0] : a.part[k] == 1 ? p[1] : p[2];
+    }
+  }
+}
+// out [R, C] = the sum of `groups` times three blocks of x, `group_apart` and `apart` numbers apart, rows ld numbers apart; the third
+// blocks, which hold the smallest numbers, first
+__global__ void __launch_bounds__(256)
+sum3_kernel(const float* __restrict__ x, float* __restrict__ out, long long R, int C, long long ld, long long apart, int groups,
+            long long group_apart) {
+  const int vecs = C / 4;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < R * vecs; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / vecs;
+    const float* p = x + r * ld + (i - r * vecs) * 4;
+    float4 s[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int g = 0; g < groups; ++g)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float4 a = *reinterpret_cast<const float4*>(p + g * group_apart + k * apart);
+        s[k].x += a.x; s[k].y += a.y; s[k].z += a.z; s[k].w += a.w;
+      }
+    reinterpret_cast<float4*>(out)[i] = make_float4((s[2].x + s[1].x) + s[0].x, (s[2].y + s[1].y) + s[0].y, (s[2].z + s[1].z) + s[0].z,
+                                                    (s[2].w + s[1].w) + s[0].w);
+  }
+}
+
 }  // namespace mfb
 
 extern "C" {
@@ -250,6 +347,40 @@ int mfb_router_bwd(const float* logits, const long long* ids, const float* dprob
   if (router_check(T, E, k, 0, 0)) return 1;
   RouterArgs a{T, E, k, sigmoid, norm, 0, 0, scale};
   MFB_ROUTER_DISPATCH(router_bwd_kernel, logits, ids, dprobs, dscores, dlogits, a);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// logits [T, E] = x [T, H] (bf16, rows ld apart) times w [E, H] (fp32) transposed. H and ld multiples of 4; x on 8, w on 16 bytes.
+int mfb_gate_rows(const void* x, long long ld, const float* w, float* logits, int T, int E, int H, cudaStream_t stream) {
+  if (H % 4 || ld % 4 || E < 1 || (reinterpret_cast<uintptr_t>(x) & 7) || (reinterpret_cast<uintptr_t>(w) & 15)) {
+    mfb_host::set_error("gate_rows: E=%d H=%d", E, H);
+    return 1;
+  }
+  if (T <= 0) return 0;
+  gate_rows_kernel<<<dim3((E + kGateExperts - 1) / kGateExperts, (T + kGateRows - 1) / kGateRows), kGateParts * kGateExperts * 32, 0, stream>>>(
+      (const __nv_bfloat16*)x, ld, w, logits, T, E, H);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// parts: six digits 0 .. 2, the first one highest. C a multiple of 8.
+int mfb_split3(const float* x, void* out, long long R, int C, int across, int parts, cudaStream_t stream) {
+  if (C % 8 || R < 0) { mfb_host::set_error("split3: %lld x %d", R, C); return 1; }
+  if (R == 0 || C == 0) return 0;
+  SplitArgs a;
+  for (int k = 5; k >= 0; --k, parts /= 10) a.part[k] = parts % 10;
+  long long blocks = (R * (C / 8) + 255) / 256;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  split3_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, (__nv_bfloat16*)out, R, C, across, a);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+int mfb_sum3(const float* x, float* out, long long R, int C, long long ld, long long apart, int groups, long long group_apart,
+             cudaStream_t stream) {
+  if (C % 4 || ld % 4 || apart % 4 || group_apart % 4 || R < 0) { mfb_host::set_error("sum3: %lld x %d", R, C); return 1; }
+  if (R == 0 || C == 0) return 0;
+  long long blocks = (R * (C / 4) + 255) / 256;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  sum3_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, out, R, C, ld, apart, groups, group_apart);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -7,6 +7,7 @@ which is the library baseline the hand-written tcgen05 kernel is measured agains
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -1010,6 +1011,76 @@ def router_topk_reference(logits, bias, k, sigmoid, norm, scale, groups=0, group
     if norm:
         probs = probs / (probs.sum(-1, keepdim=True) + 1e-20)
     return probs * scale, ids, scores
+
+
+def _split3(x: torch.Tensor, across: bool, parts: int) -> torch.Tensor:
+    R, C = x.shape
+    out = torch.empty((R, 6 * C) if across else (6 * R, C), dtype=torch.bfloat16, device=x.device)
+    _lib.check(_lib.get_lib().mfb_split3(x.data_ptr(), out.data_ptr(), R, C, int(across), parts, _lib.stream_ptr()), "mfb_split3")
+    _lib.count_launch()
+    return out
+
+
+# Up to this many rows the gate runs on the CUDA cores, weight by weight (``gate_rows_kernel``); more are a library product in fp32.
+_GATE_ROWS = 192
+_GATE_CHUNK = 256            # rows that a tensor-core sum of the weight's gradient spans
+
+
+@functools.lru_cache(maxsize=64)
+def _chunk_offsets(T: int, device: int) -> torch.Tensor:
+    """``[0, 256, 512, .., T]`` on the device; the copy has arrived when this returns."""
+    return torch.tensor(list(range(0, T, _GATE_CHUNK)) + [T], dtype=torch.int32).to(torch.device("cuda", device))
+
+
+class _GateFn(torch.autograd.Function):
+    """``x W^T`` for bf16 rows and fp32 weights in 32-bit precision. Backward, an fp32 operand enters the tensor cores as three bf16 parts
+    ``p0 + p1 + p2``; products of parts below 2^-24 of the whole are left out."""
+
+    @staticmethod
+    def forward(ctx, x, w):
+        ctx.save_for_backward(x, w)
+        T, E = x.shape[0], w.shape[0]
+        if T > _GATE_ROWS:
+            return torch.matmul(x.float(), w.t())
+        out = torch.empty((T, E), dtype=torch.float32, device=x.device)
+        rc = _lib.get_lib().mfb_gate_rows(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), T, E, w.shape[1], _lib.stream_ptr())
+        _lib.check(rc, "mfb_gate_rows")
+        _lib.count_launch()
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w = ctx.saved_tensors
+        (T, E), H = dy.shape, w.shape[1]
+        d = _split3(dy.contiguous(), True, 12001)                     # [T, 6 E]: d0 d1 d2 d0 d0 d1
+        dx = dw = None
+        if ctx.needs_input_grad[0]:
+            dx = gemm(d, _split3(w, False, 121), b_mn=True)           # against  w0 w0 w0 w1 w2 w1
+        if ctx.needs_input_grad[1]:
+            if 3 * E % 128:                                           # not whole tiles
+                return dx, torch.matmul(dy.t(), x.float())
+            lib, groups = _lib.get_lib(), -(-T // _GATE_CHUNK)
+            parts = torch.empty((groups * 3 * E, H), dtype=torch.float32, device=x.device)
+            rc = lib.mfb_gemm_bf16(d.data_ptr(), x.data_ptr(), parts.data_ptr(), 3 * E, H, 0, d.stride(0), x.stride(0), H, 1, 1, 1, 2, groups,
+                                   0, 0, _chunk_offsets(T, x.device.index).data_ptr(), T, _lib.status_word(x.device).data_ptr(), 0,
+                                   _lib.stream_ptr())
+            _lib.check(rc, "mfb_gemm_bf16[gate]")
+            dw = torch.empty((E, H), dtype=torch.float32, device=x.device)
+            rc = lib.mfb_sum3(parts.data_ptr(), dw.data_ptr(), E, H, H, E * H, groups, 3 * E * H, _lib.stream_ptr())
+            _lib.check(rc, "mfb_sum3")
+            _lib.count_launch(2)
+        return dx, dw
+
+
+def gate_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    return (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and x.dim() == w.dim() == 2 and x.shape[0] > 0
+            and x.shape[1] == w.shape[1] and w.shape[0] % 8 == 0 and w.shape[1] % 64 == 0 and w.is_contiguous() and _aligned(x) and _aligned(w)
+            and _GEMM_BACKEND == "tcgen05" and not torch.is_autocast_enabled())
+
+
+def gate_logits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """Router logits ``[T, E]`` fp32 of bf16 tokens and fp32 weights, in 32-bit precision (``gate_supported`` says where)."""
+    return apply_fn(_GateFn, x, w)
 
 
 class _RouterFn(torch.autograd.Function):

@@ -63,6 +63,8 @@ class TopKRouter(nn.Module):
         """Logits without their bias, fp32."""
         if self.weight.dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and x.is_cuda and not torch.is_grad_enabled():
             return stream.linear(x, self.weight, out_dtype=torch.float32)
+        if Fn.gate_supported(x, self.weight):
+            return Fn.gate_logits(x, self.weight)
         return F.linear(x.to(self.weight.dtype), self.weight).float()
 
     def _select(self, scores):
