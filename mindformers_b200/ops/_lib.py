@@ -46,6 +46,7 @@ def _declare(lib):
     lib.mfb_last_error.restype = ctypes.c_char_p
     lib.mfb_abi_version.restype = c_int
     sig("mfb_gemm_bf16", [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, P, I, P])
+    sig("mfb_gemm_bf16_grouped_short", [P, P, P] + [I] * 7 + [P] * 6)
     sig("mfb_gemm_bf16_decode_supported", [I, I, I])
     sig("mfb_gemm_bf16_decode", [P, P, P, P, I, I, I, L, L, L, I, P, P])
     sig("mfb_gemm_bf16_decode_ex", [P, P, P, P, I, I, I, L, L, L, I, I, I, F, P, P])

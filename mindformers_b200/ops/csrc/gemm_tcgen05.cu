@@ -39,6 +39,7 @@ struct GemmArgs {
   const int* m_block_group;     // mode 1: [num_m_blocks] expert of each 128-row block
   const int* num_m_blocks_dev;  // mode 1: actual number of row blocks (device scalar)
   const int* group_offsets;     // mode 2: [G+1] padded row offsets (multiples of 128)
+  const int* seg_fill;          // mode 1 on short tiles: [G] rows in use of each expert's segment
   int* status;
 };
 
@@ -104,13 +105,20 @@ __device__ __forceinline__ Tile get_tile(const GemmArgs& g, int tile, int mb_tot
 }
 
 // OUT_MODE: 0 bf16 store, 1 f32 store, 2 f32 reduce-add, 3 bf16 reduce-add
-template <int BN, int STAGES, bool A_MN, bool B_MN, int OUT_MODE>
+// ROWS < 128: mode 1 with few rows in use per expert (a decode step). A tile's product still has 128 rows, but only ROWS of them are loaded
+// and stored, and those past ROWS hold whatever lies behind them in shared memory (rows of a product do not touch each other). An
+// expert's 128-row block is 128 / ROWS tiles, of which those without a row in use are skipped, so weights are read once per ROWS rows in
+// use. The bytes that count are then the weights'; with whole blocks a quarter as much again went for padding rows in and out (24 tokens, 8
+// of 128 experts, 2048 x 1536 and 768 x 2048: both products 185 us for 0.95 GB of weights, 172 us so; with 128 columns per tile, whose boxes
+// are 256 contiguous bytes of a weight row instead of 512, 185 us).
+template <int BN, int STAGES, bool A_MN, bool B_MN, int OUT_MODE, int ROWS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const GemmArgs args) {
-  constexpr int A_BYTES = kBM * kBK * 2;
+  constexpr int A_BYTES = ROWS * kBK * 2;
   constexpr int B_BYTES = BN * kBK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static_assert(ROWS == kBM || (!A_MN && OUT_MODE == 0 && STAGE_BYTES >= kBM * kBK * 2), "short tiles");
   constexpr int TMEM_COLS = 2 * BN;  // two accumulators of BN fp32 columns
   constexpr bool OUT_F32 = (OUT_MODE == 1 || OUT_MODE == 2);
   constexpr int CHUNK_COLS = OUT_F32 ? 32 : 64;  // 128 bytes per row per chunk
@@ -156,8 +164,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  const int n_tiles = total_tiles(args);
-  const int mb_total = (args.mode == 1) ? n_tiles / args.num_n_blocks : args.num_m_blocks;
+  const int whole_tiles = total_tiles(args);
+  const int n_tiles = whole_tiles * (kBM / ROWS);      // the first ROWS rows of every block come first
+  const int mb_total = (args.mode == 1) ? whole_tiles / args.num_n_blocks : args.num_m_blocks;
+  // the tile's coordinates; false: nothing to compute
+  auto tile_at = [&](int tile, Tile& t) {
+    t = get_tile<BN, B_MN>(args, ROWS < kBM ? tile % whole_tiles : tile, mb_total);
+    if (ROWS == kBM) return true;
+    const int first = tile / whole_tiles * ROWS, grp = args.m_block_group[t.a_mn0 / kBM];
+    if (t.a_mn0 + first >= args.group_offsets[grp] + args.seg_fill[grp]) return false;
+    t.a_mn0 += first;
+    t.d_row += first;
+    return true;
+  };
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -166,7 +185,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const Tile t = get_tile<BN, B_MN>(args, tile, mb_total);
+        Tile t;
+        if (!tile_at(tile, t)) continue;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           ok = mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, args.status,
                          kStatusWaitTimeoutProducer);
@@ -203,7 +223,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const Tile t = get_tile<BN, B_MN>(args, tile, mb_total);
+        Tile t;
+        if (!tile_at(tile, t)) continue;
         if (t.k_blocks == 0) continue;  // empty expert: the epilogue writes zeros by itself
         ok = mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1, abort_flag, args.status,
                        kStatusWaitTimeoutMma);
@@ -244,7 +265,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t chunk_counter = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const Tile t = get_tile<BN, B_MN>(args, tile, mb_total);
+      Tile t;
+      if (!tile_at(tile, t)) continue;
       if (t.k_blocks > 0) {
         ok = mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, abort_flag, args.status,
                        kStatusWaitTimeoutEpilogue);
@@ -344,13 +366,13 @@ int num_sms() {
   return g_num_sms;
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, int OUT_MODE>
+template <int BN, int STAGES, bool A_MN, bool B_MN, int OUT_MODE, int ROWS = kBM>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, const GemmArgs& args,
            int max_tiles, int sm_limit, cudaStream_t stream) {
-  constexpr int STAGE_BYTES = kBM * kBK * 2 + BN * kBK * 2;
+  constexpr int STAGE_BYTES = ROWS * kBK * 2 + BN * kBK * 2;
   constexpr int SMEM = STAGES * STAGE_BYTES + 2 * kStagingBytes + (2 * STAGES + 4) * 8 + 16 + 1024;
   static_assert(SMEM <= 232448, "shared memory budget exceeded");
-  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, OUT_MODE>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, OUT_MODE, ROWS>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -464,11 +486,37 @@ int mfb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, in
   args.m_block_group = m_block_group;
   args.num_m_blocks_dev = num_m_blocks_dev;
   args.group_offsets = group_offsets;
+  args.seg_fill = nullptr;
   args.status = status;
   int max_tiles = args.num_m_blocks * args.num_n_blocks * (mode == 2 ? num_groups : 1);
 
   if (bn256) return dispatch<256, 4>(a_mn_major, b_mn_major, out_mode, tA, tB, tD, args, max_tiles, sm_limit, stream);
   return dispatch<128, 6>(a_mn_major, b_mn_major, out_mode, tA, tB, tD, args, max_tiles, sm_limit, stream);
+}
+
+// Mode 1 of the above (B [G, K, N], MN-major; bf16 result) for a few rows per expert: rows of A past an expert's seg_fill are not read, rows
+// of D past it are undefined.
+int mfb_gemm_bf16_grouped_short(const void* A, const void* B, void* D, int rows, int N, int K, int lda, int ldb, int ldd, int num_groups,
+                                const int* m_block_group, const int* num_m_blocks_dev, const int* group_offsets, const int* seg_fill,
+                                int* status, cudaStream_t stream) {
+  constexpr int kShort = 32, BN = 256;
+  if (rows <= 0 || rows % kBM || N <= 0 || K <= 0 || K % kBK || num_groups < 1 || !seg_fill || !group_offsets || !m_block_group) {
+    mfb_host::set_error("gemm grouped_short: rows=%d N=%d K=%d", rows, N, K);
+    return 1;
+  }
+  CUtensorMap tA, tB, tD;
+  int rc;
+  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  if ((rc = mfb_host::make_tmap_2d(&tA, A, 2, BF, rows, K, lda, kShort, kBK))) return 20 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tB, B, 2, BF, (uint64_t)num_groups * K, N, ldb, kBK, 64))) return 30 + rc;
+  if ((rc = mfb_host::make_tmap_2d(&tD, D, 2, BF, rows, N, ldd, kShort, 64))) return 40 + rc;
+  GemmArgs args;
+  args.M = rows; args.N = N; args.K = K;
+  args.num_m_blocks = rows / kBM; args.num_n_blocks = (N + BN - 1) / BN;
+  args.mode = 1; args.num_groups = num_groups; args.group_b_stride = K;
+  args.m_block_group = m_block_group; args.num_m_blocks_dev = num_m_blocks_dev; args.group_offsets = group_offsets;
+  args.seg_fill = seg_fill; args.status = status;
+  return launch<BN, 5, false, true, 0, kShort>(tA, tB, tD, args, args.num_m_blocks * args.num_n_blocks, 0, stream);
 }
 
 }  // extern "C"

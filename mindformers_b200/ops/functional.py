@@ -229,6 +229,11 @@ def _pair_workspace(device) -> torch.Tensor:
     return t
 
 
+# Rows of the (padded) buffer per expert up to which a forward-only product takes tiles of 32 rows: the buffer is as large as the worst
+# routing asks, 127 rows per expert more than there are copies, so that up to about 32 copies per expert are one short tile each.
+GROUPED_SHORT_ROWS_PER_GROUP = 160
+
+
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, block_group: torch.Tensor, num_blocks: torch.Tensor,
                  *, b_mn: bool = False, out: Optional[torch.Tensor] = None, group_offsets: Optional[torch.Tensor] = None,
                  seg_fill: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -266,6 +271,14 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, block_group: torch.Tensor, nu
     lib = _lib.get_lib()
     st = _lib.status_word(a.device)
     b2 = b.reshape(-1, b.shape[-1])
+    if b_mn and seg_fill is not None and group_offsets is not None and R <= GROUPED_SHORT_ROWS_PER_GROUP * G and R % 128 == 0 \
+            and K % 64 == 0 and out.dtype == torch.bfloat16:
+        rc = lib.mfb_gemm_bf16_grouped_short(a.data_ptr(), b2.data_ptr(), out.data_ptr(), R, N, K, a.stride(0), b2.stride(0), out.stride(0),
+                                             G, block_group.data_ptr(), num_blocks.data_ptr(), group_offsets.data_ptr(),
+                                             seg_fill.data_ptr(), st.data_ptr(), _lib.stream_ptr())
+        _lib.check(rc, "mfb_gemm_bf16_grouped_short")
+        _lib.count_launch()
+        return out
     rc = lib.mfb_gemm_bf16(a.data_ptr(), b2.data_ptr(), out.data_ptr(), R, N, K, a.stride(0), b2.stride(0),
                            out.stride(0), 0, int(b_mn), 0, 1, G, block_group.data_ptr(),
                            num_blocks.data_ptr(), 0, R, st.data_ptr(), 0, _lib.stream_ptr())

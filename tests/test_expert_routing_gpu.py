@@ -1,4 +1,5 @@
-"""Stable ranks of token copies within their experts (lists that end inside a thread, a warp and a round); the gate in 32-bit precision."""
+"""Stable ranks of token copies within their experts (lists that end inside a thread, a warp and a round); the gate in 32-bit precision;
+products of a few rows per expert."""
 import pytest
 import torch
 
@@ -42,3 +43,35 @@ def test_gate(T, E, H):
     with torch.no_grad():
         assert torch.equal(Fn.gate_logits(x, w), y)
     assert Fn._lib.read_status() == 0
+
+
+# experts without rows, with one, a whole short tile, one more, a whole block and several blocks; widths short of a tile
+@pytest.mark.parametrize("fills", [[0, 1, 32, 0, 33], [128, 5, 0, 64, 96], [300, 2, 31, 1, 0], [1] * 40])
+@pytest.mark.parametrize("N,K", [(1536, 2048), (200, 64), (136, 768)])
+def test_grouped_short_tiles(fills, N, K):
+    from mindformers_b200.ops import functional as Fn
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(N)
+    G = len(fills)
+    offsets = [0]
+    for n in fills:
+        offsets.append(offsets[-1] + -(-n // 128) * 128)
+    blocks = [g for g in range(G) for _ in range((offsets[g + 1] - offsets[g]) // 128)]
+    R = offsets[-1] + 128
+    a = torch.full((R, K), float("nan"), device=DEV).to(torch.bfloat16)        # padding rows may hold anything
+    b = (torch.randn(G, K, N, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    for g, n in enumerate(fills):
+        a[offsets[g]:offsets[g] + n] = torch.randn(n, K, device=DEV).to(torch.bfloat16)
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    out = torch.empty((R, N), dtype=torch.bfloat16, device=DEV)
+    plan = [dev(v) for v in (blocks + [G - 1], [len(blocks)], offsets, fills)]
+    rc = _lib.get_lib().mfb_gemm_bf16_grouped_short(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), R, N, K, K, N, N, G, *(t.data_ptr() for t in plan),
+        _lib.status_word(DEV).data_ptr(), _lib.stream_ptr())
+    _lib.check(rc, "mfb_gemm_bf16_grouped_short")
+    for g, n in enumerate(fills):
+        if n:
+            rows = slice(offsets[g], offsets[g] + n)
+            want = a[rows].double() @ b[g].double()
+            assert float((out[rows].double() - want).norm() / want.norm()) < 4e-3       # one rounding, at most 2^-8
+    assert _lib.read_status() == 0
