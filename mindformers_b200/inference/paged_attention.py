@@ -376,7 +376,7 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
     kc, vc = cache.key_cache[layer], cache.value_cache[layer]
     ksc, vsc = _layer_scales(cache, layer)
     if plan.past[1] and (kc.dtype != (torch.bfloat16 if ksc is None else torch.int8) or not kc.is_contiguous() or not vc.is_contiguous()
-                         or plan.n_past_rows >= 1 << 31):
+                         or plan.n_past_rows >= 1 << 31 or plan.longest * nkv * hd >= 1 << 34):
         return None
     q = _strided(q)
     lib, st, stream = _lib.get_lib(), _lib.status_word(q.device).data_ptr(), _lib.stream_ptr()
@@ -398,25 +398,29 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
             launch(plan.past, kc.data_ptr(), vc.data_ptr(), row, row, kc.shape[0] * cache.block_size, None, True)
         else:
             copies = torch.empty((2, plan.n_past_rows, row), dtype=q.dtype, device=q.device)
-            _gather_rows(cache, copies[0], kc, ksc, plan.past_rows, plan.longest)
-            _gather_rows(cache, copies[1], vc, vsc, plan.past_rows, plan.longest)
+            _gather_rows(cache, copies, (kc, vc), (ksc, vsc), plan.past_rows, plan.longest)
             launch(plan.past, copies[0].data_ptr(), copies[1].data_ptr(), row, row, plan.n_past_rows, plan.past_rows, True)
     return out
 
 
-def _gather_rows(cache, out, rows, scales, cu, longest: int):
-    """Cached rows of every sequence, one after the other (``cu [B + 1]``), de-quantised where ``scales`` are given."""
+def _gather_rows(cache, outs, rows, scales, cu, longest: int):
+    """Cached rows of every sequence, one after the other (``cu [B + 1]``), out of one or two caches of the same shape; de-quantised where
+    ``scales`` are given."""
     lib, tables = _lib.get_lib(), cache.block_tables
     B, max_blocks = tables.shape
-    heads, dim = rows.shape[2:]
-    if scales is None:
-        rc = lib.mfb_gather_cache(rows.data_ptr(), tables.data_ptr(), cu.data_ptr(), out.data_ptr(), B, longest, cache.block_size,
-                                  max_blocks, heads * dim, _lib.stream_ptr())
-    else:
-        rc = lib.mfb_gather_cache_int8(rows.data_ptr(), scales.data_ptr(), tables.data_ptr(), cu.data_ptr(), out.data_ptr(), B, longest,
+    heads, dim = rows[0].shape[2:]
+    if scales[0] is None:
+        rc = lib.mfb_gather_cache2(rows[0].data_ptr(), rows[1].data_ptr() if len(rows) > 1 else 0, tables.data_ptr(), cu.data_ptr(),
+                                   outs[0].data_ptr(), outs[1].data_ptr() if len(rows) > 1 else 0, B, longest, cache.block_size, max_blocks,
+                                   heads * dim, _lib.stream_ptr())
+        _lib.check(rc, "mfb_gather_cache2")
+        _lib.count_launch()
+        return
+    for out, src, scale in zip(outs, rows, scales):
+        rc = lib.mfb_gather_cache_int8(src.data_ptr(), scale.data_ptr(), tables.data_ptr(), cu.data_ptr(), out.data_ptr(), B, longest,
                                        cache.block_size, max_blocks, heads, dim, _lib.stream_ptr())
-    _lib.check(rc, "mfb_gather_cache")
-    _lib.count_launch()
+        _lib.check(rc, "mfb_gather_cache_int8")
+        _lib.count_launch()
 
 
 def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
@@ -531,13 +535,13 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
         return None
     plan = _prefill_plan(cache, T)
     n = plan.n_all_rows if plan.ok else 0
-    if not plan.ok or n >= 1 << 31:
+    if not plan.ok or n >= 1 << 31 or plan.longest * (rank + rope_d) >= 1 << 34:
         return None
     q_pe = q_pe.reshape(T, nh, rope_d)
-    q_nope, q_pe = _strided(q_nope), q_pe.contiguous()
+    q_nope, q_pe = _strided(q_nope), _strided(q_pe)
     lib, dev = _lib.get_lib(), q_nope.device
     latent = torch.empty((n, rank + rope_d), dtype=torch.bfloat16, device=dev)
-    _gather_rows(cache, latent, rows, None, plan.all_rows, plan.longest)
+    _gather_rows(cache, [latent], [rows], [None], plan.all_rows, plan.longest)
     out = torch.empty((plan.rows, nh * vd), dtype=torch.bfloat16, device=dev)
     w = w.view(nh, nope + vd, rank)
     step = max(1, min(nh, _EXPANDED_BYTES // (n * 256 * 8)))
@@ -548,13 +552,27 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
         rc = lib.mfb_split_f32(kv.data_ptr(), parts[0].data_ptr(), parts[1].data_ptr(), kv.numel(), _lib.stream_ptr())
         _lib.check(rc, "mfb_split_f32")
         rc = lib.mfb_latent_prefill_tc(
-            q_nope.data_ptr() + 2 * h * q_nope.stride(1), q_nope.stride(0), q_nope.stride(1), q_pe.data_ptr() + 2 * h * rope_d,
-            q_pe.stride(0), rope_d, parts[0].data_ptr(), parts[1].data_ptr(), latent.data_ptr() + 2 * rank, rank + rope_d, n,
+            q_nope.data_ptr() + 2 * h * q_nope.stride(1), q_nope.stride(0), q_nope.stride(1), q_pe.data_ptr() + 2 * h * q_pe.stride(1),
+            q_pe.stride(0), q_pe.stride(1), parts[0].data_ptr(), parts[1].data_ptr(), latent.data_ptr() + 2 * rank, rank + rope_d, n,
             plan.all_rows.data_ptr(), plan.all[0].data_ptr(), plan.all[1], out.data_ptr() + 2 * h * vd, out.stride(0), T, heads,
             float(attn.scale), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "mfb_latent_prefill_tc")
         _lib.count_launch(2)
     return out
+
+
+def _write_latents(cache, layer: int, kv_c: torch.Tensor, k_pe: torch.Tensor):
+    """New latents ``[T, rank]`` and rotated key parts ``[T, rope]``, side by side, into the layer's cache."""
+    rows, (T, rank), rope = cache.key_cache[layer], kv_c.shape, k_pe.shape[1]
+    if kv_c.is_cuda and kv_c.dtype == k_pe.dtype == rows.dtype == torch.bfloat16 and rank % 8 == rope % 8 == 0 and T \
+            and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (kv_c, k_pe)) \
+            and rows.is_contiguous() and rows.shape[-1] == rank + rope:
+        rc = _lib.get_lib().mfb_latent_to_cache(kv_c.data_ptr(), kv_c.stride(0), k_pe.data_ptr(), k_pe.stride(0), rows.data_ptr(),
+                                                cache.slot_mapping.data_ptr(), T, rank, rope, _lib.stream_ptr())
+        _lib.check(rc, "mfb_latent_to_cache")
+        _lib.count_launch()
+        return
+    _write_cache(cache, layer, torch.cat((kv_c, k_pe), dim=-1).unsqueeze(1).contiguous(), None)
 
 
 def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
@@ -567,8 +585,7 @@ def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
     cache: KVCacheContext = meta.cache
     layer = attn.layer_number - 1 - cache.layer_offset
     T = q_nope.shape[0]
-    latent = torch.cat((kv_c, k_pe.reshape(T, -1)), dim=-1).unsqueeze(1)     # [T, 1, rank + rope]
-    _write_cache(cache, layer, latent.contiguous(), None)
+    _write_latents(cache, layer, kv_c, k_pe.reshape(T, -1))
     nh, nope, rope_d, vd, rank = attn.nh, attn.nope, attn.rope_d, attn.vd, attn.kv_rank
     w = attn.linear_kvb.weight.view(nh, nope + vd, rank)
     w_uk, w_uv = w[:, :nope], w[:, nope:]                                      # [nh, nope, rank], [nh, vd, rank]

@@ -100,6 +100,8 @@ def _declare(lib):
     sig("mfb_mla_decode_set_variant", [I], None)
     sig("mfb_mla_decode_get_variant", [])
     sig("mfb_mla_decode_scratch_bytes", [I, I, I], L)
+    sig("mfb_gather_cache2", [P, P, P, P, P, P, I, I, I, I, I, P])
+    sig("mfb_latent_to_cache", [P, L, P, L, P, P, L, I, I, P])
     sig("mfb_gather_cache", [P, P, P, P, I, I, I, I, I, P])
     sig("mfb_ll_allreduce_buffer_bytes", [I, L], L)
     sig("mfb_ll_allreduce_state_words", [])

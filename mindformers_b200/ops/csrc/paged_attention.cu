@@ -42,6 +42,17 @@ __global__ void reshape_and_cache_kernel(const __nv_bfloat16* __restrict__ key, 
   }
 }
 
+// a row of the latent cache from its two parts; slot_mapping[t] < 0 skips the token
+__global__ void latent_to_cache_kernel(const uint4* __restrict__ latent, long long ld_c, const uint4* __restrict__ pe, long long ld_p,
+                                       uint4* __restrict__ cache, const int* __restrict__ slot_mapping, long long T, int rank, int rope) {
+  const int vecs = rank + rope;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < T * vecs; i += (long long)gridDim.x * blockDim.x) {
+    const long long t = i / vecs;
+    const int c = (int)(i - t * vecs), slot = slot_mapping[t];
+    if (slot >= 0) cache[(long long)slot * vecs + c] = c < rank ? latent[t * ld_c + c] : pe[t * ld_p + c - rank];
+  }
+}
+
 // One warp per (token, head): scale = absmax / 127, codes = round(x / scale).
 __global__ void reshape_and_cache_int8_kernel(const __nv_bfloat16* __restrict__ key, const __nv_bfloat16* __restrict__ value,
                                               int8_t* __restrict__ key_cache, int8_t* __restrict__ value_cache,
@@ -288,15 +299,19 @@ __global__ void paged_combine_kernel(const float* __restrict__ part_acc, const f
 
 // out[t, :] = cache[slot(t), :] gathered through the block table: token i of sequence b for i < lens[b],
 // written at row cu[b] + i. Used to materialise a contiguous K/V (or MLA latent) for prefill with history.
-__global__ void gather_cache_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_tables,
-                                    const int* __restrict__ cu_lens, __nv_bfloat16* __restrict__ out, int B,
-                                    int block_size, int max_blocks, int row_elems) {
+// blockIdx.z: one of two caches with the same tables. The index arithmetic is 32 bits wide and done once per 16 bytes.
+__global__ void gather_cache_kernel(const __nv_bfloat16* __restrict__ cache0, const __nv_bfloat16* __restrict__ cache1,
+                                    const int* __restrict__ block_tables, const int* __restrict__ cu_lens,
+                                    __nv_bfloat16* __restrict__ out0, __nv_bfloat16* __restrict__ out1, int block_size, int max_blocks,
+                                    int row_elems) {
+  const __nv_bfloat16* cache = blockIdx.z ? cache1 : cache0;
+  __nv_bfloat16* out = blockIdx.z ? out1 : out0;
   const int b = blockIdx.y;
   const int start = cu_lens[b], n = cu_lens[b + 1] - start;
   const int vecs = row_elems / 8;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)n * vecs;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int tok = (int)(i / vecs), c = (int)(i - (long long)tok * vecs);
+  const uint32_t total = (uint32_t)n * (uint32_t)vecs;               // the launcher keeps it below 2^31
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int tok = (int)(i / (uint32_t)vecs), c = (int)(i - (uint32_t)tok * vecs);
     const int blk = max(block_tables[(size_t)b * max_blocks + tok / block_size], 0);   // none: any block, as in the decode kernels
     const uint4 v = *reinterpret_cast<const uint4*>(cache + ((size_t)blk * block_size + tok % block_size) * row_elems + c * 8);
     *reinterpret_cast<uint4*>(out + (size_t)(start + tok) * row_elems + c * 8) = v;
@@ -431,15 +446,38 @@ int mfb_paged_decode_attention(const void* q, const void* key_cache, const void*
                                        scratch, splits, B, Hq, Hkv, hd, block_size, max_blocks, scale, stream);
 }
 
-int mfb_gather_cache(const void* cache, const int* block_tables, const int* cu_lens, void* out, int B, int max_len,
-                     int block_size, int max_blocks, int row_elems, cudaStream_t stream) {
+// Cached rows of every sequence, one after the other: token i of sequence b at row cu_lens[b] + i, at most max_len of them; a second cache
+// (or null) into a second copy.
+int mfb_gather_cache2(const void* cache0, const void* cache1, const int* block_tables, const int* cu_lens, void* out0, void* out1, int B,
+                      int max_len, int block_size, int max_blocks, int row_elems, cudaStream_t stream) {
   if (row_elems % 8) { mfb_host::set_error("gather_cache: row of %d elements is not a multiple of 8", row_elems); return 1; }
   if (B <= 0 || max_len <= 0) return 0;
+  if ((long long)max_len * (row_elems / 8) >= 1LL << 31) { mfb_host::set_error("gather_cache: %d rows of %d elements", max_len, row_elems); return 1; }
   long long per = ((long long)max_len * (row_elems / 8) + 255) / 256;
   if (per > 1024) per = 1024;
-  dim3 grid((unsigned)per, B);
-  gather_cache_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)cache, block_tables, cu_lens, (__nv_bfloat16*)out, B,
-                                                block_size, max_blocks, row_elems);
+  gather_cache_kernel<<<dim3((unsigned)per, B, cache1 ? 2 : 1), 256, 0, stream>>>(
+      (const __nv_bfloat16*)cache0, (const __nv_bfloat16*)cache1, block_tables, cu_lens, (__nv_bfloat16*)out0, (__nv_bfloat16*)out1,
+      block_size, max_blocks, row_elems);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+int mfb_gather_cache(const void* cache, const int* block_tables, const int* cu_lens, void* out, int B, int max_len,
+                     int block_size, int max_blocks, int row_elems, cudaStream_t stream) {
+  return mfb_gather_cache2(cache, nullptr, block_tables, cu_lens, out, nullptr, B, max_len, block_size, max_blocks, row_elems, stream);
+}
+
+// Latents [T, rank] and rotated key parts [T, rope] (rows ld_c / ld_p elements apart) side by side into cache rows of rank + rope.
+int mfb_latent_to_cache(const void* latent, long long ld_c, const void* pe, long long ld_p, void* cache, const int* slot_mapping,
+                        long long T, int rank, int rope, cudaStream_t stream) {
+  if (rank % 8 || rope % 8 || ld_c % 8 || ld_p % 8 || ((reinterpret_cast<uintptr_t>(latent) | reinterpret_cast<uintptr_t>(pe)) & 15)) {
+    mfb_host::set_error("latent_to_cache: %d + %d columns, rows %lld and %lld apart", rank, rope, ld_c, ld_p);
+    return 1;
+  }
+  if (T <= 0) return 0;
+  long long blocks = (T * ((rank + rope) / 8) + 255) / 256;
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  latent_to_cache_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const uint4*)latent, ld_c / 8, (const uint4*)pe, ld_p / 8, (uint4*)cache,
+                                                               slot_mapping, T, rank / 8, rope / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

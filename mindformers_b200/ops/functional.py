@@ -645,6 +645,21 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: torch
     return rope_reference(x, cos, sin, positions, n_heads, rot, interleaved)
 
 
+def rope_heads_supported(x: torch.Tensor, rot: int) -> bool:
+    """``[T, heads, hd]`` with heads side by side (rows may lie further apart) that ``rope_heads_`` rotates in place."""
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 3 and x.stride(2) == 1 and (x.shape[1] == 1 or x.stride(1) == x.shape[2])
+            and x.shape[0] > 0 and rot <= x.shape[2] and (x.shape[0] == 1 or x.stride(0) >= x.shape[1] * x.shape[2]))
+
+
+def rope_heads_(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions32: torch.Tensor, rot: int, interleaved: bool):
+    """Rotates the last ``rot`` columns of every head of ``x`` in place (no gradient); ``positions32`` int32."""
+    T, heads, hd = x.shape
+    rc = _lib.get_lib().mfb_rope(x.data_ptr() + 2 * (hd - rot), cos.data_ptr(), sin.data_ptr(), positions32.data_ptr(), T, heads, hd, rot,
+                                 x.stride(0), int(interleaved), 0, cos.shape[0], _lib.stream_ptr())
+    _lib.check(rc, "mfb_rope")
+    _lib.count_launch()
+
+
 # =================================================================================================
 # Embedding
 # =================================================================================================
