@@ -391,12 +391,14 @@ int mfb_paged_decode_int8_supported(int Hq, int Hkv, int hd, int block_size) {
   return (hd == 64 || hd == 128) && Hkv >= 1 && Hq >= 1 && Hq % Hkv == 0 && Hq / Hkv <= 16 && block_size >= 16 && block_size % 16 == 0;
 }
 
-// Ranges per sequence. The lengths are on the device, so the number follows from what the tables could hold: three waves of the 4 x 148
-// resident CTAs even out sequences of different lengths; a sequence shorter than that uses 64-token ranges and leaves the rest empty.
+// Ranges per sequence. The lengths are on the device, so the number follows from what the tables could hold: two waves of the 4 x 148
+// resident CTAs even out sequences of different lengths (64 x 2048 - 4096 tokens, 8 KV heads: 157 us with one range per sequence, 142 to 148 us
+// with two to eight), and no range is shorter than 512 tokens if the tables are full (100 x 150 - 300 tokens, 4 KV heads, tables of 8192: 28, 32
+// and 36 us with 1, 3 and 5). A sequence shorter than that uses 64-token ranges and leaves the rest empty.
 int mfb_paged_decode_int8_splits(int B, int Hkv, int max_len) {
   const long long pairs = (long long)B * Hkv;
-  long long s = (3 * 4 * 148 + pairs - 1) / pairs;
-  const long long most = ((long long)max_len + 255) / 256;
+  long long s = (2 * 4 * 148 + pairs - 1) / pairs;
+  const long long most = ((long long)max_len + 511) / 512;
   if (s > most) s = most;
   if (s > 64) s = 64;
   return s < 1 ? 1 : (int)s;

@@ -146,45 +146,43 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const uint32_t tmem_S = tmem_base + 32;         // 2 buffers of 16 columns, 32 apart
 
   if (warp == 0) {
-    // ------------------------------------ producer ------------------------------------
-    if (lane == 0 && n_tiles > 0) {
+    // ------------------------------------ producer (the whole warp, one lane issues) ------------------------------------
+    if (n_tiles > 0) {
+      const bool leader = elect_one();
       const uint32_t qb = smem_u32(q_full);
-      mbar_expect_tx(qb, k_halves * (kHeads * 128));
-      for (int c = 0; c < k_halves; ++c)
-        tma_load_3d(smem_u32(sQ) + c * (kHeads * 128), &tmQ, qb, c * 64, head0, q_row);
+      if (leader) {
+        mbar_expect_tx(qb, k_halves * (kHeads * 128));
+        for (int c = 0; c < k_halves; ++c)
+          tma_load_3d(smem_u32(sQ) + c * (kHeads * 128), &tmQ, qb, c * 64, head0, q_row);
+      }
+      __syncwarp();
       const int bs = args.block_size;
-      const int pages = kTile / bs;               // pages per tile (block_size divides 128)
       const int* table = args.block_tables + static_cast<size_t>(b) * args.max_blocks;
       uint32_t unit = 0;
       bool ok = true;
-      // one K or V tile into the next ring slot
-      auto load_tile = [&](const CUtensorMap* tm, int j, int col0, int halves) {
+      // one K or V tile into the next ring slot; its pages were looked up a tile earlier
+      auto load_tile = [&](const CUtensorMap* tm, int page, int col0, int halves) {
         const int slot = unit % kSlots;
-        const uint32_t ph = (unit / kSlots) & 1;
-        ok = mbar_wait(smem_u32(&empty[slot]), ph ^ 1, abort_flag, args.status, kStatusWaitTimeoutProducer);
+        ok = mbar_wait(smem_u32(&empty[slot]), ((unit / kSlots) & 1) ^ 1, abort_flag, args.status, kStatusWaitTimeoutProducer);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) return;
-        const int tok0 = (t0 + j) * kTile;
-        const int first_page = table[tok0 / bs];
-        const uint32_t fb = smem_u32(&full[slot]);
-        const uint32_t dst = smem_u32(sRing + slot * kUnit);
-        mbar_expect_tx(fb, halves * kSub);
-        for (int i = 0; i < pages; ++i) {
-          // pages past the end of the sequence may be unallocated: read the tile's first page instead (masked)
-          int pg = (tok0 + i * bs < len) ? table[tok0 / bs + i] : first_page;
-          if (pg < 0) pg = first_page;
-          tma_load_2d(dst + i * bs * 128, tm, fb, col0, pg * bs);
-          if (halves > 1) tma_load_2d(dst + kSub + i * bs * 128, tm, fb, col0 + 64, pg * bs);
-        }
+        if (leader) mbar_expect_tx(smem_u32(&full[slot]), halves * kSub);
+        __syncwarp();
+        tma_load_pages(leader, smem_u32(sRing + slot * kUnit), kSub, tm, smem_u32(&full[slot]), page, bs, col0, halves);
         ++unit;
       };
       const int kcol = kvh * args.D, vcol = (args.vheads > 1 ? vsel : kvh) * args.DV;
-      load_tile(&tmK, 0, kcol, k_halves);
+      int page = tile_page(table, bs, t0 * kTile, len);
+      int next = n_tiles > 1 ? tile_page(table, bs, (t0 + 1) * kTile, len) : 0;
+      load_tile(&tmK, page, kcol, k_halves);
       for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) load_tile(&tmK, j + 1, kcol, k_halves);
-        if (ok) load_tile(&tmV, j, vcol, v_halves);
+        const int after = j + 2 < n_tiles ? tile_page(table, bs, (t0 + j + 2) * kTile, len) : 0;
+        if (j + 1 < n_tiles) load_tile(&tmK, next, kcol, k_halves);
+        if (ok) load_tile(&tmV, page, vcol, v_halves);
+        page = next;
+        next = after;
       }
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------ MMA issuer ------------------------------------
     if (lane == 0 && n_tiles > 0) {
@@ -415,14 +413,17 @@ int mfb_paged_decode_tc_supported(int Hq, int Hkv, int hd, int block_size) {
 
 // Number of sequence splits that fills the GPU for B sequences of up to max_len tokens.
 int mfb_paged_decode_tc_splits(int B, int Hkv, int max_len) {
-  // cost of a choice = waves of CTAs over the 2 x 148 resident CTAs x (tiles per CTA + about one tile of fixed work)
+  // cost of a choice = waves of CTAs over the 2 x 148 resident CTAs x (tiles per CTA + a fixed part). Setting a CTA up and writing its partial
+  // result take about as long as three tiles, and sequences are seldom as long as their tables, so that a range holds fewer tiles than
+  // max_len says: a fixed part of eight. 64 sequences, 8 KV heads, tables of 8192: 163 us with one range and 181 us with four for 2048 - 4096
+  // tokens, 62 and 83 us for 500 - 1000; 8 sequences of 2000 - 4000 tokens, tables of 32768: 40 us with four ranges, 46 us with nine.
   const int tiles = (max_len + pdt::kTile - 1) / pdt::kTile;
   int best = 1;
   long long best_cost = -1;
   for (int s = 1; s <= tiles && s <= 32; ++s) {
     const long long ctas = static_cast<long long>(B) * Hkv * s;
     const long long waves = (ctas + 295) / 296;
-    const long long cost = waves * ((tiles + s - 1) / s + 1);
+    const long long cost = waves * ((tiles + s - 1) / s + 8);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
   }
   return best;
