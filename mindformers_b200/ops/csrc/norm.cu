@@ -382,9 +382,9 @@ colsum_partials_kernel(const float* __restrict__ partial, int parts, int H,
 }
 
 // ---- narrow rows: LPR lanes of a warp per row, NV 16-byte vectors per lane (H <= LPR * NV * 8 <= 1024) ----
-// Heads (128 numbers) and latents (512) would leave most of a 256-thread CTA idle and cost two block barriers per row: 65536 rows of 128
-// numbers took 66 us forward and 130 + 22 us backward (dx, dw) that way, against 12 and 18 us for their bytes. A row's sums are three
-// to five shuffles here and there is no barrier until the end.
+// Heads (128 numbers) and latents (512) would leave most of a 256-thread CTA idle and cost two block barriers per row: 65536 + 16384 rows of 128
+// numbers took 78 us forward and 149 + 27 us backward (dx, dw) that way, of which their bytes need 6 and 10 us. A row's sums are three to five
+// shuffles here and there is no barrier until the end.
 __device__ __forceinline__ float lanes_sum(float v, int lpr) {
   for (int o = lpr >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -536,8 +536,8 @@ rmsnorm_narrow_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloa
 }
 
 // ---- the query and key heads of a packed [T, nq + 2 nkv, hd] buffer, each kind with its own weight; value heads are copied ----
-// One pass over the buffer in place of a copy of each slice, a norm of each and a concatenation: 2048 tokens of 32 + 2 x 8 heads of 128
-// took 62 us more than this forward and 270 us more backward.
+// One pass over the buffer in place of a copy of each slice, a norm of each and a concatenation, and their counterparts backward: 2048 tokens
+// of 32 + 2 x 8 heads of 128, forward and backward together, 430 us; 15 + 22 us here.
 template <int LPR>
 __global__ void __launch_bounds__(256)
 qk_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
