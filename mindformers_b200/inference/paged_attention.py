@@ -22,11 +22,6 @@ from ..ops import _lib
 from ..ops import functional as Fn
 
 
-def _version(t: torch.Tensor) -> int:
-    """Counts changes in place (tensors made in inference mode keep no count)."""
-    return 0 if t.is_inference() else t._version
-
-
 def _to_device(arrays, device):
     """int32 arrays as device tensors, each on 16 bytes, through one pinned buffer and one copy in stream order."""
     at, spans = 0, []
@@ -42,11 +37,9 @@ def _to_device(arrays, device):
 
 
 def _host_lens(cache) -> list:
-    """The step's context lengths on the host: those ``set_step`` was given, unless the device tensor was replaced or changed since."""
-    known = getattr(cache, "host_lens", None)
-    if known is not None and known[0] is cache.context_lens and known[1] == _version(cache.context_lens):
-        return known[2]
-    return cache.context_lens.tolist()
+    """The step's context lengths on the host: those ``set_step`` was given, or a read of the device once somebody else may have changed
+    them (``KVCacheContext.context_lens``)."""
+    return cache.host_lens if cache.host_lens is not None else cache._lens.tolist()
 
 
 class KVCacheContext:
@@ -116,16 +109,27 @@ class KVCacheContext:
         self.is_prefill = True
         self.block_tables = None      # int32 [B, max_blocks]
         self.slot_mapping = None      # int32 [T]
-        self.context_lens = None      # int32 [B] tokens in cache after this step
+        self._lens = None             # context_lens: int32 [B] tokens in cache after this step
         self.q_seq_lens = None        # int32 [B] new tokens of each sequence in this step
         self.last_token_index = None  # int64 [B] row of the last new token of each sequence
         self.cu_q = None              # python list of cumulative q lengths
         self.layer_offset = 0
-        self.host_lens = None         # what set_step was given: (context_lens, its version, the lengths)
+        self.host_lens = None         # the lengths as set_step was given them, while nobody else holds the tensor
         self.cu_q_dev = None          # int32 [B+1]: cu_q on the device (ragged caches, prefill steps)
         self.prefill_work = {}        # work lists of the prefill kernels, made when a layer needs them
         self.q_lens_host = self.context_lens_host = ()
         self.n_long_rows = self.n_single_rows = 0     # sequences with several new rows / with one
+
+    @property
+    def context_lens(self) -> Optional[torch.Tensor]:
+        """Tokens in the cache after this step, per sequence. Whoever reads this may keep the tensor and write to it at any time (in
+        inference mode, through ``.data`` or from a kernel nothing would show it), so the host's copy is not used from then on."""
+        self.host_lens = None
+        return self._lens
+
+    @context_lens.setter
+    def context_lens(self, lens):
+        self._lens, self.host_lens = lens, None
 
     @property
     def has_state(self) -> bool:
@@ -161,7 +165,6 @@ class KVCacheContext:
         # no row of their own: one entry per sequence that has tokens
         last = [c - 1 for c, n in zip(cu[1:], q) if n > 0]
         given = (block_tables, slot_mapping, context_lens)
-        self.host_lens = None
         if torch.device(device).type != "cuda" or any(isinstance(x, torch.Tensor) and x.is_cuda for x in given):
             self.block_tables, self.slot_mapping, self.context_lens = (
                 torch.as_tensor(x, dtype=torch.int32, device=device).contiguous() for x in given)
@@ -173,7 +176,7 @@ class KVCacheContext:
             self.block_tables, self.slot_mapping, self.context_lens, self.q_seq_lens, index = _to_device(
                 given + [np.asarray(last, np.int64).view(np.int32)], device)
             self.last_token_index = index.view(torch.int64)
-            self.host_lens = (self.context_lens, _version(self.context_lens), given[2].tolist())
+            self.host_lens = given[2].tolist()
         if self.carry is not None and is_prefill:
             self.carry_before.copy_(self.carry)
         if self.ragged and is_prefill:
@@ -264,9 +267,8 @@ class _PrefillPlan:
     row of every sequence in q, and in a gathered copy of all cached rows that a step with history sees. ``ok`` False: a step that
     these kernels do not take (a sequence longer than its block table, rows that are not there)."""
 
-    def __init__(self, cache, rows: int):
-        self.key = (cache.context_lens, cache.cu_q, rows, _version(cache.context_lens))
-        lens, cu = _host_lens(cache), cache.cu_q
+    def __init__(self, cache, rows: int, lens: list):
+        cu = cache.cu_q
         B = len(lens)
         reach = cache.block_tables.shape[1] * cache.block_size
         news = [cu[b + 1] - cu[b] for b in range(B)] if len(cu) == B + 1 else []
@@ -274,7 +276,6 @@ class _PrefillPlan:
         self.ok = 0 < self.rows <= rows and len(news) == B and cu[0] == 0 and all(0 <= n <= m <= reach for n, m in zip(news, lens) if n)
         if not self.ok:
             return
-        self.aligned = all(n == m and n % _TILE == 0 for n, m in zip(news, lens) if n)
         tiles = {False: [], True: []}
         gather = {False: [0], True: [0]}       # of the sequences with history / of all that have new rows
         for b, (n, m) in enumerate(zip(news, lens)):
@@ -296,13 +297,13 @@ class _PrefillPlan:
 
 
 def _prefill_plan(cache, rows: int) -> _PrefillPlan:
-    """The step's plan, shared by its layers: kept until the step's metadata are replaced."""
-    plan = cache.prefill_work.get("plan") if cache.is_prefill else None
-    if plan is None or plan.key[0] is not cache.context_lens or plan.key[1] is not cache.cu_q \
-            or plan.key[2:] != (rows, _version(cache.context_lens)):
-        plan = _PrefillPlan(cache, rows)
-        if cache.is_prefill:
-            cache.prefill_work["plan"] = plan
+    """The step's plan, shared by its layers: kept while all that it follows from has the values it had, on the stream that made it."""
+    lens, tables = _host_lens(cache), cache.block_tables
+    key = (rows, tuple(lens), tuple(cache.cu_q), tables.shape, cache.block_size, _lib.stream_ptr() if tables.is_cuda else 0)
+    plan = cache.prefill_work.get("plan")
+    if plan is None or plan.key != key:
+        plan = cache.prefill_work["plan"] = _PrefillPlan(cache, rows, lens)
+        plan.key = key
     return plan
 
 
@@ -330,7 +331,7 @@ def _decode_step(q, k, v, cache, layer: int, scale: float):
     """One new row per sequence: into the cache and attention over it in one call (bf16 cache of head dim 128: ``paged_decode_tc.cu``, int8
     cache: ``paged_decode_int8.cu``). None where those kernels do not take the call; nothing was written then."""
     B, nq, hd = q.shape
-    kc, lens = cache.key_cache[layer], cache.context_lens
+    kc, lens = cache.key_cache[layer], cache._lens
     ksc, vsc = _layer_scales(cache, layer)
     if not q.is_cuda or not (q.dtype == k.dtype == v.dtype == torch.bfloat16) or B != lens.shape[0] or k.shape != v.shape \
             or k.shape[0] != B or k.shape[2] != hd or kc.dtype != (torch.bfloat16 if ksc is None else torch.int8):
@@ -434,7 +435,7 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
     _write_cache(cache, layer, k, v)
     T, nq, hd = q.shape
     nkv = k.shape[1]
-    B = cache.context_lens.shape[0]
+    B = cache._lens.shape[0]
     if not cache.is_prefill and T == B:
         out = torch.empty((T, nq, hd), dtype=q.dtype, device=q.device)
         if q.is_cuda and q.dtype == torch.bfloat16 and hd in (64, 128) and nq // nkv <= 16:
@@ -446,13 +447,13 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
             rc = lib.mfb_paged_decode_attention_ex(
                 qc.data_ptr(), cache.key_cache[layer].data_ptr(), cache.value_cache[layer].data_ptr(),
                 _lib.ptr(ksc), _lib.ptr(vsc),
-                cache.block_tables.data_ptr(), cache.context_lens.data_ptr(), out.data_ptr(),
+                cache.block_tables.data_ptr(), cache._lens.data_ptr(), out.data_ptr(),
                 _decode_scratch(cache, lib.mfb_paged_decode_scratch_bytes(B, nq, hd, splits), q.device).data_ptr(), splits, B, nq, nkv, hd,
                 cache.block_size, max_blocks, float(scale), _lib.stream_ptr())
             _lib.check(rc, "mfb_paged_decode_attention_ex")
             _lib.count_launch(2)
             return out.view(T, nq * hd)
-        lens = cache.context_lens.tolist()
+        lens = cache._lens.tolist()
         ksc, vsc = _layer_scales(cache, layer)
         for b in range(B):
             kk = _gather(cache.key_cache[layer], cache.block_tables[b], lens[b], cache.block_size, ksc, q.dtype)
@@ -466,7 +467,7 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
         return out
     # other types, sizes and layouts: sequence by sequence
     outs = []
-    lens = cache.context_lens.tolist()
+    lens = _host_lens(cache)
     for b in range(B):
         a, e = cache.cu_q[b], cache.cu_q[b + 1]
         if e == a:
@@ -589,13 +590,13 @@ def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
     nh, nope, rope_d, vd, rank = attn.nh, attn.nope, attn.rope_d, attn.vd, attn.kv_rank
     w = attn.linear_kvb.weight.view(nh, nope + vd, rank)
     w_uk, w_uv = w[:, :nope], w[:, nope:]                                      # [nh, nope, rank], [nh, vd, rank]
-    B = cache.context_lens.shape[0]
+    B = cache._lens.shape[0]
     if (not cache.is_prefill and T == B and q_nope.is_cuda and q_nope.dtype == torch.bfloat16 and rank == 512
             and rope_d == 64 and cache.block_size in (16, 32, 64, 128)):
         # decode: absorbed queries against the latent cache in one tcgen05 kernel (ops/csrc/mla_decode.cu)
         q_lat = torch.einsum("bhn,hnr->bhr", q_nope, w_uk)
         q_cat = torch.cat((q_lat, q_pe.reshape(B, nh, rope_d)), dim=-1).contiguous()
-        o_lat = mla_decode_attention(q_cat, cache.key_cache[layer], cache.block_tables, cache.context_lens,
+        o_lat = mla_decode_attention(q_cat, cache.key_cache[layer], cache.block_tables, cache._lens,
                                      cache.block_size, attn.scale, cache)
         return torch.einsum("bhr,hvr->bhv", o_lat, w_uv).reshape(B, nh * vd)
     lens = _host_lens(cache)

@@ -195,3 +195,59 @@ def test_latent_decode_heads_on_rows(heads, block):
         err = (got[b].double() - want).norm() / want.norm()
         assert err < 4e-3, (b, float(err))           # the weights and the result are rounded, 1.7e-3 in the mean square each
     assert _lib.read_status() == 0
+
+
+def _set(ctx, tables, block, lens, news):
+    ctx.set_step(is_prefill=True, slot_mapping=_slots(tables, block, lens, news).numpy(), q_seq_lens=news, block_tables=tables.numpy(),
+                 context_lens=lens, device=DEV)
+
+
+def _prefill_call(path, rows):
+    """A context of two sequences and a prefill call on it: grouped-query attention over a bf16 cache, multi-latent attention by expansion
+    or (other head sizes) by the general path."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(rows)
+    if path == "grouped":
+        ctx = pa.KVCacheContext(1, 16, 16, 2, 64, torch.bfloat16, DEV)
+        ctx.key_cache[0].normal_()
+        ctx.value_cache[0].normal_()
+        x = torch.randn(rows, 8, 64, device=DEV).to(torch.bfloat16)
+        return ctx, lambda: pa.paged_attention_forward(x[:, :4], x[:, 4:6], x[:, 6:], types.SimpleNamespace(cache=ctx), 1, 0.125)
+    nope, heads = (128 if path == "expanded" else 64), 3
+    ctx = pa.KVCacheContext(1, 16, 16, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
+    ctx.key_cache[0].normal_()
+    w = (torch.randn(heads * 2 * nope, 512, device=DEV) * 512 ** -0.5).to(torch.bfloat16)
+    attn = types.SimpleNamespace(nh=heads, nope=nope, rope_d=64, vd=nope, kv_rank=512, layer_number=1, scale=0.07,
+                                 linear_kvb=types.SimpleNamespace(weight=w))
+    q = torch.randn(rows, heads, nope + 64, device=DEV).to(torch.bfloat16)
+    new = torch.randn(rows, 576, device=DEV).to(torch.bfloat16)
+    return ctx, lambda: pa.mla_paged_attention_forward(attn, q[..., :nope], q[..., nope:].clone(), new[:, :512], new[:, 512:],
+                                                       types.SimpleNamespace(cache=ctx))
+
+
+@pytest.mark.parametrize("path", ["grouped", "expanded", "general"])
+@pytest.mark.parametrize("how", ["inference", "data", "version", "kept", "boundaries"])
+def test_step_changed_after_set_step(path, how):
+    """A prefill call answers for the lengths and boundaries that its context has now."""
+    first, then, news = [90, 70], [85, 70], [3, 5]
+    tables, _ = _tables([96, 96], 16)
+    ctx, call = _prefill_call(path, sum(news))
+    with torch.inference_mode(how == "inference"), torch.no_grad():
+        _set(ctx, tables, 16, first, news)
+        slots = ctx.slot_mapping.clone()
+        kept = ctx.context_lens if how == "kept" else None
+        if how in ("kept", "boundaries"):
+            call()                                   # what the layers of a step share has been made
+        if how == "boundaries":
+            ctx.cu_q[1] = 4
+            then, news = first, [4, 4]
+        elif how == "kept":
+            kept.data.copy_(torch.tensor(then))
+        elif how == "data":
+            ctx.context_lens.data.copy_(torch.tensor(then))
+        else:
+            ctx.context_lens.copy_(torch.tensor(then))
+        got = call()
+        _set(ctx, tables, 16, then, news)
+        ctx.slot_mapping = slots
+        assert torch.equal(got, call())

@@ -1,0 +1,36 @@
+"""What a prefill step's plan is made from, and which steps it leaves to the general path."""
+import numpy as np
+import torch
+
+from mindformers_b200.inference import paged_attention as pa
+
+
+def _ctx(tables, lens=(40, 20), news=(8, 4)):
+    ctx = pa.KVCacheContext(1, 8, 16, 1, 64, torch.float32, "cpu")
+    ctx.set_step(is_prefill=True, block_tables=tables, slot_mapping=np.zeros(sum(news), np.int32), context_lens=list(lens),
+                 q_seq_lens=list(news), device="cpu")
+    return ctx
+
+
+def test_plan_follows_the_values_it_was_made_from():
+    ctx = _ctx(np.zeros((2, 3), np.int32))
+    plan = pa._prefill_plan(ctx, 12)
+    assert plan.ok and plan.n_past_rows == 60 and pa._prefill_plan(ctx, 12) is plan
+    ctx.cu_q[1] = 9                                          # the same list, other boundaries
+    assert pa._prefill_plan(ctx, 12).cu.tolist() == [0, 9, 12]
+    ctx.context_lens.data.add_(1)
+    assert pa._prefill_plan(ctx, 12).n_past_rows == 62
+    ctx.block_tables = torch.zeros((2, 2), dtype=torch.int32)
+    assert not pa._prefill_plan(ctx, 12).ok                  # 41 tokens in tables of 32
+
+
+def test_host_copy_of_the_lengths_ends_when_the_tensor_is_handed_out():
+    ctx = _ctx(np.zeros((2, 3), np.int32))
+    ctx.host_lens = [40, 20]                                 # as set_step leaves it for a CUDA device
+    assert pa._host_lens(ctx) == [40, 20] and ctx.host_lens is not None
+    held = ctx.context_lens
+    held.data.add_(1)
+    assert pa._host_lens(ctx) == [41, 21]
+    ctx.host_lens = [41, 21]
+    ctx.context_lens = torch.tensor([7, 7], dtype=torch.int32)
+    assert pa._host_lens(ctx) == [7, 7]
