@@ -265,12 +265,14 @@ class _PrefillPlan:
     """What the prefill kernels need to know about a step: per query tile ``(sequence, first row of q, rows, position of the first
     row)``, longest first, for the sequences whose keys are all new (``fresh``) and for those with cached ones (``past``); the first
     row of every sequence in q, and in a gathered copy of all cached rows that a step with history sees. ``ok`` False: a step that
-    these kernels do not take (a sequence longer than its block table, rows that are not there)."""
+    these kernels do not take (a sequence longer than its block table or without one, rows that are not there, tables of another form)."""
 
     def __init__(self, cache, rows: int, lens: list):
         cu = cache.cu_q
         B = len(lens)
-        reach = cache.block_tables.shape[1] * cache.block_size
+        tables = cache.block_tables
+        fits = tables.dim() == 2 and tables.shape[0] >= B and tables.dtype == torch.int32 and tables.is_contiguous()
+        reach = tables.shape[1] * cache.block_size if fits else -1
         news = [cu[b + 1] - cu[b] for b in range(B)] if len(cu) == B + 1 else []
         self.rows = cu[-1]
         self.ok = 0 < self.rows <= rows and len(news) == B and cu[0] == 0 and all(0 <= n <= m <= reach for n, m in zip(news, lens) if n)
@@ -405,10 +407,10 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
 
 
 def _gather_rows(cache, outs, rows, scales, cu, longest: int):
-    """Cached rows of every sequence, one after the other (``cu [B + 1]``), out of one or two caches of the same shape; de-quantised where
+    """Cached rows of the sequences of ``cu [B + 1]``, one after the other, out of one or two caches of the same shape; de-quantised where
     ``scales`` are given."""
     lib, tables = _lib.get_lib(), cache.block_tables
-    B, max_blocks = tables.shape
+    B, max_blocks = cu.numel() - 1, tables.shape[1]
     heads, dim = rows[0].shape[2:]
     if scales[0] is None:
         rc = lib.mfb_gather_cache2(rows[0].data_ptr(), rows[1].data_ptr() if len(rows) > 1 else 0, tables.data_ptr(), cu.data_ptr(),

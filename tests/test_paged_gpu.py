@@ -251,3 +251,28 @@ def test_step_changed_after_set_step(path, how):
         _set(ctx, tables, 16, then, news)
         ctx.slot_mapping = slots
         assert torch.equal(got, call())
+
+
+@pytest.mark.parametrize("kind", ["int8", "odd pages", "latent"])
+def test_more_tables_than_sequences(kind):
+    """Rows of the block tables past the step's sequences are not looked at, where the rows that a step sees are copied out first."""
+    from mindformers_b200.inference import paged_attention as pa
+    block, lens, news = (24 if kind == "odd pages" else 16), [90, 70], [3, 5]
+    tables, blocks = _tables([96, 96], block)
+    if kind == "latent":
+        ctx, call = _prefill_call("expanded", sum(news))
+    else:
+        ctx = pa.KVCacheContext(1, blocks, block, 1, 64, torch.bfloat16, DEV, kv_cache_dtype="int8" if kind == "int8" else None)
+        x = torch.randn(sum(news), 4, 64, device=DEV).to(torch.bfloat16)
+        rows = torch.randn(2, sum(lens), 1, 64, device=DEV).to(torch.bfloat16)
+        _set(ctx, tables, block, lens, lens)
+        pa._write_cache(ctx, 0, rows[0], rows[1])
+
+        def call():
+            return pa.paged_attention_forward(x[:, :2], x[:, 2:3], x[:, 3:], types.SimpleNamespace(cache=ctx), 1, 0.125)
+    with torch.no_grad():
+        _set(ctx, tables, block, lens, news)
+        want = call()
+        more = torch.cat((tables, torch.full((5, tables.shape[1]), -1, dtype=torch.int32)))
+        _set(ctx, more, block, lens, news)
+        assert torch.equal(call(), want)

@@ -34,3 +34,14 @@ def test_host_copy_of_the_lengths_ends_when_the_tensor_is_handed_out():
     ctx.host_lens = [41, 21]
     ctx.context_lens = torch.tensor([7, 7], dtype=torch.int32)
     assert pa._host_lens(ctx) == [7, 7]
+
+
+def test_tables_of_another_form_stay_on_the_general_path():
+    good = np.zeros((2, 3), np.int32)
+    for tables, ok in ((good, True), (np.zeros((3, 3), np.int32), True), (good[:1], False), (np.zeros(0, np.int32), False)):
+        assert pa._prefill_plan(_ctx(tables), 12).ok == ok, tables.shape
+    ctx = _ctx(good)
+    ctx.block_tables = torch.zeros((2, 3), dtype=torch.int64)
+    assert not pa._prefill_plan(ctx, 12).ok
+    ctx.block_tables = torch.zeros((3, 2), dtype=torch.int32).t()
+    assert not pa._prefill_plan(ctx, 12).ok
