@@ -39,6 +39,9 @@ def _to_device(arrays, device):
 def _host_lens(cache) -> list:
     """The step's context lengths on the host: those ``set_step`` was given, or a read of the device once somebody else may have changed
     them (``KVCacheContext.context_lens``)."""
+    if cache._lens.is_cuda and torch.cuda.is_current_stream_capturing():
+        # a replay would go on with the tiles of the captured step's lengths
+        raise RuntimeError("attention of this step needs the context lengths on the host: it cannot be captured in a CUDA graph")
     return cache.host_lens if cache.host_lens is not None else cache._lens.tolist()
 
 

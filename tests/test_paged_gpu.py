@@ -276,3 +276,22 @@ def test_more_tables_than_sequences(kind):
         more = torch.cat((tables, torch.full((5, tables.shape[1]), -1, dtype=torch.int32)))
         _set(ctx, more, block, lens, news)
         assert torch.equal(call(), want)
+
+
+@pytest.mark.parametrize("path", ["grouped", "expanded", "general"])
+@pytest.mark.parametrize("planned", [False, True])
+def test_prefill_is_not_captured(path, planned):
+    """A graph would keep the tiles of one step's lengths: a prefill call under capture raises, also where its plan is there already."""
+    tables, _ = _tables([96, 96], 16)
+    ctx, call = _prefill_call(path, 8)
+    with torch.no_grad():
+        _set(ctx, tables, 16, [90, 70], [3, 5])
+        want = call()
+        if not planned:
+            _set(ctx, tables, 16, [90, 70], [3, 5])
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="captured"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                call()
+        torch.cuda.synchronize()
+        assert torch.equal(call(), want)
