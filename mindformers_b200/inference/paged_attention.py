@@ -22,6 +22,13 @@ from ..ops import _lib
 from ..ops import functional as Fn
 
 
+def _strides(shape) -> list:
+    out = [1] * len(shape)
+    for i in range(len(shape) - 1, 0, -1):
+        out[i - 1] = out[i] * shape[i]
+    return out
+
+
 def _to_device(arrays, device):
     """int32 arrays as device tensors, each on 16 bytes, through one pinned buffer and one copy in stream order."""
     at, spans = 0, []
@@ -33,22 +40,52 @@ def _to_device(arrays, device):
     for a, (start, n, _) in zip(arrays, spans):
         flat[start:start + n] = a.reshape(-1)
     dev = host.to(device, non_blocking=True)       # the pinned buffer is not handed out again before the copy is done
-    return [dev[start:start + n].view(shape) for start, n, shape in spans]
+    return [dev.as_strided(shape, _strides(shape), start) for start, n, shape in spans]
 
 
 def _host_lens(cache) -> list:
     """The step's context lengths on the host: those ``set_step`` was given, or a read of the device once somebody else may have changed
     them (``KVCacheContext.context_lens``)."""
-    if cache._lens.is_cuda and torch.cuda.is_current_stream_capturing():
+    if cache._context_lens.is_cuda and torch.cuda.is_current_stream_capturing():
         # a replay would go on with the tiles of the captured step's lengths
         raise RuntimeError("attention of this step needs the context lengths on the host: it cannot be captured in a CUDA graph")
-    return cache.host_lens if cache.host_lens is not None else cache._lens.tolist()
+    return cache.host_lens if cache.host_lens is not None else cache._context_lens.tolist()
+
+
+class _StepTensor:
+    """A tensor of the step's metadata. ``set_step`` queues its copy on the current stream and does not wait. The kernels of this module
+    follow in the order of that stream (``_in_order``); whoever reads the attribute may use the tensor on any stream, so it is complete
+    by then."""
+
+    def __set_name__(self, owner, name):
+        self.name = "_" + name
+
+    def __get__(self, ctx, owner=None):
+        if ctx is None:
+            return self
+        ctx._await_copy()
+        if self.name == "_context_lens":
+            # the reader may keep the tensor and write to it at any time (in inference mode, through .data or from a kernel nothing would
+            # show it): the host's copy is not used from then on
+            ctx.host_lens = None
+        return ctx.__dict__[self.name]
+
+    def __set__(self, ctx, value):
+        ctx.__dict__[self.name] = value
+        if self.name == "_context_lens":
+            ctx.host_lens = None
 
 
 class KVCacheContext:
     """Per-layer paged caches ``[num_blocks, block_size, kv_heads, head_dim]`` (or the 576-wide latent cache of
     multi-latent attention) plus the metadata of the current step: block tables, slot mapping, context lengths, new
     tokens per sequence."""
+
+    block_tables = _StepTensor()      # int32 [B, max_blocks]
+    slot_mapping = _StepTensor()      # int32 [T]
+    context_lens = _StepTensor()      # int32 [B] tokens in cache after this step
+    q_seq_lens = _StepTensor()        # int32 [B] new tokens of each sequence in this step
+    last_token_index = _StepTensor()  # int64 [B] row of the last new token of each sequence
 
     def __init__(self, num_layers: int, num_blocks: int, block_size: int, kv_heads: int, head_dim: int,
                  dtype=torch.bfloat16, device="cuda", mla_latent_dim: Optional[int] = None,
@@ -110,11 +147,9 @@ class KVCacheContext:
         self.carry = torch.zeros((num_layers, slots, carry_width), dtype=torch.float32, device=device) if carry_width else None
         self.carry_before = torch.zeros_like(self.carry) if carry_width else None
         self.is_prefill = True
-        self.block_tables = None      # int32 [B, max_blocks]
-        self.slot_mapping = None      # int32 [T]
-        self._lens = None             # context_lens: int32 [B] tokens in cache after this step
-        self.q_seq_lens = None        # int32 [B] new tokens of each sequence in this step
-        self.last_token_index = None  # int64 [B] row of the last new token of each sequence
+        self._copied = None           # (event behind the copy of the step's tensors, its stream) while it may be under way
+        self._event = None            # (the event, its device)
+        self.block_tables = self.slot_mapping = self.context_lens = self.q_seq_lens = self.last_token_index = None
         self.cu_q = None              # python list of cumulative q lengths
         self.layer_offset = 0
         self.host_lens = None         # the lengths as set_step was given them, while nobody else holds the tensor
@@ -123,16 +158,39 @@ class KVCacheContext:
         self.q_lens_host = self.context_lens_host = ()
         self.n_long_rows = self.n_single_rows = 0     # sequences with several new rows / with one
 
-    @property
-    def context_lens(self) -> Optional[torch.Tensor]:
-        """Tokens in the cache after this step, per sequence. Whoever reads this may keep the tensor and write to it at any time (in
-        inference mode, through ``.data`` or from a kernel nothing would show it), so the host's copy is not used from then on."""
-        self.host_lens = None
-        return self._lens
+    def _await_copy(self):
+        """Returns when the step's tensors are on the device."""
+        copied = self._copied
+        if copied is not None:
+            rc = _lib.get_lib().mfb_event_done(copied[0].cuda_event, 1)
+            _lib.check(rc, "mfb_event_done")
+            self._copied = None
 
-    @context_lens.setter
-    def context_lens(self, lens):
-        self._lens, self.host_lens = lens, None
+    def _in_order(self):
+        """Before kernels on the current stream read the step's tensors: on the stream that copies them there is nothing to wait for."""
+        copied = self._copied
+        if copied is None:
+            return
+        if copied[1] != _lib.stream_ptr() or torch.cuda.is_current_stream_capturing():
+            self._await_copy()
+        elif not self.is_prefill and _lib.get_lib().mfb_event_done(copied[0].cuda_event, 0) == 0:
+            self._copied = None              # the short layers of a decode step need not ask again
+
+    def _mark_copy(self, index: Optional[int]):
+        """Behind the copy of the step's tensors on the current stream of a device."""
+        here = torch.cuda.current_device()
+        index = here if index is None else index
+        stream = _lib.stream_ptr(index)
+        if self._event is None or self._event[1] != index or index != here:
+            self._event = (torch.cuda.Event(), index)
+            self._event[0].record(torch.cuda.current_stream(index))
+        else:                                # (a stream object costs more host time than this)
+            _lib.check(_lib.get_lib().mfb_event_record(self._event[0].cuda_event, stream), "mfb_event_record")
+        self._copied = (self._event[0], stream)
+
+    def __getstate__(self):
+        self._await_copy()
+        return dict(self.__dict__, _event=None)
 
     @property
     def has_state(self) -> bool:
@@ -168,6 +226,7 @@ class KVCacheContext:
         # no row of their own: one entry per sequence that has tokens
         last = [c - 1 for c, n in zip(cu[1:], q) if n > 0]
         given = (block_tables, slot_mapping, context_lens)
+        self._copied = None
         if torch.device(device).type != "cuda" or any(isinstance(x, torch.Tensor) and x.is_cuda for x in given):
             self.block_tables, self.slot_mapping, self.context_lens = (
                 torch.as_tensor(x, dtype=torch.int32, device=device).contiguous() for x in given)
@@ -175,10 +234,13 @@ class KVCacheContext:
             self.last_token_index = torch.as_tensor(last, dtype=torch.int64, device=device)
         else:
             # one copy, in the order of the current stream, that the host does not wait for
+            if torch.cuda.is_current_stream_capturing():
+                raise RuntimeError("a step's metadata come from the host: set_step cannot be captured in a CUDA graph")
             given = [np.asarray(x).astype(np.int32) for x in given] + [np.asarray(q, np.int32)]
             self.block_tables, self.slot_mapping, self.context_lens, self.q_seq_lens, index = _to_device(
                 given + [np.asarray(last, np.int64).view(np.int32)], device)
             self.last_token_index = index.view(torch.int64)
+            self._mark_copy(torch.device(device).index)
             self.host_lens = given[2].tolist()
         if self.carry is not None and is_prefill:
             self.carry_before.copy_(self.carry)
@@ -199,11 +261,11 @@ def _write_cache(cache: KVCacheContext, layer: int, k: torch.Tensor, v: Optional
                 and v.stride(2) == 1 and v.stride(1) == v.shape[2]:
             rc = _lib.get_lib().mfb_reshape_and_cache_int8(
                 k.data_ptr(), v.data_ptr(), kc.data_ptr(), vc.data_ptr(), ks.data_ptr(), vs.data_ptr(),
-                cache.slot_mapping.data_ptr(), T, k.shape[1], k.shape[2], k.stride(0), v.stride(0), _lib.stream_ptr())
+                cache._slot_mapping.data_ptr(), T, k.shape[1], k.shape[2], k.stride(0), v.stride(0), _lib.stream_ptr())
             _lib.check(rc, "mfb_reshape_and_cache_int8")
             _lib.count_launch()
             return
-        slots = cache.slot_mapping.long()
+        slots = cache._slot_mapping.long()
         ok = slots >= 0
         for src, dst, sc in ((k, kc, ks), (v, vc, vs)):
             x = src.reshape(T, src.shape[1], src.shape[2])[ok].float()
@@ -215,12 +277,12 @@ def _write_cache(cache: KVCacheContext, layer: int, k: torch.Tensor, v: Optional
         return
     if k.is_cuda and k.dtype == torch.bfloat16 and row % 8 == 0 and k.stride(2) == 1 and k.stride(1) == k.shape[2]:
         rc = _lib.get_lib().mfb_reshape_and_cache(k.data_ptr(), _lib.ptr(v), kc.data_ptr(), _lib.ptr(vc),
-                                                  cache.slot_mapping.data_ptr(), T, row, k.stride(0),
+                                                  cache._slot_mapping.data_ptr(), T, row, k.stride(0),
                                                   v.stride(0) if v is not None else 0, _lib.stream_ptr())
         _lib.check(rc, "mfb_reshape_and_cache")
         _lib.count_launch()
         return
-    slots = cache.slot_mapping.long()
+    slots = cache._slot_mapping.long()
     ok = slots >= 0
     kc.view(-1, row)[slots[ok]] = k.reshape(T, row)[ok].to(kc.dtype)
     if v is not None:
@@ -273,7 +335,7 @@ class _PrefillPlan:
     def __init__(self, cache, rows: int, lens: list):
         cu = cache.cu_q
         B = len(lens)
-        tables = cache.block_tables
+        tables = cache._block_tables
         fits = tables.dim() == 2 and tables.shape[0] >= B and tables.dtype == torch.int32 and tables.is_contiguous()
         reach = tables.shape[1] * cache.block_size if fits else -1
         news = [cu[b + 1] - cu[b] for b in range(B)] if len(cu) == B + 1 else []
@@ -295,7 +357,7 @@ class _PrefillPlan:
             flat += [x for t in items for x in t]
         at = len(flat)
         flat += list(cu) + gather[False] + gather[True]
-        dev, = _to_device([np.asarray(flat, np.int32)], cache.block_tables.device)
+        dev, = _to_device([np.asarray(flat, np.int32)], cache._block_tables.device)
         self.fresh, self.past, self.all = ((dev[a:a + 4 * n], n, p) for a, n, p in spans)
         self.cu, self.past_rows, self.all_rows = (dev[at + i * (B + 1):at + (i + 1) * (B + 1)] for i in range(3))
         self.n_past_rows, self.n_all_rows, self.longest = gather[False][-1], gather[True][-1], max(lens)
@@ -303,7 +365,7 @@ class _PrefillPlan:
 
 def _prefill_plan(cache, rows: int) -> _PrefillPlan:
     """The step's plan, shared by its layers: kept while all that it follows from has the values it had, on the stream that made it."""
-    lens, tables = _host_lens(cache), cache.block_tables
+    lens, tables = _host_lens(cache), cache._block_tables
     key = (rows, tuple(lens), tuple(cache.cu_q), tables.shape, cache.block_size, _lib.stream_ptr() if tables.is_cuda else 0)
     plan = cache.prefill_work.get("plan")
     if plan is None or plan.key != key:
@@ -336,19 +398,19 @@ def _decode_step(q, k, v, cache, layer: int, scale: float):
     """One new row per sequence: into the cache and attention over it in one call (bf16 cache of head dim 128: ``paged_decode_tc.cu``, int8
     cache: ``paged_decode_int8.cu``). None where those kernels do not take the call; nothing was written then."""
     B, nq, hd = q.shape
-    kc, lens = cache.key_cache[layer], cache._lens
+    kc, lens = cache.key_cache[layer], cache._context_lens
     ksc, vsc = _layer_scales(cache, layer)
     if not q.is_cuda or not (q.dtype == k.dtype == v.dtype == torch.bfloat16) or B != lens.shape[0] or k.shape != v.shape \
             or k.shape[0] != B or k.shape[2] != hd or kc.dtype != (torch.bfloat16 if ksc is None else torch.int8):
         return None
     out = torch.empty((B, nq * hd), dtype=torch.bfloat16, device=q.device)
-    tables = cache.block_tables
+    tables = cache._block_tables
     need = 0
     for _ in range(2):
         scratch = _decode_scratch(cache, need, q.device)
         rc = _lib.get_lib().mfb_paged_decode_step(
             q.data_ptr(), *q.stride(), k.data_ptr(), *k.stride(), v.data_ptr(), *v.stride(), kc.data_ptr(),
-            cache.value_cache[layer].data_ptr(), _lib.ptr(ksc), _lib.ptr(vsc), cache.slot_mapping.data_ptr(), tables.data_ptr(),
+            cache.value_cache[layer].data_ptr(), _lib.ptr(ksc), _lib.ptr(vsc), cache._slot_mapping.data_ptr(), tables.data_ptr(),
             lens.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel() * 4, B, nq, k.shape[1], hd, kc.shape[0],
             cache.block_size, tables.shape[1], scale, _lib.status_word(q.device).data_ptr(), _lib.stream_ptr())
         if rc <= 0:
@@ -390,8 +452,8 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
 
     def launch(work, keys, values, ld_k, ld_v, key_rows, key_row, exact):
         rc = lib.mfb_ragged_prefill_tc(
-            q.data_ptr(), q.stride(0), q.stride(1), keys, values, ld_k, ld_v, work[0].data_ptr(), work[1], cache.block_tables.data_ptr(),
-            cache.block_tables.shape[1], cache.block_size, key_rows, _lib.ptr(key_row), out.data_ptr(), out.stride(0), T, nq, nkv, hd,
+            q.data_ptr(), q.stride(0), q.stride(1), keys, values, ld_k, ld_v, work[0].data_ptr(), work[1], cache._block_tables.data_ptr(),
+            cache._block_tables.shape[1], cache.block_size, key_rows, _lib.ptr(key_row), out.data_ptr(), out.stride(0), T, nq, nkv, hd,
             hd, int(exact), int(work[2]), float(scale), st, stream)
         _lib.check(rc, "mfb_ragged_prefill_tc")
         _lib.count_launch()
@@ -412,7 +474,7 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
 def _gather_rows(cache, outs, rows, scales, cu, longest: int):
     """Cached rows of the sequences of ``cu [B + 1]``, one after the other, out of one or two caches of the same shape; de-quantised where
     ``scales`` are given."""
-    lib, tables = _lib.get_lib(), cache.block_tables
+    lib, tables = _lib.get_lib(), cache._block_tables
     B, max_blocks = cu.numel() - 1, tables.shape[1]
     heads, dim = rows[0].shape[2:]
     if scales[0] is None:
@@ -432,6 +494,7 @@ def _gather_rows(cache, outs, rows, scales, cu, longest: int):
 def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
     """q: [T, nq, hd]; k/v: [T, nkv, hd] of the new tokens. Returns [T, nq*hd]."""
     cache: KVCacheContext = meta.cache
+    cache._in_order()
     layer = layer_number - 1 - cache.layer_offset
     if not cache.is_prefill and _DECODE_KERNEL == "tensor_core":
         out = _decode_step(q, k, v, cache, layer, scale)
@@ -440,29 +503,29 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
     _write_cache(cache, layer, k, v)
     T, nq, hd = q.shape
     nkv = k.shape[1]
-    B = cache._lens.shape[0]
+    B = cache._context_lens.shape[0]
     if not cache.is_prefill and T == B:
         out = torch.empty((T, nq, hd), dtype=q.dtype, device=q.device)
         if q.is_cuda and q.dtype == torch.bfloat16 and hd in (64, 128) and nq // nkv <= 16:
             lib = _lib.get_lib()
-            max_blocks = cache.block_tables.shape[1]
+            max_blocks = cache._block_tables.shape[1]
             ksc, vsc = _layer_scales(cache, layer)
             qc = q.contiguous()
             splits = lib.mfb_paged_decode_splits(B, nkv, cache.block_size, max_blocks)
             rc = lib.mfb_paged_decode_attention_ex(
                 qc.data_ptr(), cache.key_cache[layer].data_ptr(), cache.value_cache[layer].data_ptr(),
                 _lib.ptr(ksc), _lib.ptr(vsc),
-                cache.block_tables.data_ptr(), cache._lens.data_ptr(), out.data_ptr(),
+                cache._block_tables.data_ptr(), cache._context_lens.data_ptr(), out.data_ptr(),
                 _decode_scratch(cache, lib.mfb_paged_decode_scratch_bytes(B, nq, hd, splits), q.device).data_ptr(), splits, B, nq, nkv, hd,
                 cache.block_size, max_blocks, float(scale), _lib.stream_ptr())
             _lib.check(rc, "mfb_paged_decode_attention_ex")
             _lib.count_launch(2)
             return out.view(T, nq * hd)
-        lens = cache._lens.tolist()
+        lens = cache._context_lens.tolist()
         ksc, vsc = _layer_scales(cache, layer)
         for b in range(B):
-            kk = _gather(cache.key_cache[layer], cache.block_tables[b], lens[b], cache.block_size, ksc, q.dtype)
-            vv = _gather(cache.value_cache[layer], cache.block_tables[b], lens[b], cache.block_size, vsc, q.dtype)
+            kk = _gather(cache.key_cache[layer], cache._block_tables[b], lens[b], cache.block_size, ksc, q.dtype)
+            vv = _gather(cache.value_cache[layer], cache._block_tables[b], lens[b], cache.block_size, vsc, q.dtype)
             o = Fn.attention_reference(q[b:b + 1].unsqueeze(0), kk.unsqueeze(0), vv.unsqueeze(0), causal=False, scale=scale)
             out[b] = o[0, 0]
         return out.view(T, nq * hd)
@@ -482,8 +545,8 @@ def paged_attention_forward(q, k, v, meta, layer_number: int, scale: float):
             o = Fn.attention(q[a:e].unsqueeze(0), k[a:e].unsqueeze(0), v[a:e].unsqueeze(0), causal=True, scale=scale)
         else:
             ksc, vsc = _layer_scales(cache, layer)
-            kk = _gather(cache.key_cache[layer], cache.block_tables[b], lens[b], cache.block_size, ksc, q.dtype)
-            vv = _gather(cache.value_cache[layer], cache.block_tables[b], lens[b], cache.block_size, vsc, q.dtype)
+            kk = _gather(cache.key_cache[layer], cache._block_tables[b], lens[b], cache.block_size, ksc, q.dtype)
+            vv = _gather(cache.value_cache[layer], cache._block_tables[b], lens[b], cache.block_size, vsc, q.dtype)
             o = Fn.attention_reference(q[a:e].unsqueeze(0), kk.unsqueeze(0), vv.unsqueeze(0), causal=True, scale=scale,
                                        q_offset=lens[b] - nq_tok)
         outs.append(o.reshape(nq_tok, nq * v.shape[-1]))
@@ -574,7 +637,7 @@ def _write_latents(cache, layer: int, kv_c: torch.Tensor, k_pe: torch.Tensor):
             and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (kv_c, k_pe)) \
             and rows.is_contiguous() and rows.shape[-1] == rank + rope:
         rc = _lib.get_lib().mfb_latent_to_cache(kv_c.data_ptr(), kv_c.stride(0), k_pe.data_ptr(), k_pe.stride(0), rows.data_ptr(),
-                                                cache.slot_mapping.data_ptr(), T, rank, rope, _lib.stream_ptr())
+                                                cache._slot_mapping.data_ptr(), T, rank, rope, _lib.stream_ptr())
         _lib.check(rc, "mfb_latent_to_cache")
         _lib.count_launch()
         return
@@ -589,19 +652,20 @@ def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
     mapped back with ``W_UV`` (reference ``multi_latent_attention.py:219-231,434-448``).
     """
     cache: KVCacheContext = meta.cache
+    cache._in_order()
     layer = attn.layer_number - 1 - cache.layer_offset
     T = q_nope.shape[0]
     _write_latents(cache, layer, kv_c, k_pe.reshape(T, -1))
     nh, nope, rope_d, vd, rank = attn.nh, attn.nope, attn.rope_d, attn.vd, attn.kv_rank
     w = attn.linear_kvb.weight.view(nh, nope + vd, rank)
     w_uk, w_uv = w[:, :nope], w[:, nope:]                                      # [nh, nope, rank], [nh, vd, rank]
-    B = cache._lens.shape[0]
+    B = cache._context_lens.shape[0]
     if (not cache.is_prefill and T == B and q_nope.is_cuda and q_nope.dtype == torch.bfloat16 and rank == 512
             and rope_d == 64 and cache.block_size in (16, 32, 64, 128)):
         # decode: absorbed queries against the latent cache in one tcgen05 kernel (ops/csrc/mla_decode.cu)
         q_lat = torch.einsum("bhn,hnr->bhr", q_nope, w_uk)
         q_cat = torch.cat((q_lat, q_pe.reshape(B, nh, rope_d)), dim=-1).contiguous()
-        o_lat = mla_decode_attention(q_cat, cache.key_cache[layer], cache.block_tables, cache._lens,
+        o_lat = mla_decode_attention(q_cat, cache.key_cache[layer], cache._block_tables, cache._context_lens,
                                      cache.block_size, attn.scale, cache)
         return torch.einsum("bhr,hvr->bhv", o_lat, w_uv).reshape(B, nh * vd)
     lens = _host_lens(cache)
@@ -632,7 +696,7 @@ def mla_paged_attention_forward(attn, q_nope, q_pe, kv_c, k_pe, meta):
         a, e = cache.cu_q[b], cache.cu_q[b + 1]
         if e == a:
             continue
-        lat = _gather(cache.key_cache[layer], cache.block_tables[b], lens[b], cache.block_size)[:, 0]  # [L, rank+rope]
+        lat = _gather(cache.key_cache[layer], cache._block_tables[b], lens[b], cache.block_size)[:, 0]  # [L, rank+rope]
         c, pe = lat[:, :rank].float(), lat[:, rank:].float()
         q_lat = torch.einsum("thn,hnr->thr", q_nope[a:e].float(), w_uk.float())    # absorbed query
         s = (torch.einsum("thr,lr->htl", q_lat, c) + torch.einsum("thd,ld->htl", q_pe[a:e].float(), pe)) * attn.scale

@@ -152,6 +152,8 @@ def _declare(lib):
     sig("mfb_paged_decode_attention_tc_ex", [P] * 9 + [I] * 13 + [F, F, L, F, P, P])
     sig("mfb_paged_decode_attention_tc_q", [P, L, L] + [P] * 8 + [I] * 13 + [F, F, L, F, P, P])
     sig("mfb_paged_decode_step", [P, L, L, L, P, L, L, L, P, L, L, L] + [P] * 9 + [L] + [I] * 7 + [F, P, P], L)
+    sig("mfb_event_done", [P, I])
+    sig("mfb_event_record", [P, P])
     sig("mfb_paged_decode_int8_supported", [I, I, I, I])
     sig("mfb_paged_decode_int8_splits", [I, I, I])
     sig("mfb_paged_decode_attention_int8", [P, L, L] + [P] * 8 + [I] * 7 + [F, P])
@@ -263,10 +265,10 @@ def check(rc: int, what: str):
         raise KernelLibraryError(f"{what} failed (code {rc}): {msg}")
 
 
-def stream_ptr() -> int:
-    """Raw handle of the current CUDA stream of the current device (the direct binding: building a
+def stream_ptr(index=None) -> int:
+    """Raw handle of the current CUDA stream of a device, by default the current one (the direct binding: building a
     ``torch.cuda.Stream`` object per kernel launch costs more host time than the launch itself)."""
-    return _raw_stream(torch.cuda.current_device())
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 try:

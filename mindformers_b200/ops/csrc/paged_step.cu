@@ -53,4 +53,24 @@ long long mfb_paged_decode_step(const void* q, long long q0, long long q1, long 
   return rc ? -200 - rc : 0;
 }
 
+int mfb_event_record(cudaEvent_t event, cudaStream_t stream) {
+  const cudaError_t rc = cudaEventRecord(event, stream);
+  if (rc != cudaSuccess) { mfb_host::set_error("event_record: %s", cudaGetErrorString(rc)); return 2; }
+  return 0;
+}
+
+// Whether all work in front of an event is done (0; 1: not yet), after waiting for it if wait != 0; other values: an error. The event stands
+// outside of whatever this thread is capturing, so the call is harmless to a capture, which forbids it by default.
+int mfb_event_done(cudaEvent_t event, int wait) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) { mfb_host::set_error("event_done: capture mode"); return 2; }
+  const cudaError_t rc = wait ? cudaEventSynchronize(event) : cudaEventQuery(event);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (rc == cudaSuccess) return 0;
+  cudaGetLastError();              // "not ready" would otherwise look like a failed launch
+  if (rc == cudaErrorNotReady) return 1;
+  mfb_host::set_error("event_done: %s", cudaGetErrorString(rc));
+  return 3;
+}
+
 }  // extern "C"

@@ -1,4 +1,5 @@
 """Attention over the paged cache on the tensor cores (ragged prefill, decode over int8 rows), against 64-bit PyTorch."""
+import copy
 import types
 
 import pytest
@@ -295,3 +296,66 @@ def test_prefill_is_not_captured(path, planned):
                 call()
         torch.cuda.synchronize()
         assert torch.equal(call(), want)
+
+
+def _decode_call(int8=False):
+    """A context of three sequences with full caches, its step and a decode call on it."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(0)
+    ctx = pa.KVCacheContext(1, 32, 16, 2, 128, torch.bfloat16, DEV, kv_cache_dtype="int8" if int8 else None)
+    for c in (ctx.key_cache[0], ctx.value_cache[0]):
+        c.copy_(torch.randn(c.shape, device=DEV) * (50 if int8 else 1))
+    lens = [90, 33, 128]
+    tables, _ = _tables(lens, 16)
+    step = dict(is_prefill=False, slot_mapping=_slots(tables, 16, lens, [1] * 3).numpy(), q_seq_lens=[1] * 3, block_tables=tables.numpy(),
+                context_lens=lens, device=DEV)
+    x = torch.randn(3, 8, 128, device=DEV).to(torch.bfloat16)
+    return ctx, step, lambda: pa.paged_attention_forward(x[:, :4], x[:, 4:6], x[:, 6:], types.SimpleNamespace(cache=ctx), 1, 0.09)
+
+
+def test_step_used_on_another_stream():
+    """The tensors of a step are complete for whoever reads them, and the attention of the step may run on another stream, although the
+    stream of ``set_step`` is still busy."""
+    ctx, step, call = _decode_call()
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        ctx.set_step(**step)
+        want = call()
+        wide = torch.arange(100000, dtype=torch.int32)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(100_000_000)               # some tens of milliseconds
+        ctx.set_step(**dict(step, slot_mapping=wide.numpy()))
+        with torch.cuda.stream(side):
+            assert torch.equal(ctx.slot_mapping.cpu(), wide)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(100_000_000)
+        ctx.set_step(**step)
+        with torch.cuda.stream(side):
+            got = call()
+        side.synchronize()
+        assert torch.equal(got, want)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(100_000_000)
+        ctx.set_step(**step)
+        twin = copy.deepcopy(ctx)
+        assert all(torch.equal(getattr(twin, n), getattr(ctx, n)) for n in ("block_tables", "slot_mapping", "context_lens"))
+
+
+def test_step_in_a_captured_graph():
+    """A step that was set before a capture serves the captured call; setting one under capture raises."""
+    ctx, step, call = _decode_call()
+    with torch.no_grad():
+        ctx.set_step(**step)
+        want = call()
+        ctx.set_step(**step)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = call()
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="captured"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                ctx.set_step(**step)
+        torch.cuda.synchronize()
