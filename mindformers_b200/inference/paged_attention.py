@@ -35,7 +35,7 @@ def _to_device(arrays, device):
     for a in arrays:
         spans.append((at, a.size, a.shape))
         at += -(-a.size // 4) * 4
-    host = torch.empty(max(at, 1), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
+    host = torch.empty(max(at, 1), dtype=torch.int32, device="cpu", pin_memory=torch.device(device).type == "cuda")
     flat = host.numpy()
     for a, (start, n, _) in zip(arrays, spans):
         flat[start:start + n] = a.reshape(-1)
@@ -236,7 +236,8 @@ class KVCacheContext:
             # one copy, in the order of the current stream, that the host does not wait for
             if torch.cuda.is_current_stream_capturing():
                 raise RuntimeError("a step's metadata come from the host: set_step cannot be captured in a CUDA graph")
-            given = [np.asarray(x).astype(np.int32) for x in given] + [np.asarray(q, np.int32)]
+            # (numbers that do not fit are refused, as in the copies above)
+            given = [np.asarray(x, dtype=np.int32) for x in given + (q,)]
             self.block_tables, self.slot_mapping, self.context_lens, self.q_seq_lens, index = _to_device(
                 given + [np.asarray(last, np.int64).view(np.int32)], device)
             self.last_token_index = index.view(torch.int64)

@@ -359,3 +359,17 @@ def test_step_in_a_captured_graph():
             with torch.cuda.graph(torch.cuda.CUDAGraph()):
                 ctx.set_step(**step)
         torch.cuda.synchronize()
+
+
+def test_step_from_the_host():
+    """Where new tensors go by default does not matter to a step; numbers that do not fit into 32 bits are refused."""
+    ctx, step, call = _decode_call()
+    with torch.no_grad():
+        ctx.set_step(**step)
+        want = call()
+        with torch.device(DEV):
+            ctx.set_step(**step)
+        assert torch.equal(call(), want)
+        for name in ("slot_mapping", "context_lens", "q_seq_lens"):
+            with pytest.raises((RuntimeError, OverflowError)):
+                ctx.set_step(**dict(step, **{name: [2 ** 31 + 5, 1, 1]}))
