@@ -350,18 +350,53 @@ class _PrefillPlan:
             tiles[n < m] += [(b, cu[b] + r, min(_TILE, n - r), m - n + r) for r in range(0, n, _TILE)]
             gather[False].append(gather[False][-1] + (m if 0 < n < m else 0))
             gather[True].append(gather[True][-1] + (m if n else 0))
-        keys = lambda t: (t[3] + t[2] - 1) // _TILE + 1
         flat, spans = [], []
         for items in (tiles[False], tiles[True], tiles[False] + tiles[True]):
-            items = sorted(items, key=keys, reverse=True)
-            spans.append((len(flat), len(items), sum(map(keys, items)) <= _PERSISTENT_UP_TO * len(items)))
-            flat += [x for t in items for x in t]
+            spans.append(self._add(flat, items))
         at = len(flat)
         flat += list(cu) + gather[False] + gather[True]
         dev, = _to_device([np.asarray(flat, np.int32)], cache._block_tables.device)
         self.fresh, self.past, self.all = ((dev[a:a + 4 * n], n, p) for a, n, p in spans)
         self.cu, self.past_rows, self.all_rows = (dev[at + i * (B + 1):at + (i + 1) * (B + 1)] for i in range(3))
         self.n_past_rows, self.n_all_rows, self.longest = gather[False][-1], gather[True][-1], max(lens)
+        self.past_host = (tiles[True], gather[False])
+        self.groups = {}
+
+    @staticmethod
+    def _add(flat: list, items: list):
+        """Appends a launch's tiles, longest first: where they start in ``flat``, how many they are, whether CTAs walk over several."""
+        keys = lambda t: (t[3] + t[2] - 1) // _TILE + 1
+        at, items = len(flat), sorted(items, key=keys, reverse=True)
+        flat += [x for t in items for x in t]
+        return at, len(items), sum(map(keys, items)) <= _PERSISTENT_UP_TO * len(items)
+
+    def copied(self, limit: int) -> list:
+        """``past`` in groups of sequences that see at most ``limit`` rows together (or one sequence): per group the work, the first row of
+        every sequence in a copy of the rows that the group sees (``[B + 1]``, none for the others) and the rows of that copy."""
+        if self.n_past_rows <= limit:
+            return [(self.past, self.past_rows, self.n_past_rows)]
+        if limit not in self.groups:
+            tiles, first = self.past_host
+            rows = [b - a for a, b in zip(first, first[1:])]
+            members, held = [[]], 0
+            for b, n in enumerate(rows):
+                if n and held and held + n > limit:
+                    members.append([])
+                    held = 0
+                if n:
+                    members[-1].append(b)
+                    held += n
+            flat, parts = [], []
+            for seqs in members:
+                own, cu = set(seqs), [0]
+                for b, n in enumerate(rows):
+                    cu.append(cu[-1] + (n if b in own else 0))
+                span = self._add(flat, [t for t in tiles if t[0] in own])
+                parts.append((span, len(flat), cu[-1]))
+                flat += cu + [0] * (-len(cu) % 4)            # the next group's tiles start on 16 bytes
+            dev, = _to_device([np.asarray(flat, np.int32)], self.past_rows.device)
+            self.groups[limit] = [((dev[a:a + 4 * n], n, p), dev[at:at + len(rows) + 1], total) for (a, n, p), at, total in parts]
+        return self.groups[limit]
 
 
 def _prefill_plan(cache, rows: int) -> _PrefillPlan:
@@ -430,6 +465,9 @@ def _rows_ok(t: torch.Tensor) -> bool:
             and t.stride(0) >= t.shape[1] * t.shape[2] and t.data_ptr() % 16 == 0)
 
 
+_COPIED_BYTES = 1 << 30          # of cached rows copied out at a time; the sequences of a step that see more take turns
+
+
 def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
     """Prefill attention of a step's sequences: those without history attend over their own rows of ``k`` / ``v``, the others over
     the cache (an int8 cache, or one of other block sizes than the kernel's, through a copy of the rows they see) with weights that are not
@@ -466,9 +504,11 @@ def _ragged_prefill(q, k, v, cache, layer: int, scale: float):
         if ksc is None and lib.mfb_ragged_prefill_tc_supported(nq, nkv, hd, hd, cache.block_size):
             launch(plan.past, kc.data_ptr(), vc.data_ptr(), row, row, kc.shape[0] * cache.block_size, None, True)
         else:
-            copies = torch.empty((2, plan.n_past_rows, row), dtype=q.dtype, device=q.device)
-            _gather_rows(cache, copies, (kc, vc), (ksc, vsc), plan.past_rows, plan.longest)
-            launch(plan.past, copies[0].data_ptr(), copies[1].data_ptr(), row, row, plan.n_past_rows, plan.past_rows, True)
+            groups = plan.copied(max(1, _COPIED_BYTES // (2 * row * 2)))
+            copies = torch.empty((2, max(g[2] for g in groups), row), dtype=q.dtype, device=q.device)
+            for work, first, rows in groups:
+                _gather_rows(cache, copies, (kc, vc), (ksc, vsc), first, plan.longest)
+                launch(work, copies[0].data_ptr(), copies[1].data_ptr(), row, row, rows, first, True)
     return out
 
 

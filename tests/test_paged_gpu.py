@@ -373,3 +373,28 @@ def test_step_from_the_host():
         for name in ("slot_mapping", "context_lens", "q_seq_lens"):
             with pytest.raises((RuntimeError, OverflowError)):
                 ctx.set_step(**dict(step, **{name: [2 ** 31 + 5, 1, 1]}))
+
+
+@pytest.mark.parametrize("block,int8", [(64, True), (24, False)])
+def test_copied_rows_in_turns(block, int8, monkeypatch):
+    """A step whose sequences see more cached rows than may be copied out at a time: the same result in less memory."""
+    from mindformers_b200.inference import paged_attention as pa
+    lens, news = [900, 1400, 64, 2000, 33, 700], [3, 200, 64, 130, 1, 5]
+    tables, blocks = _tables(lens, block)
+    ctx = pa.KVCacheContext(1, blocks, block, 4, 128, torch.bfloat16, DEV, kv_cache_dtype="int8" if int8 else None)
+    rows = torch.randn(2, sum(lens), 4, 128, device=DEV).to(torch.bfloat16)
+    x = torch.randn(sum(news), 16, 128, device=DEV).to(torch.bfloat16)
+    _set(ctx, tables, block, lens, lens)
+    pa._write_cache(ctx, 0, rows[0], rows[1])
+    taken = []
+    with torch.no_grad():
+        for budget in (pa._COPIED_BYTES, 1):
+            monkeypatch.setattr(pa, "_COPIED_BYTES", budget)
+            _set(ctx, tables, block, lens, news)
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            taken.append((pa.paged_attention_forward(x[:, :8], x[:, 8:12], x[:, 12:], types.SimpleNamespace(cache=ctx), 1, 0.09),
+                          torch.cuda.max_memory_allocated() - before))
+    assert torch.equal(taken[0][0], taken[1][0])
+    row = 2 * 4 * 128 * 2
+    assert taken[1][1] < (2000 + 500) * row < sum(lens) * row < taken[0][1] + 64 * row     # 500: the result and the step's lists

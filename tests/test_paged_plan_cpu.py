@@ -45,3 +45,21 @@ def test_tables_of_another_form_stay_on_the_general_path():
     assert not pa._prefill_plan(ctx, 12).ok
     ctx.block_tables = torch.zeros((3, 2), dtype=torch.int32).t()
     assert not pa._prefill_plan(ctx, 12).ok
+
+
+def test_copies_in_groups():
+    """Every tile in one group with the rows of its sequence, no group above the limit but for a sequence that is alone."""
+    lens, news = [40, 20, 8, 300, 30, 25], [8, 4, 8, 200, 0, 25]         # the third and the last have no history, the fifth no new rows
+    ctx = _ctx(np.zeros((6, 20), np.int32), lens, news)
+    plan = pa._prefill_plan(ctx, sum(news))
+    assert [(w[1], r) for w, _, r in plan.copied(360)] == [(4, 360)]
+    for limit, rows in ((359, [60, 300]), (59, [40, 20, 300]), (1, [40, 20, 300])):
+        groups = plan.copied(limit)
+        assert [r for _, _, r in groups] == rows
+        seen = []
+        for (work, n, _), first, total in groups:
+            tiles = work.view(n, 4).tolist()
+            assert first.numel() == 7 and first[-1] == total
+            assert all(first[b + 1] - first[b] == lens[b] for b, *_ in tiles)
+            seen += tiles
+        assert sorted(seen) == sorted(plan.past[0].view(-1, 4).tolist())
