@@ -360,7 +360,20 @@ class _PrefillPlan:
         self.cu, self.past_rows, self.all_rows = (dev[at + i * (B + 1):at + (i + 1) * (B + 1)] for i in range(3))
         self.n_past_rows, self.n_all_rows, self.longest = gather[False][-1], gather[True][-1], max(lens)
         self.past_host = (tiles[True], gather[False])
-        self.groups = {}
+        self.groups, self.forms = {}, {}
+        self.new_and_seen = [(n, m) for n, m in zip(news, lens) if n]
+
+    def expands(self, heads: int) -> bool:
+        """Whether multi-latent attention of ``heads`` heads expands the cached latents (one product over all rows that the step sees, whatever
+        the new ones, 0.9 ns per row and head) or takes the queries into the latent space (sequence by sequence, 32-bit products: 0.056 ns per new
+        row, cached row and head, some 0.1 ms besides, and 265 us of launches at least). Measured, expanded and absorbed: 128 heads, 32 sequences
+        of 8000 rows, 1 / 4 / 16 new ones each 29.8 / 30.1 / 29.9 and 9.5 / 15.8 / 35.2 ms; 1 sequence 0.97 / 0.99 / 0.96 and 0.41 / 0.56 / 1.19 ms;
+        32 of 2300 rows 8.5 / 8.5 / 8.8 and 8.5 / 9.1 / 14.2 ms; 16 heads, 4 of 2300 rows, 1 / 200 new ones 0.26 / 0.28 and 1.15 / 2.5 ms."""
+        if heads not in self.forms:
+            expanded = 110 + 0.9e-3 * self.n_all_rows * heads
+            absorbed = sum(max(265, 90 + m * (0.005 + 0.0002 * heads) + 0.056e-3 * n * m * heads) for n, m in self.new_and_seen)
+            self.forms[heads] = expanded <= absorbed
+        return self.forms[heads]
 
     @staticmethod
     def _add(flat: list, items: list):
@@ -636,7 +649,7 @@ _EXPANDED_BYTES = 2 << 30        # of expanded keys and values at a time; more h
 def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
     """Multi-latent attention of a step's new rows (any lengths, with or without history) over keys and values expanded from the
     cached latents once per call. Expanded numbers are kept as the sum of two bf16 numbers and the softmax weights likewise, so that
-    nothing between query and result is rounded to 16 bits. None where the kernel does not take the call."""
+    nothing between query and result is rounded to 16 bits. None where the kernel does not take the call or too few rows ask for it."""
     T, nh, nope = q_nope.shape
     rope_d, vd, rank = attn.rope_d, attn.vd, attn.kv_rank
     w, rows = attn.linear_kvb.weight, cache.key_cache[layer]
@@ -645,7 +658,7 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
         return None
     plan = _prefill_plan(cache, T)
     n = plan.n_all_rows if plan.ok else 0
-    if not plan.ok or n >= 1 << 31 or plan.longest * (rank + rope_d) >= 1 << 34:
+    if not plan.ok or n >= 1 << 31 or plan.longest * (rank + rope_d) >= 1 << 34 or not plan.expands(nh):
         return None
     q_pe = q_pe.reshape(T, nh, rope_d)
     q_nope, q_pe = _strided(q_nope), _strided(q_pe)

@@ -398,3 +398,28 @@ def test_copied_rows_in_turns(block, int8, monkeypatch):
     assert torch.equal(taken[0][0], taken[1][0])
     row = 2 * 4 * 128 * 2
     assert taken[1][1] < (2000 + 500) * row < sum(lens) * row < taken[0][1] + 64 * row     # 500: the result and the step's lists
+
+
+def test_latent_prefill_of_few_rows():
+    """One and two new rows behind long histories: the queries go into the latent space."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(0)
+    heads, block, lens, news = 128, 16, [3000, 2900], [1, 2]
+    tables, blocks = _tables(lens, block)
+    ctx = pa.KVCacheContext(1, blocks, block, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
+    ctx.key_cache[0].normal_()
+    w = (torch.randn(heads * 256, 512, device=DEV) * 512 ** -0.5).to(torch.bfloat16)
+    attn = types.SimpleNamespace(nh=heads, nope=128, rope_d=64, vd=128, kv_rank=512, layer_number=1, scale=192 ** -0.5,
+                                 linear_kvb=types.SimpleNamespace(weight=w))
+    q = torch.randn(3, heads, 192, device=DEV).to(torch.bfloat16)
+    new = torch.randn(3, 576, device=DEV).to(torch.bfloat16)
+    _set(ctx, tables, block, lens, news)
+    assert not pa._prefill_plan(ctx, 3).expands(heads)
+    with torch.no_grad():
+        got = pa.mla_paged_attention_forward(attn, q[..., :128], q[..., 128:].clone(), new[:, :512], new[:, 512:],
+                                             types.SimpleNamespace(cache=ctx))
+    for rows, b, m in ((slice(0, 1), 0, 3000), (slice(1, 3), 1, 2900)):
+        lat = _cached(ctx.key_cache[0][:, :, 0], tables, b, m, block).double()
+        kv = (lat[:, :512] @ w.double().t()).view(m, heads, 256)
+        want = _attend(q[rows], torch.cat((kv[..., :128], lat[:, None, 512:].expand(m, heads, 64)), -1), kv[..., 128:], attn.scale)
+        assert (got[rows].double() - want).norm() / want.norm() < 2e-3           # rounding of the result alone
