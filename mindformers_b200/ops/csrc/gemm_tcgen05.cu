@@ -38,7 +38,7 @@ struct GemmArgs {
   int group_b_stride;  // rows of B per group (mode 1); rows of D per group (mode 2)
   const int* m_block_group;     // mode 1: [num_m_blocks] expert of each 128-row block
   const int* num_m_blocks_dev;  // mode 1: actual number of row blocks (device scalar)
-  const int* group_offsets;     // mode 2: [G+1] padded row offsets (multiples of 128)
+  const int* group_offsets;     // mode 2: [G+1] padded row offsets (multiples of 128), or null: groups of K rows
   const int* seg_fill;          // mode 1 on short tiles: [G] rows in use of each expert's segment
   int* status;
 };
@@ -69,8 +69,8 @@ __device__ __forceinline__ Tile get_tile(const GemmArgs& g, int tile, int mb_tot
     const int r = tile - grp * per_group;
     const int m_blk = r % g.num_m_blocks;
     const int n_blk = r / g.num_m_blocks;
-    const int k0 = g.group_offsets[grp];
-    const int k1 = g.group_offsets[grp + 1];
+    const int k0 = g.group_offsets ? g.group_offsets[grp] : grp * g.K;
+    const int k1 = g.group_offsets ? g.group_offsets[grp + 1] : k0 + g.K;         // rows past the last one read as zero
     t.a_mn0 = m_blk * kBM;
     t.b_mn0 = n_blk * BN;
     t.a_k0 = k0;
@@ -428,7 +428,8 @@ extern "C" {
 //           (`M` is the allocated upper bound of rows). B holds `num_groups` matrices stacked on its
 //           row axis: [G*N, K] when K-major, [G*K, N] when MN-major.
 //   mode 2: per-expert wgrad: D[g] [M,N] = A[rows_g, M]^T B[rows_g, N] with
-//           rows_g = [group_offsets[g], group_offsets[g+1]); A and B MN-major; D is [G*M, N].
+//           rows_g = [group_offsets[g], group_offsets[g+1]); A and B MN-major; D is [G*M, N]. Without group_offsets
+//           rows_g = [g*K, (g+1)*K), of which `total_rows` end the last group.
 // out_mode: 0 bf16 store, 1 f32 store, 2 f32 reduce-add into D, 3 bf16 reduce-add into D.
 // `status` is a device int that receives a non-zero code if a bounded wait ran out (may be null).
 // `sm_limit` > 0 restricts the persistent grid (used to leave SMs to a concurrent kernel).
@@ -462,6 +463,10 @@ int mfb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, in
   } else {
     if (!a_mn_major || !b_mn_major) { mfb_host::set_error("gemm mode 2 needs MN-major A and B"); return 2; }
     if (M % kBM != 0) { mfb_host::set_error("gemm mode 2 needs M %% 128 == 0"); return 2; }
+    if (!group_offsets && (K <= 0 || K % kBK || (long long)K * num_groups >= 1LL << 31)) {
+      mfb_host::set_error("gemm mode 2: %d groups of %d rows", num_groups, K);
+      return 2;
+    }
     a_rows = total_rows;  a_cols = M;
     b_rows = total_rows;  b_cols = N;
     d_rows = (uint64_t)num_groups * M;

@@ -7,7 +7,6 @@ which is the library baseline the hand-written tcgen05 kernel is measured agains
 """
 from __future__ import annotations
 
-import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -1054,12 +1053,6 @@ _GATE_ROWS = 192
 _GATE_CHUNK = 256            # rows that a tensor-core sum of the weight's gradient spans
 
 
-@functools.lru_cache(maxsize=64)
-def _chunk_offsets(T: int, device: int) -> torch.Tensor:
-    """``[0, 256, 512, .., T]`` on the device; the copy has arrived when this returns."""
-    return torch.tensor(list(range(0, T, _GATE_CHUNK)) + [T], dtype=torch.int32).to(torch.device("cuda", device))
-
-
 class _GateFn(torch.autograd.Function):
     """``x W^T`` for bf16 rows and fp32 weights in 32-bit precision. Backward, an fp32 operand enters the tensor cores as three bf16 parts
     ``p0 + p1 + p2``; products of parts below 2^-24 of the whole are left out."""
@@ -1089,9 +1082,8 @@ class _GateFn(torch.autograd.Function):
                 return dx, torch.matmul(dy.t(), x.float())
             lib, groups = _lib.get_lib(), -(-T // _GATE_CHUNK)
             parts = torch.empty((groups * 3 * E, H), dtype=torch.float32, device=x.device)
-            rc = lib.mfb_gemm_bf16(d.data_ptr(), x.data_ptr(), parts.data_ptr(), 3 * E, H, 0, d.stride(0), x.stride(0), H, 1, 1, 1, 2, groups,
-                                   0, 0, _chunk_offsets(T, x.device.index).data_ptr(), T, _lib.status_word(x.device).data_ptr(), 0,
-                                   _lib.stream_ptr())
+            rc = lib.mfb_gemm_bf16(d.data_ptr(), x.data_ptr(), parts.data_ptr(), 3 * E, H, _GATE_CHUNK, d.stride(0), x.stride(0), H, 1, 1, 1, 2,
+                                   groups, 0, 0, 0, T, _lib.status_word(x.device).data_ptr(), 0, _lib.stream_ptr())
             _lib.check(rc, "mfb_gemm_bf16[gate]")
             dw = torch.empty((E, H), dtype=torch.float32, device=x.device)
             rc = lib.mfb_sum3(parts.data_ptr(), dw.data_ptr(), E, H, H, E * H, groups, 3 * E * H, _lib.stream_ptr())

@@ -75,3 +75,29 @@ def test_grouped_short_tiles(fills, N, K):
             want = a[rows].double() @ b[g].double()
             assert float((out[rows].double() - want).norm() / want.norm()) < 4e-3       # one rounding, at most 2^-8
     assert _lib.read_status() == 0
+
+
+def test_gate_backward_in_a_graph():
+    """The backward pass of a token count that was not there before can be captured."""
+    from mindformers_b200.ops import functional as Fn
+    torch.manual_seed(0)
+    x = torch.randn(700, 256, device=DEV).to(torch.bfloat16).requires_grad_()
+    w = torch.randn(128, 256, device=DEV).requires_grad_()
+    dy = torch.randn(700, 128, device=DEV)
+
+    def step(n):
+        return torch.autograd.grad(Fn.gate_logits(x[:n], w), (x, w), dy[:n])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step(700)
+        step(700)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step(513)
+    for t in got:
+        t.zero_()
+    graph.replay()
+    assert all(torch.equal(a, b) for a, b in zip(got, step(513)))
+    assert Fn._lib.read_status() == 0
