@@ -72,6 +72,12 @@ def apply_fn(fn, *args):
 
 
 
+def _plain_call() -> bool:
+    """No forward-mode level, function transform, trace or dispatch mode looks on, which a kernel on raw pointers would pass by."""
+    return not (torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+                or torch._C._len_torch_dispatch_stack() or torch.jit.is_tracing() or torch.compiler.is_compiling())
+
+
 def _cached_output(compute):
     from ..parallel.recompute import cached_output
     return cached_output(compute)
@@ -1072,6 +1078,8 @@ class _GateFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
+        if torch.is_grad_enabled():                                   # a graph of this pass is wanted: in operations that have derivatives
+            return (dy @ w).to(x.dtype) if ctx.needs_input_grad[0] else None, dy.t() @ x.float() if ctx.needs_input_grad[1] else None
         (T, E), H = dy.shape, w.shape[1]
         d = _split3(dy.contiguous(), True, 12001)                     # [T, 6 E]: d0 d1 d2 d0 d0 d1
         dx = dw = None
@@ -1093,7 +1101,7 @@ class _GateFn(torch.autograd.Function):
 
 
 def gate_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
-    return (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and x.dim() == w.dim() == 2 and x.shape[0] > 0
+    return (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and _plain_call() and x.dim() == w.dim() == 2 and x.shape[0] > 0
             and x.shape[1] == w.shape[1] and w.shape[0] % 8 == 0 and w.shape[1] % 64 == 0 and w.is_contiguous() and _aligned(x) and _aligned(w)
             and _GEMM_BACKEND == "tcgen05" and not torch.is_autocast_enabled())
 

@@ -101,3 +101,35 @@ def test_gate_backward_in_a_graph():
     graph.replay()
     assert all(torch.equal(a, b) for a, b in zip(got, step(513)))
     assert Fn._lib.read_status() == 0
+
+
+def _gate(x, w):
+    """The router's logits, by the kernels where they take the call."""
+    from mindformers_b200.ops import functional as Fn
+    return Fn.gate_logits(x, w) if Fn.gate_supported(x, w) else torch.nn.functional.linear(x.float(), w)
+
+
+@pytest.mark.parametrize("T", [40, 300])
+def test_gate_under_transforms(T):
+    """Second derivatives, forward mode, vmap and traces of the gate are those of the plain product."""
+    import torch.autograd.forward_ad as fwd
+    torch.manual_seed(T)
+    x = torch.randn(T, 64, device=DEV).to(torch.bfloat16).requires_grad_()
+    w = torch.randn(8, 64, device=DEV).requires_grad_()
+    seconds = []
+    for gate in (_gate, lambda x, w: torch.nn.functional.linear(x.float(), w)):
+        gx, gw = torch.autograd.grad(gate(x, w).pow(3).sum(), (x, w), create_graph=True)
+        seconds.append(torch.autograd.grad(gx.float().pow(2).sum() + gw.pow(2).sum(), (x, w)))
+    for a, b in zip(*seconds):
+        # the first pass adds up in another order (1e-6) and its gradient of x is rounded to bf16, at most 2^-8
+        assert (a.float() - b.float()).norm() / b.float().norm() < 8e-3
+    with torch.no_grad():
+        plain, xd, wd = torch.nn.functional.linear(x.float(), w), x.detach(), w.detach()
+        with fwd.dual_level():
+            out = fwd.unpack_dual(_gate(fwd.make_dual(xd, torch.ones_like(xd)), wd))
+        want = wd.sum(1).expand_as(out.tangent)
+        assert (out.tangent - want).norm() / want.norm() < 1e-5
+        both = torch.func.vmap(_gate, (0, None))(torch.stack((xd, xd)), wd)
+        assert (both[1] - plain).norm() / plain.norm() < 1e-5
+        traced = torch.jit.trace(_gate, (xd, wd), check_trace=False)
+        assert (traced(2 * xd, wd) - 2 * plain).norm() / plain.norm() < 1e-5
