@@ -1081,7 +1081,10 @@ class _GateFn(torch.autograd.Function):
         if torch.is_grad_enabled():                                   # a graph of this pass is wanted: in operations that have derivatives
             return (dy @ w).to(x.dtype) if ctx.needs_input_grad[0] else None, dy.t() @ x.float() if ctx.needs_input_grad[1] else None
         (T, E), H = dy.shape, w.shape[1]
-        d = _split3(dy.contiguous(), True, 12001)                     # [T, 6 E]: d0 d1 d2 d0 d0 d1
+        dy = dy.contiguous()
+        if dy.data_ptr() % 16:                                        # a view into a larger gradient
+            dy = dy.clone()
+        d = _split3(dy, True, 12001)                                  # [T, 6 E]: d0 d1 d2 d0 d0 d1
         dx = dw = None
         if ctx.needs_input_grad[0]:
             dx = gemm(d, _split3(w, False, 121), b_mn=True)           # against  w0 w0 w0 w1 w2 w1
@@ -1102,7 +1105,7 @@ class _GateFn(torch.autograd.Function):
 
 def gate_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
     return (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.float32 and _plain_call() and x.dim() == w.dim() == 2 and x.shape[0] > 0
-            and x.shape[1] == w.shape[1] and w.shape[0] % 8 == 0 and w.shape[1] % 64 == 0 and w.is_contiguous() and _aligned(x) and _aligned(w)
+            and x.shape[1] == w.shape[1] and x.stride(0) >= x.shape[1] and w.shape[0] % 8 == 0 and w.shape[1] % 64 == 0 and w.is_contiguous() and _aligned(x) and _aligned(w)
             and _GEMM_BACKEND == "tcgen05" and not torch.is_autocast_enabled())
 
 

@@ -133,3 +133,22 @@ def test_gate_under_transforms(T):
         assert (both[1] - plain).norm() / plain.norm() < 1e-5
         traced = torch.jit.trace(_gate, (xd, wd), check_trace=False)
         assert (traced(2 * xd, wd) - 2 * plain).norm() / plain.norm() < 1e-5
+
+
+def test_gate_on_views():
+    """A gradient that starts between two 16-byte boundaries; rows that are one row repeated."""
+    from mindformers_b200.ops import functional as Fn
+    torch.manual_seed(0)
+    T, E, H = 300, 128, 64
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16).requires_grad_()
+    w = torch.randn(E, H, device=DEV).requires_grad_()
+    dy = torch.randn(T * E + 1, device=DEV)[1:].view(T, E)
+    got = torch.autograd.grad(Fn.gate_logits(x, w), (x, w), dy)
+    want = torch.autograd.grad(Fn.gate_logits(x, w), (x, w), dy.clone())
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    row = x.detach()[:1].expand(T, H).requires_grad_()
+    logits = _gate(row, w)
+    grads = torch.autograd.grad(logits, (row, w), dy)
+    plain = torch.nn.functional.linear(row.float(), w)
+    for a, b in zip((logits, *grads), (plain, *torch.autograd.grad(plain, (row, w), dy))):
+        assert (a.float() - b.float()).norm() / b.float().norm() < 8e-3          # bf16 gradients, at most 2^-8 on either side
