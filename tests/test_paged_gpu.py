@@ -423,3 +423,37 @@ def test_latent_prefill_of_few_rows():
         kv = (lat[:, :512] @ w.double().t()).view(m, heads, 256)
         want = _attend(q[rows], torch.cat((kv[..., :128], lat[:, None, 512:].expand(m, heads, 64)), -1), kv[..., 128:], attn.scale)
         assert (got[rows].double() - want).norm() / want.norm() < 2e-3           # rounding of the result alone
+
+
+def _latent_layer(**over):
+    from mindformers_b200.models.presets import get_preset
+    from mindformers_b200.parallel.layers.attention import MLASelfAttention
+    from mindformers_b200.parallel.layers.rotary import get_rope
+    from mindformers_b200.parallel.transformer_config_utils import convert_to_transformer_config
+    cfg = get_preset("deepseek_v3", num_attention_heads=4, num_key_value_heads=4, hidden_size=256, max_position_embeddings=512, **over)
+    cfg.update(params_dtype="bfloat16", compute_dtype="bfloat16")
+    cfg = convert_to_transformer_config(cfg, is_mla_model=True)
+    cfg.device = DEV
+    return MLASelfAttention(cfg).eval(), get_rope(cfg, device=DEV)()
+
+
+@pytest.mark.parametrize("prefill", [True, False])
+def test_latent_layer_leaves_its_projections_alone(prefill):
+    """What a forward hook keeps of a projection's output in serving is that output."""
+    from mindformers_b200.inference import paged_attention as pa
+    from mindformers_b200.parallel.layers.attention import AttnMeta
+    torch.manual_seed(0)
+    layer, rotary = _latent_layer()
+    lens = [40, 70, 3]
+    news = [7, 20, 3] if prefill else [1] * 3
+    tables, blocks = _tables(lens, 16)
+    ctx = pa.KVCacheContext(1, blocks, 16, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
+    ctx.set_step(is_prefill=prefill, slot_mapping=_slots(tables, 16, lens, news).numpy(), q_seq_lens=news, block_tables=tables.numpy(),
+                 context_lens=lens, device=DEV)
+    pos = torch.cat([torch.arange(n - m, n) for n, m in zip(lens, news)]).to(DEV)
+    x = torch.randn(sum(news), 256, device=DEV).to(torch.bfloat16)
+    kept = []
+    layer.linear_qkv.register_forward_hook(lambda mod, args, out: kept.append(out[0]))
+    with torch.no_grad():
+        layer(x, rotary, AttnMeta(batch=1, seq_len=sum(news), positions=pos, cache=ctx))
+        assert torch.equal(kept[0], layer.linear_qkv(x)[0])
