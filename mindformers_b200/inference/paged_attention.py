@@ -465,6 +465,8 @@ def _decode_step(q, k, v, cache, layer: int, scale: float):
         if rc <= 0:
             break
         need = rc
+    if rc == -2:
+        return _decode_step(*(t.clone(memory_format=torch.contiguous_format) for t in (q, k, v)), cache, layer, scale)
     if rc == -1:
         return None
     _lib.check(rc, "mfb_paged_decode_step")

@@ -27,18 +27,19 @@ long long mfb_paged_decode_scratch_bytes(int B, int Hq, int hd, int splits);
 
 // q [B, Hq, hd], k / v [B, Hkv, hd] bf16, strides in elements; caches [num_blocks, block_size, Hkv, hd] bf16, or int8 with scales
 // [num_blocks, block_size, Hkv]; out [B, Hq, hd]. 0: launched. Positive: nothing was launched, that many bytes of scratch are needed.
-// -1: nothing was launched, the general path takes the call. Others: an error of a launch.
+// -1: nothing was launched, the general path takes the call. -2: likewise, but for contiguous q, k and v. Others: an error of a launch.
 long long mfb_paged_decode_step(const void* q, long long q0, long long q1, long long q2, const void* k, long long k0, long long k1,
                                 long long k2, const void* v, long long v0, long long v1, long long v2, void* key_cache,
                                 void* value_cache, float* key_scale, float* value_scale, const int* slots, const int* tables,
                                 const int* lens, void* out, void* scratch, long long scratch_bytes, int B, int Hq, int Hkv, int hd,
                                 int num_blocks, int block_size, int max_blocks, float scale, int* status, cudaStream_t stream) {
-  auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
-  if (B < 1 || q2 != 1 || k2 != 1 || v2 != 1 || k1 != hd || v1 != hd || q1 < hd || q0 < hd || q1 % 8 || q0 % 8 || k0 % 8 || v0 % 8 ||
-      off16(q) || off16(k) || off16(v) || off16(key_cache) || off16(value_cache))
-    return -1;
   const bool i8 = key_scale != nullptr;
-  if (i8 ? !mfb_paged_decode_int8_supported(Hq, Hkv, hd, block_size) : !mfb_paged_decode_tc_supported(Hq, Hkv, hd, block_size)) return -1;
+  if (B < 1 || (i8 ? !mfb_paged_decode_int8_supported(Hq, Hkv, hd, block_size) : !mfb_paged_decode_tc_supported(Hq, Hkv, hd, block_size))) return -1;
+  auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  if (off16(key_cache) || off16(value_cache)) return -1;
+  if (q2 != 1 || k2 != 1 || v2 != 1 || k1 != hd || v1 != hd || q1 < hd || q0 < hd || q1 % 8 || q0 % 8 || k0 % 8 || v0 % 8 ||
+      off16(q) || off16(k) || off16(v))
+    return i8 ? -1 : -2;
   const int splits = i8 ? mfb_paged_decode_int8_splits(B, Hkv, max_blocks * block_size) : mfb_paged_decode_tc_splits(B, Hkv, max_blocks * block_size);
   const long long need = mfb_paged_decode_scratch_bytes(B, Hq, hd, splits);
   if (scratch_bytes < need) return need;

@@ -457,3 +457,25 @@ def test_latent_layer_leaves_its_projections_alone(prefill):
     with torch.no_grad():
         layer(x, rotary, AttnMeta(batch=1, seq_len=sum(news), positions=pos, cache=ctx))
         assert torch.equal(kept[0], layer.linear_qkv(x)[0])
+
+
+@pytest.mark.parametrize("which", ["query columns", "keys interleaved", "values off by one"])
+def test_decode_of_other_layouts(which):
+    """Rows of a bf16 step that no tensor map describes run on the tensor cores like others."""
+    from mindformers_b200.inference import paged_attention as pa
+    ctx, step, _ = _decode_call()
+    x = torch.randn(3, 8, 128, device=DEV).to(torch.bfloat16)
+    plain = [x[:, :4].contiguous(), x[:, 4:6].contiguous(), x[:, 6:].contiguous()]
+    q, k, v = plain
+    if which == "query columns":
+        q = q.transpose(1, 2).contiguous().transpose(1, 2)
+    elif which == "keys interleaved":
+        k = torch.stack((k, k), 2)[:, :, 0]
+    else:
+        v = torch.cat((v.flatten(), v.flatten()[:1])).roll(1)[1:].view(3, 2, 128)
+    ctx.set_step(**step)
+    with torch.no_grad():
+        want = pa._decode_step(*plain, ctx, 0, 0.09)
+        ctx.key_cache[0].view(-1, 2, 128)[ctx.slot_mapping.long()] = 0
+        got = pa._decode_step(q, k, v, ctx, 0, 0.09)
+    assert got is not None and torch.equal(got, want)
