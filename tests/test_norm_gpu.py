@@ -64,3 +64,19 @@ def test_qk_norm(T, nq, nkv, hd, buffers):
         if buffers:
             assert w.grad is None
         _close(w.main_grad - 3.0 if buffers else w.grad, ref.grad, 4e-3)
+
+
+def test_swiglu_in_several_launches():
+    """Rows so wide that the vector indexes of a launch would pass 2^31 with more than one of them."""
+    from mindformers_b200.ops import functional as Fn
+    torch.manual_seed(0)
+    T, F = 3, 1 << 24
+    x = torch.randn(T, 2 * F, device=DEV, dtype=torch.bfloat16).requires_grad_()
+    dy = torch.randn(T, F, device=DEV, dtype=torch.bfloat16)
+    y = Fn.swiglu(x)
+    dx = torch.autograd.grad(y, x, dy)[0]
+    for t in range(T):
+        row = x.detach()[t].float().requires_grad_()
+        want = torch.nn.functional.silu(row[:F]) * row[F:]
+        _close(y[t].detach(), want.detach().double(), 4e-3)              # rounded once, at most 2^-8 of every number
+        _close(dx[t], torch.autograd.grad(want, row, dy[t].float())[0].double(), 4e-3)

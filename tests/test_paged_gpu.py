@@ -479,3 +479,152 @@ def test_decode_of_other_layouts(which):
         ctx.key_cache[0].view(-1, 2, 128)[ctx.slot_mapping.long()] = 0
         got = pa._decode_step(q, k, v, ctx, 0, 0.09)
     assert got is not None and torch.equal(got, want)
+
+
+def _bits(t):
+    return t.view(torch.int16 if t.dtype == torch.bfloat16 else torch.int32 if t.dtype == torch.float32 else t.dtype)
+
+
+@pytest.mark.parametrize("heads,kv,block", [(8, 2, 16), (4, 4, 128)])
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("fused", [True, False])
+def test_new_rows_reach_the_cache(heads, kv, block, int8, fused):
+    """The rows of a step lie in its slots, in no others, and a row without a slot nowhere; ``fused``: written by the call that attends."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(kv)
+    dim, B = 128, 5
+    ctx = pa.KVCacheContext(1, 12, block, kv, dim, torch.bfloat16, DEV, kv_cache_dtype="int8" if int8 else None)
+    caches = [ctx.key_cache[0], ctx.value_cache[0]]
+    scales = [ctx.key_scale[0], ctx.value_scale[0]] if int8 else []
+    for c in caches:
+        c.fill_(77 if int8 else float("nan"))
+    for s in scales:
+        s.fill_(float("inf"))
+    before = [t.clone() for t in caches + scales]
+    tables = torch.randperm(10).view(B, 2).to(torch.int32)
+    lens = [1, block, block + 1, 2 * block, 7]
+    slots = _slots(tables, block, lens, [1] * B)
+    slots[3] = -1
+    ctx.set_step(is_prefill=False, block_tables=tables.numpy(), slot_mapping=slots.numpy(), context_lens=lens, q_seq_lens=[1] * B, device=DEV)
+    x = torch.randn(B, heads + 2 * kv, dim, device=DEV).to(torch.bfloat16)
+    x[1] = 0                                                # a row of zeros has scale one
+    k, v = x[:, heads:heads + kv], x[:, heads + kv:]
+    with torch.no_grad():
+        if fused:
+            assert pa._decode_step(x[:, :heads], k, v, ctx, 0, 0.09) is not None
+        else:
+            pa._write_cache(ctx, 0, k, v)
+    used = [0, 1, 2, 4]
+    at = slots[used].to(DEV)
+    for i, (cache, rows) in enumerate(zip(caches, (k, v))):
+        got, rows = cache.view(-1, kv, dim)[at], rows[used]
+        if int8:
+            top = rows.float().abs().amax(-1)
+            scale = torch.where(top > 0, top / 127, torch.ones_like(top))
+            assert torch.allclose(scales[i].view(-1, kv)[at], scale, rtol=1e-6)
+            # codes are the nearest ones: half a step, and what a reciprocal instead of a division adds
+            assert ((got.float() * scale.unsqueeze(-1) - rows.float()).abs() <= scale.unsqueeze(-1) * 0.5001).all()
+        else:
+            assert torch.equal(got, rows)
+    for now, old in zip(caches + scales, before):
+        now, old = (_bits(t).flatten(0, 1).clone() for t in (now, old))
+        now[at] = old[at]
+        assert torch.equal(now, old)
+
+
+@pytest.mark.parametrize("view", [True, False])
+def test_latents_reach_the_cache(view):
+    """``view``: the parts are columns of wider rows that start on 16 bytes; otherwise on other addresses (the general path)."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(0)
+    ctx = pa.KVCacheContext(1, 6, 16, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
+    ctx.key_cache[0].fill_(float("nan"))
+    before = ctx.key_cache[0].clone()
+    slots = torch.randperm(96)[:33]
+    slots[5] = -1
+    ctx.set_step(is_prefill=True, block_tables=[[0, 1, 2, 3, 4, 5]], slot_mapping=slots.numpy(), context_lens=[33], q_seq_lens=[33], device=DEV)
+    wide = torch.randn(33, 640, device=DEV).to(torch.bfloat16)
+    at = 16 if view else 3
+    pa._write_latents(ctx, 0, wide[:, at:at + 512], wide[:, at + 512:at + 576])
+    used = [i for i in range(33) if i != 5]
+    to = slots[used].to(DEV)
+    rows = ctx.key_cache[0].view(-1, 576)
+    assert torch.equal(rows[to], wide[used, at:at + 576])
+    rest, old = _bits(rows).clone(), _bits(before).view(-1, 576)
+    rest[to] = old[to]
+    assert torch.equal(rest, old)
+
+
+@pytest.mark.parametrize("T,heads,hd,rot,left", [(1, 1, 64, 64, 32), (33, 1, 64, 64, 64), (33, 5, 192, 64, 0), (1, 3, 192, 64, 0), (7, 2, 40, 24, 0)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rope_of_heads_in_place(T, heads, hd, rot, left, interleaved):
+    """The last columns of every head, in rows that may be a slice of wider ones; the other columns keep their bits."""
+    from mindformers_b200.ops import functional as Fn
+    torch.manual_seed(T)
+    wide = torch.randn(T, left + heads * hd + 8 * (left > 0), device=DEV).to(torch.bfloat16)
+    old = wide.clone()
+    angle = torch.rand(50, rot // 2, device=DEV) * 6
+    cos, sin, pos = angle.cos(), angle.sin(), torch.randint(0, 50, (T,), device=DEV)
+    view = lambda t: t[:, left:left + heads * hd].view(T, heads, hd)
+    assert Fn.rope_heads_supported(view(wide), rot)
+    Fn.rope_heads_(view(wide), cos, sin, pos.to(torch.int32), rot, interleaved)
+    want = Fn.rope_reference(view(old)[..., hd - rot:].contiguous(), cos, sin, pos, heads, rot, interleaved)
+    got = view(wide)[..., hd - rot:]
+    # rounded once, at most 2^-8 of a number; a difference of two products may cancel, so relative to the pair
+    assert (got.float() - want.float()).abs().max() <= 2 ** -8 * 2 * want.float().abs().max()
+    view(old)[..., hd - rot:] = got
+    assert torch.equal(_bits(wide), _bits(old))
+
+
+@pytest.mark.parametrize("heads", [16, 17, 64, 128])
+@pytest.mark.parametrize("block", [16, 128])
+def test_latent_decode_of_idle_rows(heads, block):
+    """Sequences of no tokens and rows without blocks give zeros and leave the others as they are; large numbers behind a sequence's end
+    have no effect."""
+    from mindformers_b200.inference import paged_attention as pa
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(heads)
+    lens = [300, 0, 130, 5, 1]
+    tables, blocks = _tables([300, 1, 130, 5, 1], block)
+    cache = torch.full((blocks, block, 1, 576), 1e30, device=DEV).to(torch.bfloat16)
+    for b, n in enumerate(lens):
+        for i in range(-(-n // block)):
+            rows = min(block, n - i * block)
+            cache[tables[b, i].long(), :rows] = torch.randn(rows, 1, 576, device=DEV).to(torch.bfloat16)
+    want = cache.clone()
+    tables[3] = -1                                          # an idle slot: a length, no blocks
+    q = torch.randn(5, heads, 576, device=DEV).to(torch.bfloat16)
+    got = pa.mla_decode_attention(q, cache, tables.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), block, 192 ** -0.5)
+    assert not got[1].any() and not got[3].any()
+    for b in (0, 2, 4):
+        lat = _cached(want[:, :, 0], tables, b, lens[b], block).double()
+        ref = torch.softmax(q[b].double() @ lat.t() * 192 ** -0.5, -1) @ lat[:, :512]
+        assert (got[b].double() - ref).norm() / ref.norm() < 4e-3        # as above
+    assert _lib.read_status() == 0
+
+
+def test_prefill_with_gradients():
+    """A call whose result needs a gradient goes through operations that have one."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(0)
+    ctx = pa.KVCacheContext(1, 16, 16, 2, 64, torch.bfloat16, DEV)
+    x = torch.randn(128, 8, 64, device=DEV).to(torch.bfloat16).requires_grad_()
+    tables, _ = _tables([128], 16)
+    _set(ctx, tables, 16, [128], [128])
+
+    def call(x):
+        return pa.paged_attention_forward(x[:, :4], x[:, 4:6], x[:, 6:], types.SimpleNamespace(cache=ctx), 1, 0.125)
+    out = call(x)
+    dy = torch.randn_like(out)
+    got = torch.autograd.grad(out, x, dy)[0]
+    x64 = x.detach().double().requires_grad_()
+    q, k, v = x64[:, :4], x64[:, 4:6].repeat_interleave(2, 1), x64[:, 6:].repeat_interleave(2, 1)
+    s = torch.einsum("qhd,khd->hqk", q, k) * 0.125
+    hide = torch.ones(128, 128, device=DEV, dtype=torch.bool).triu(1)
+    ref = torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(hide, float("-inf")), -1), v).flatten(1)
+    want = torch.autograd.grad(ref, x64, dy.double())[0]
+    # the weights, their gradients and the results are rounded to 16 bits, at most 2^-8 each
+    assert (got.double() - want).norm() / want.norm() < 1.2e-2
+    with torch.no_grad():
+        plain = call(x)
+    assert (plain.double() - ref.detach()).norm() / ref.detach().norm() < 4e-3
