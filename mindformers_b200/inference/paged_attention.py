@@ -329,11 +329,12 @@ _PERSISTENT_UP_TO = 8.0
 
 class _PrefillPlan:
     """What the prefill kernels need to know about a step: per query tile ``(sequence, first row of q, rows, position of the first
-    row)``, longest first, for the sequences whose keys are all new (``fresh``) and for those with cached ones (``past``); the first
-    row of every sequence in q, and in a gathered copy of all cached rows that a step with history sees. ``ok`` False: a step that
+    row)``, longest first, for the sequences whose keys are all new (``fresh``) and for those with cached ones (``past``), or for both
+    (``all``, caches of latents); the first row of every sequence in q (``cu``), and in a gathered copy of the cached rows that the sequences
+    with history see (``past_rows``) or all that have new rows (``all_rows``). ``ok`` False: a step that
     these kernels do not take (a sequence longer than its block table or without one, rows that are not there, tables of another form)."""
 
-    def __init__(self, cache, rows: int, lens: list):
+    def __init__(self, cache, rows: int, lens: list, latent: bool):
         cu = cache.cu_q
         B = len(lens)
         tables = cache._block_tables
@@ -344,24 +345,25 @@ class _PrefillPlan:
         self.ok = 0 < self.rows <= rows and len(news) == B and cu[0] == 0 and all(0 <= n <= m <= reach for n, m in zip(news, lens) if n)
         if not self.ok:
             return
-        tiles = {False: [], True: []}
-        gather = {False: [0], True: [0]}       # of the sequences with history / of all that have new rows
+        fresh, seeing = [], []
+        first = [0]                            # rows of the copy
         for b, (n, m) in enumerate(zip(news, lens)):
-            tiles[n < m] += [(b, cu[b] + r, min(_TILE, n - r), m - n + r) for r in range(0, n, _TILE)]
-            gather[False].append(gather[False][-1] + (m if 0 < n < m else 0))
-            gather[True].append(gather[True][-1] + (m if n else 0))
-        flat, spans = [], []
-        for items in (tiles[False], tiles[True], tiles[False] + tiles[True]):
-            spans.append(self._add(flat, items))
+            copied = n and (latent or n < m)
+            (seeing if copied else fresh).extend((b, cu[b] + r, min(_TILE, n - r), m - n + r) for r in range(0, n, _TILE))
+            first.append(first[-1] + (m if copied else 0))
+        flat, self.longest = [], max(lens)
+        spans = [self._add(flat, items) for items in (fresh, seeing)]
         at = len(flat)
-        flat += list(cu) + gather[False] + gather[True]
-        dev, = _to_device([np.asarray(flat, np.int32)], cache._block_tables.device)
-        self.fresh, self.past, self.all = ((dev[a:a + 4 * n], n, p) for a, n, p in spans)
-        self.cu, self.past_rows, self.all_rows = (dev[at + i * (B + 1):at + (i + 1) * (B + 1)] for i in range(3))
-        self.n_past_rows, self.n_all_rows, self.longest = gather[False][-1], gather[True][-1], max(lens)
-        self.past_host = (tiles[True], gather[False])
-        self.groups, self.forms = {}, {}
-        self.new_and_seen = [(n, m) for n, m in zip(news, lens) if n]
+        dev, = _to_device([np.asarray(flat + list(cu) + first, np.int32)], tables.device)
+        (a, n, p), (b, m, s) = spans
+        works = (dev[a:a + 4 * n], n, p), (dev[b:b + 4 * m], m, s)
+        cu_dev, rows_dev = dev[at:at + B + 1], dev[at + B + 1:]
+        if latent:
+            self.all, self.all_rows, self.n_all_rows, self.forms = works[1], rows_dev, first[-1], {}
+            self.new_and_seen = [(n, m) for n, m in zip(news, lens) if n]
+        else:
+            (self.fresh, self.past), self.cu, self.past_rows, self.n_past_rows = works, cu_dev, rows_dev, first[-1]
+            self.past_host, self.groups = (seeing, first), {}
 
     def expands(self, heads: int) -> bool:
         """Whether multi-latent attention of ``heads`` heads expands the cached latents (one product over all rows that the step sees, whatever
@@ -412,13 +414,14 @@ class _PrefillPlan:
         return self.groups[limit]
 
 
-def _prefill_plan(cache, rows: int) -> _PrefillPlan:
-    """The step's plan, shared by its layers: kept while all that it follows from has the values it had, on the stream that made it."""
+def _prefill_plan(cache, rows: int, latent: bool = False) -> _PrefillPlan:
+    """The step's plan, shared by its layers: kept while all that it follows from has the values it had, on the stream that made it. A cache of
+    latents wants other lists than one of keys and values."""
     lens, tables = _host_lens(cache), cache._block_tables
-    key = (rows, tuple(lens), tuple(cache.cu_q), tables.shape, cache.block_size, _lib.stream_ptr() if tables.is_cuda else 0)
+    key = (rows, latent, tuple(lens), tuple(cache.cu_q), tables.shape, cache.block_size, _lib.stream_ptr() if tables.is_cuda else 0)
     plan = cache.prefill_work.get("plan")
     if plan is None or plan.key != key:
-        plan = cache.prefill_work["plan"] = _PrefillPlan(cache, rows, lens)
+        plan = cache.prefill_work["plan"] = _PrefillPlan(cache, rows, lens, latent)
         plan.key = key
     return plan
 
@@ -658,7 +661,7 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
     if not (q_nope.is_cuda and q_nope.dtype == q_pe.dtype == rows.dtype == w.dtype == torch.bfloat16 and (nope, rope_d, vd) == (128, 64, 128)
             and rank % 8 == 0 and T and w.is_contiguous() and rows.is_contiguous() and Fn.get_gemm_backend() == "tcgen05") or _needs_graph(q_nope, q_pe, w):
         return None
-    plan = _prefill_plan(cache, T)
+    plan = _prefill_plan(cache, T, latent=True)
     n = plan.n_all_rows if plan.ok else 0
     if not plan.ok or n >= 1 << 31 or plan.longest * (rank + rope_d) >= 1 << 34 or not plan.expands(nh):
         return None

@@ -414,7 +414,7 @@ def test_latent_prefill_of_few_rows():
     q = torch.randn(3, heads, 192, device=DEV).to(torch.bfloat16)
     new = torch.randn(3, 576, device=DEV).to(torch.bfloat16)
     _set(ctx, tables, block, lens, news)
-    assert not pa._prefill_plan(ctx, 3).expands(heads)
+    assert not pa._prefill_plan(ctx, 3, latent=True).expands(heads)
     with torch.no_grad():
         got = pa.mla_paged_attention_forward(attn, q[..., :128], q[..., 128:].clone(), new[:, :512], new[:, 512:],
                                              types.SimpleNamespace(cache=ctx))

@@ -69,7 +69,7 @@ def test_form_of_latent_attention():
     """Few new rows behind long histories are not worth expanding every cached latent for all heads."""
     def expands(B, past, new, heads):
         ctx = _ctx(np.zeros((B, (past + new) // 16 + 1), np.int32), [past + new] * B, [new] * B)
-        return pa._prefill_plan(ctx, B * new).expands(heads)
+        return pa._prefill_plan(ctx, B * new, latent=True).expands(heads)
     assert not expands(32, 8000, 1, 128) and not expands(32, 8000, 4, 128) and expands(32, 8000, 64, 128)
     assert not expands(1, 8000, 4, 128) and expands(1, 8000, 64, 128)
     assert expands(32, 8000, 1, 16) and expands(4, 1200, 900, 16) and expands(32, 500, 1, 128)
