@@ -308,9 +308,9 @@ def _layer_scales(cache, layer):
     return None, None
 
 
-# Decode attention over a bf16 cache with head dim 128 runs on the tensor cores (``paged_decode_tc.cu``);
-# ``MFB_PAGED_DECODE=cuda_core`` (or ``set_paged_decode_kernel``) keeps the split-KV kernel on the CUDA cores, which also
-# serves head dim 64 and the int8 cache.
+# Decode attention runs on the tensor cores: ``paged_decode_tc.cu`` over a bf16 cache with head dim 128, ``paged_decode_int8.cu`` over an
+# int8 cache with blocks of a multiple of 16 tokens. ``MFB_PAGED_DECODE=cuda_core`` (or ``set_paged_decode_kernel``) keeps the split-KV
+# kernel on the CUDA cores, which also serves what those two do not take: a bf16 cache with head dim 64, other block sizes.
 _DECODE_KERNEL = "cuda_core" if os.environ.get("MFB_PAGED_DECODE", "tensor_core") == "cuda_core" else "tensor_core"
 
 

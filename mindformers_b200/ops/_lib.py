@@ -102,7 +102,6 @@ def _declare(lib):
     sig("mfb_mla_decode_scratch_bytes", [I, I, I], L)
     sig("mfb_gather_cache2", [P, P, P, P, P, P, I, I, I, I, I, P])
     sig("mfb_latent_to_cache", [P, L, P, L, P, P, L, I, I, P])
-    sig("mfb_gather_cache", [P, P, P, P, I, I, I, I, I, P])
     sig("mfb_ll_allreduce_buffer_bytes", [I, L], L)
     sig("mfb_ll_allreduce_state_words", [])
     sig("mfb_ll_allreduce_init", [P, L, P])
@@ -150,13 +149,9 @@ def _declare(lib):
     sig("mfb_quant_act_int8", [P, L, P, L, P, P, L, I, P])
     sig("mfb_paged_decode_tc_supported_ex", [I, I, I, I, I])
     sig("mfb_paged_decode_attention_tc_ex", [P] * 9 + [I] * 13 + [F, F, L, F, P, P])
-    sig("mfb_paged_decode_attention_tc_q", [P, L, L] + [P] * 8 + [I] * 13 + [F, F, L, F, P, P])
     sig("mfb_paged_decode_step", [P, L, L, L, P, L, L, L, P, L, L, L] + [P] * 9 + [L] + [I] * 7 + [F, P, P], L)
     sig("mfb_event_done", [P, I])
     sig("mfb_event_record", [P, P])
-    sig("mfb_paged_decode_int8_supported", [I, I, I, I])
-    sig("mfb_paged_decode_int8_splits", [I, I, I])
-    sig("mfb_paged_decode_attention_int8", [P, L, L] + [P] * 8 + [I] * 7 + [F, P])
     sig("mfb_paged_prefill_tc_supported", [I, I, I, I, I])
     sig("mfb_paged_prefill_tc_wide_supported", [I, I, I, I, I])
     sig("mfb_paged_prefill_tc", [P, P, P, P, I, I, P, P, P] + [I] * 11 + [L, L, F, F, L, F, P, P])

@@ -499,8 +499,8 @@ int mfb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, in
   return dispatch<128, 6>(a_mn_major, b_mn_major, out_mode, tA, tB, tD, args, max_tiles, sm_limit, stream);
 }
 
-// Mode 1 of the above (B [G, K, N], MN-major; bf16 result) for a few rows per expert: rows of A past an expert's seg_fill are not read, rows
-// of D past it are undefined.
+// Mode 1 of the above (B [G, K, N], MN-major; bf16 result) for a few rows per expert: rows of A past an expert's seg_fill have no effect
+// (tiles of 32 rows without one in use are not read at all), rows of D past it are undefined.
 int mfb_gemm_bf16_grouped_short(const void* A, const void* B, void* D, int rows, int N, int K, int lda, int ldb, int ldd, int num_groups,
                                 const int* m_block_group, const int* num_m_blocks_dev, const int* group_offsets, const int* seg_fill,
                                 int* status, cudaStream_t stream) {

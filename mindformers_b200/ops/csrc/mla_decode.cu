@@ -4,7 +4,7 @@
 // absorbed into the query, one decode step is, per sequence and head h:
 //     s[t]   = scale * <q[h, 0:576], c[t, 0:576]>          t < len
 //     o[h,:] = sum_t softmax(s)[t] * c[t, 0:512]
-// A CTA handles (split of the sequence, chunk of 16 heads, sequence). The products are laid out TRANSPOSED so
+// A CTA handles (split of the sequence, sequence) for up to 16 heads. The products are laid out TRANSPOSED so
 // that the token dimension, not the (small) head count, fills the 128 rows of the tensor core:
 //     S^T [128 tokens x 16 heads]   = C_tile [128 x 576] (A, K-major) . Q^T (B, K-major)          -> TMEM, 16 columns
 //     O^T [512 x 16]  (4 x M=128)  += C_tile^T (A, MN-major: the same bytes) . P^T [16 heads x 128 tokens] (B, K-major)
@@ -27,7 +27,7 @@ namespace mfb {
 
 constexpr int kMlaThreads = 192;
 constexpr int kMlaTile = 128;              // tokens per tile
-constexpr int kMlaHeads = 16;              // heads per CTA
+constexpr int kMlaHeads = 16;              // heads at most
 constexpr int kMlaRank = 512;
 constexpr int kMlaRope = 64;
 constexpr int kMlaDim = kMlaRank + kMlaRope;
@@ -77,14 +77,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int split = blockIdx.x, chunk = blockIdx.y, b = blockIdx.z;
+  const int split = blockIdx.x, b = blockIdx.y;
   const int len = args.context_lens[b];
   const int n_tiles_all = (len + kMlaTile - 1) / kMlaTile;
   const int per = (n_tiles_all + args.splits - 1) / args.splits;
   const int t0 = split * per;
   const int t1 = (t0 + per < n_tiles_all) ? t0 + per : n_tiles_all;
   const int n_tiles = t1 > t0 ? t1 - t0 : 0;
-  const int head0 = chunk * kMlaHeads;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -121,7 +120,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const uint32_t qb = smem_u32(q_full);
       mbar_expect_tx(qb, kMlaQBytes);
       for (int c = 0; c < 9; ++c)
-        tma_load_2d(smem_u32(sQ) + c * kMlaQSub, &tmQ, qb, c * 64, b * args.num_heads + head0);
+        tma_load_2d(smem_u32(sQ) + c * kMlaQSub, &tmQ, qb, c * 64, b * args.num_heads);
       const int bs = args.block_size;
       const int pages = kMlaTile / bs;            // pages per tile (block_size divides 128)
       const int* table = args.block_tables + static_cast<size_t>(b) * args.max_blocks;
@@ -316,13 +315,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int h = 0; h < kMlaHeads; ++h)
       l_tot[h] = (red[h] + red[kMlaHeads + h]) + (red[2 * kMlaHeads + h] + red[3 * kMlaHeads + h]);
     const size_t ps = static_cast<size_t>(b) * args.splits + split;
-    if (row < kMlaHeads && head0 + row < args.num_heads) {
+    if (row < args.num_heads) {
       float mh = -INFINITY, lh = 0.f;
 #pragma unroll
       for (int h = 0; h < kMlaHeads; ++h)
         if (h == row) { mh = m_used[h]; lh = l_tot[h]; }
       if (!ok || n_tiles == 0) { mh = -INFINITY; lh = 0.f; }
-      float* ml = args.part_ml + (ps * args.num_heads + head0 + row) * 2;
+      float* ml = args.part_ml + (ps * args.num_heads + row) * 2;
       ml[0] = mh;
       ml[1] = lh;
     }
@@ -335,8 +334,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         tmem_ld_wait();
 #pragma unroll
         for (int h = 0; h < kMlaHeads; ++h) {
-          if (head0 + h < args.num_heads)
-            args.part_o[(ps * args.num_heads + head0 + h) * kMlaRank + m * 128 + row] = __uint_as_float(r[h]);
+          if (h < args.num_heads)
+            args.part_o[(ps * args.num_heads + h) * kMlaRank + m * 128 + row] = __uint_as_float(r[h]);
         }
       }
     }
@@ -402,7 +401,7 @@ mla_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ p
 extern "C" {
 using namespace mfb;
 
-// Kernel variant: 0 = one CTA per (sequence, split, head chunk), two passes over the cache (this file);
+// Kernel variant: 0 = up to 16 heads: one CTA per (sequence, split), two passes over the cache (this file), more: mla_decode_heads.cu;
 // 1 = a cluster of two CTAs that split the latent columns, one pass (mla_decode_cluster.cu).
 static int g_mla_variant = 0;
 int mfb_mla_cluster_splits(int B, int num_heads, int max_len);
@@ -413,9 +412,9 @@ int mfb_mla_decode_heads_splits(int B, int num_heads, int max_len);
 int mfb_mla_decode_heads_launch(const void* q, const void* cache, const int* block_tables, const int* context_lens, float* part_o,
                                 float* part_ml, int splits, int B, int num_heads, int num_blocks, int block_size, int max_blocks,
                                 float scale, int* status, cudaStream_t stream);
-// More than one chunk of 16 heads: heads on the rows (mla_decode_heads.cu), which reads a tile 1.4 times for all of them where this file's
-// kernel reads it twice per chunk: 32 heads, 32 x 2304 / 8 x 4000 / 64 x 1500 tokens 42 / 34 / 56 us against 58 / 38 / 68 us, 128 heads 56 / 36 /
-// 72 us against 146 / 87 / 190 us. With one chunk the scores are not worth computing twice: 16 heads 42 / 30 / 52 us against 44 / 34 / 48 us.
+// More than 16 heads: heads on the rows (mla_decode_heads.cu), which reads a tile 1.4 times for all of them where this file's kernel,
+// with a CTA per 16 heads, read it twice for each: 32 heads, 32 x 2304 / 8 x 4000 / 64 x 1500 tokens 42 / 34 / 56 us against 58 / 38 / 68 us, 128 heads 56 / 36 /
+// 72 us against 146 / 87 / 190 us. Up to 16 heads the scores are not worth computing twice: 16 heads 42 / 30 / 52 us against 44 / 34 / 48 us.
 static bool heads_on_rows(int num_heads) { return num_heads > kMlaHeads; }
 void mfb_mla_decode_set_variant(int v) { g_mla_variant = v == 1 ? 1 : 0; }
 int mfb_mla_decode_get_variant() { return g_mla_variant; }
@@ -425,12 +424,11 @@ int mfb_mla_decode_splits(int B, int num_heads, int max_len) {
   if (g_mla_variant == 1) return mfb_mla_cluster_splits(B, num_heads, max_len);
   if (heads_on_rows(num_heads)) return mfb_mla_decode_heads_splits(B, num_heads, max_len);
   // cost of a choice = waves of CTAs over the 2 x 148 resident CTAs x (tiles per CTA + about one tile of fixed work per CTA)
-  const int chunks = (num_heads + kMlaHeads - 1) / kMlaHeads;
   const int tiles = (max_len + kMlaTile - 1) / kMlaTile;
   int best = 1;
   long long best_cost = -1;
   for (int s = 1; s <= tiles && s <= 32; ++s) {
-    const long long ctas = static_cast<long long>(B) * chunks * s;
+    const long long ctas = static_cast<long long>(B) * s;
     const long long waves = (ctas + 295) / 296;          // two CTAs per SM
     const long long cost = waves * ((tiles + s - 1) / s + 1);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
@@ -483,9 +481,7 @@ int mfb_mla_decode_attention(const void* q, const void* cache, const int* block_
     }
     attr_set = true;
   }
-  const int chunks = (num_heads + kMlaHeads - 1) / kMlaHeads;
-  dim3 grid(splits, chunks, B);
-  mla_decode_kernel<<<grid, kMlaThreads, SMEM, stream>>>(tQ, tC, a);
+  mla_decode_kernel<<<dim3(splits, B), kMlaThreads, SMEM, stream>>>(tQ, tC, a);
   if (cudaGetLastError() != cudaSuccess) { mfb_host::set_error("mla_decode: launch failed"); return 11; }
   mla_combine_kernel<<<dim3(num_heads, B), 128, 0, stream>>>(a.part_o, a.part_ml, reinterpret_cast<__nv_bfloat16*>(out), splits,
                                                               num_heads);

@@ -461,11 +461,6 @@ int mfb_gather_cache2(const void* cache0, const void* cache1, const int* block_t
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
-int mfb_gather_cache(const void* cache, const int* block_tables, const int* cu_lens, void* out, int B, int max_len,
-                     int block_size, int max_blocks, int row_elems, cudaStream_t stream) {
-  return mfb_gather_cache2(cache, nullptr, block_tables, cu_lens, out, nullptr, B, max_len, block_size, max_blocks, row_elems, stream);
-}
-
 // Latents [T, rank] and rotated key parts [T, rope] (rows ld_c / ld_p elements apart) side by side into cache rows of rank + rope.
 int mfb_latent_to_cache(const void* latent, long long ld_c, const void* pe, long long ld_p, void* cache, const int* slot_mapping,
                         long long T, int rank, int rope, cudaStream_t stream) {
