@@ -299,13 +299,16 @@ class MLASelfAttention(nn.Module):
         q_nope, q_pe = q[..., :self.nope], q[..., self.nope:]
         kv_c = self.k_layernorm(kv_c)
         k_pe = k_pe.reshape(T, 1, self.rope_d)
-        if meta.cache is not None and meta.positions is not None and not torch.is_grad_enabled() and Fn.rope_heads_supported(q, self.rope_d):
-            # serving: the last columns of the query heads are rotated where they lie, in the product that _col_nosp has just made (the
-            # key part belongs to the output of linear_qkv, which a hook may have kept)
-            Fn.rope_heads_(q, rotary[0], rotary[1], meta.positions.to(torch.int32), self.rope_d, self.config.rotary_interleaved)
+        if meta.cache is not None and meta.positions is not None and not torch.is_grad_enabled() \
+                and Fn.rope_heads_supported(q, self.rope_d) and Fn.rope_heads_supported(k_pe, self.rope_d):
+            # serving: the last columns of the query heads are rotated where they lie, in the product that _col_nosp has just made; the key
+            # part in a copy, since it belongs to the output of linear_qkv, which a hook may have kept
+            pos, k_pe = meta.positions.to(torch.int32), k_pe.clone(memory_format=torch.contiguous_format)
+            Fn.rope_heads_(q, rotary[0], rotary[1], pos, self.rope_d, self.config.rotary_interleaved)
+            Fn.rope_heads_(k_pe, rotary[0], rotary[1], pos, self.rope_d, self.config.rotary_interleaved)
         else:
             q_pe = self._rope(q_pe, rotary, meta, self.nh)
-        k_pe = self._rope(k_pe, rotary, meta, 1)
+            k_pe = self._rope(k_pe, rotary, meta, 1)
         if meta.cache is not None:
             from ...inference.paged_attention import mla_paged_attention_forward
             ctx = mla_paged_attention_forward(self, q_nope, q_pe, kv_c, k_pe, meta)

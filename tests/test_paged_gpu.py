@@ -437,15 +437,15 @@ def _latent_layer(**over):
     return MLASelfAttention(cfg).eval(), get_rope(cfg, device=DEV)()
 
 
-@pytest.mark.parametrize("prefill", [True, False])
-def test_latent_layer_leaves_its_projections_alone(prefill):
+@pytest.mark.parametrize("prefill,seqs", [(True, 3), (False, 3), (False, 1)])
+def test_latent_layer_leaves_its_projections_alone(prefill, seqs):
     """What a forward hook keeps of a projection's output in serving is that output."""
     from mindformers_b200.inference import paged_attention as pa
     from mindformers_b200.parallel.layers.attention import AttnMeta
     torch.manual_seed(0)
     layer, rotary = _latent_layer()
-    lens = [40, 70, 3]
-    news = [7, 20, 3] if prefill else [1] * 3
+    lens = [40, 70, 3][:seqs]
+    news = ([7, 20, 3] if prefill else [1] * 3)[:seqs]
     tables, blocks = _tables(lens, 16)
     ctx = pa.KVCacheContext(1, blocks, 16, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
     ctx.set_step(is_prefill=prefill, slot_mapping=_slots(tables, 16, lens, news).numpy(), q_seq_lens=news, block_tables=tables.numpy(),
