@@ -79,7 +79,8 @@ class _StepTensor:
 class KVCacheContext:
     """Per-layer paged caches ``[num_blocks, block_size, kv_heads, head_dim]`` (or the 576-wide latent cache of
     multi-latent attention) plus the metadata of the current step: block tables, slot mapping, context lengths, new
-    tokens per sequence."""
+    tokens per sequence. A tensor of the step that is read from here is on the device, for any stream; the attention calls follow a
+    change of it."""
 
     block_tables = _StepTensor()      # int32 [B, max_blocks]
     slot_mapping = _StepTensor()      # int32 [T]

@@ -19,7 +19,8 @@
 //
 // 48 sequences of 3000 - 6000 tokens, 28 / 4 heads of 128: 587 us on the CUDA cores (fp32 products and a five-step shuffle
 // reduction per key and head); 90 us with bf16 operands (830 instructions per group) and one group ahead in registers; 76 us now, 3.0 TB/s:
-// 590 instructions per group fill 44 % of the issue slots, for the rest the 15 warps of an SM wait for their copies.
+// 590 instructions per group fill 44 % of the issue slots, for the rest the 15 warps of an SM wait for their copies; the 1344 CTAs are 2.3 waves,
+// so that an SM is busy 80 % of the time.
 #include <cuda_fp16.h>
 
 #include "mma_sync.cuh"

@@ -126,8 +126,8 @@ constexpr float kTanhRatio[5] = {0.999999926f, -0.33332302f, 0.133100644f, -0.05
 //   kRows     kBf16 for ragged rows.
 // All but kBf16 take keys and values that lie one after the other (key_row) as well as pages, and honour zero_tail.
 // What the split costs and what it replaces: 4 portions of up to 512 rows behind 5000 cached tokens (32 / 8 heads of 128, two layers)
-// take 0.64 ms with kSplitP, 12.0 ms as 32-bit products and a softmax over whole score matrices, both 0.0017 off the 64-bit result
-// (the rounding of the result); 3000 rows of 16 latent heads behind 1200 tokens 0.75 ms against 4.9 ms, projections included.
+// take 0.49 ms with kSplitP, 12.0 ms as 32-bit products and a softmax over whole score matrices, both 0.00166 off the 64-bit result
+// (the rounding of the result); 4 portions of 225 - 900 rows of 16 latent heads behind 1200 tokens 0.50 ms against 4.9 ms, projections included.
 enum Parts { kBf16 = 0, kSplitP = 1, kLatent = 2, kRows = 3 };
 
 // HQ: padded query / key size (64, 128 or 192), HV: padded value size (64 or 128); CAP: scores are soft-capped

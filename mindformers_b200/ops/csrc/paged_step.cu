@@ -1,6 +1,7 @@
 // One call per layer of a decode step: the new rows into the paged cache, attention over it, the merge of its partial results. Three
 // launches; what it saves is host time: which kernel serves the shapes, the number of splits, the scratch they need and the layout of q, k
-// and v were a dozen calls from Python per layer, 34 us per layer with the launches where the kernels of one short sequence take 13 us; 29 us so.
+// and v were a dozen calls from Python per layer, 34 us per layer with the launches where the kernels of one short sequence take 13 us; 30 us so
+// (14 us replayed from a captured graph, where the host has no part).
 #include "common.cuh"
 
 extern "C" {
