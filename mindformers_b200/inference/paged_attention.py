@@ -672,17 +672,17 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
     latent = torch.empty((n, rank + rope_d), dtype=torch.bfloat16, device=dev)
     _gather_rows(cache, [latent], [rows], [None], plan.all_rows, plan.longest)
     out = torch.empty((plan.rows, nh * vd), dtype=torch.bfloat16, device=dev)
-    w = w.view(nh, nope + vd, rank)
     step = max(1, min(nh, _EXPANDED_BYTES // (n * 256 * 8)))
     for h in range(0, nh, step):
         heads = min(step, nh - h)
-        kv = Fn.gemm(latent[:, :rank], w[h:h + heads].view(-1, rank), out_dtype=torch.float32)
+        kv = Fn.gemm(latent[:, :rank], w[h * 256:(h + heads) * 256], out_dtype=torch.float32)
         parts = torch.empty((2,) + kv.shape, dtype=torch.bfloat16, device=dev)
-        rc = lib.mfb_split_f32(kv.data_ptr(), parts[0].data_ptr(), parts[1].data_ptr(), kv.numel(), _lib.stream_ptr())
+        hi, lo = parts.data_ptr(), parts.data_ptr() + 2 * kv.numel()
+        rc = lib.mfb_split_f32(kv.data_ptr(), hi, lo, kv.numel(), _lib.stream_ptr())
         _lib.check(rc, "mfb_split_f32")
         rc = lib.mfb_latent_prefill_tc(
             q_nope.data_ptr() + 2 * h * q_nope.stride(1), q_nope.stride(0), q_nope.stride(1), q_pe.data_ptr() + 2 * h * q_pe.stride(1),
-            q_pe.stride(0), q_pe.stride(1), parts[0].data_ptr(), parts[1].data_ptr(), latent.data_ptr() + 2 * rank, rank + rope_d, n,
+            q_pe.stride(0), q_pe.stride(1), hi, lo, latent.data_ptr() + 2 * rank, rank + rope_d, n,
             plan.all_rows.data_ptr(), plan.all[0].data_ptr(), plan.all[1], out.data_ptr() + 2 * h * vd, out.stride(0), T, heads,
             float(attn.scale), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
         _lib.check(rc, "mfb_latent_prefill_tc")
