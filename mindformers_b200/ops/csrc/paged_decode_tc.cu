@@ -452,9 +452,10 @@ int mfb_paged_decode_attention_tc_q(const void* q, long long ld_q, long long ld_
   int rc;
   const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const uint64_t slots = (uint64_t)num_blocks * block_size, kp = (uint64_t)Hkv * D, vp = (uint64_t)Hkv * DV;
-  if ((rc = pdt::make_q_map(&tQ, q, rows, Hq, D, ld_q, ld_head))) return 20 + rc;
+  // (make_tmap_2d comes first: it sees to it that a new thread has a context)
   if ((rc = mfb_host::make_tmap_2d(&tK, key_cache, 2, BF, slots, kp, kp, block_size, 64))) return 30 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tV, value_cache, 2, BF, slots, vp, vp, block_size, 64))) return 40 + rc;
+  if ((rc = pdt::make_q_map(&tQ, q, rows, Hq, D, ld_q, ld_head))) return 20 + rc;
   pdt::Args a;
   a.block_tables = block_tables; a.context_lens = context_lens; a.cu_q = cu_q; a.max_blocks = max_blocks;
   a.block_size = block_size; a.num_q_heads = Hq; a.num_kv_heads = Hkv; a.group = Hq / Hkv; a.splits = splits;

@@ -909,7 +909,7 @@ int launch_values(const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMa
 }
 
 // three-dimensional map of q [T, Hq, D] with rows ld and heads ld_head elements apart: box of 128 tokens x 1 head x 64 columns;
-// columns past D read as zero
+// columns past D read as zero. To be made after a map of make_tmap_2d, which sees to it that a new thread has a context.
 int make_q_map(CUtensorMap* out, const void* q, uint64_t T, uint64_t Hq, uint64_t D, uint64_t ld, uint64_t ld_head) {
   mfb_host::EncodeTiledFn enc = mfb_host::get_encode_tiled();
   if (!enc) { mfb_host::set_error("cuTensorMapEncodeTiled entry point not available"); return 1; }
@@ -1091,11 +1091,11 @@ int mfb_latent_prefill_tc(const void* q_nope, long long ld_q, long long hd_q, co
   CUtensorMap tQ, tQ2, tK, tV, tK2;
   int rc;
   const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  if ((rc = ppt::make_q_map(&tQ, q_nope, T, H, 128, ld_q, hd_q))) return 20 + rc;
-  if ((rc = ppt::make_q_map(&tQ2, q_pe, T, H, 64, ld_qp, hd_qp))) return 25 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tK, kv_hi, 2, BF, key_rows, (uint64_t)H * 256, (uint64_t)H * 256, ppt::kTile, 64))) return 30 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tV, kv_lo, 2, BF, key_rows, (uint64_t)H * 256, (uint64_t)H * 256, ppt::kTile, 64))) return 40 + rc;
   if ((rc = mfb_host::make_tmap_2d(&tK2, pe, 2, BF, key_rows, 64, (uint64_t)ld_pe, ppt::kTile, 64))) return 50 + rc;
+  if ((rc = ppt::make_q_map(&tQ, q_nope, T, H, 128, ld_q, hd_q))) return 20 + rc;
+  if ((rc = ppt::make_q_map(&tQ2, q_pe, T, H, 64, ld_qp, hd_qp))) return 25 + rc;
   ppt::Args a = {};
   a.work = reinterpret_cast<const int4*>(work); a.vheads = 1; a.n_items = n_work * H;
   a.out = reinterpret_cast<__nv_bfloat16*>(out);

@@ -628,3 +628,27 @@ def test_prefill_with_gradients():
     with torch.no_grad():
         plain = call(x)
     assert (plain.double() - ref.detach()).norm() / ref.detach().norm() < 4e-3
+
+
+def test_decode_kernel_first_in_a_thread():
+    """A thread whose first work on the GPU is the decode kernel."""
+    import threading
+    from mindformers_b200.ops import _lib
+    torch.manual_seed(0)
+    lib = _lib.get_lib()
+    q, kc, vc = (torch.randn(*s, device=DEV).to(torch.bfloat16) for s in ((2, 4, 128), (6, 16, 2, 128), (6, 16, 2, 128)))
+    tables, lens = (torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([[0, 1, 2], [3, 4, 5]], [40, 17]))
+    splits = lib.mfb_paged_decode_tc_splits(2, 2, 48)
+    scratch = torch.empty(lib.mfb_paged_decode_scratch_bytes(2, 4, 128, splits) // 4 + 4, device=DEV)
+    outs = [torch.zeros(2, 4, 128, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    args = [(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), tables.data_ptr(), lens.data_ptr(), out.data_ptr(), scratch.data_ptr(), splits, 2, 4,
+             2, 6, 16, 3, 0.09, _lib.status_word(DEV).data_ptr(), 0) for out in outs]
+    torch.cuda.synchronize()
+    codes = [lib.mfb_paged_decode_attention_tc(*args[0])]
+    torch.cuda.synchronize()
+    other = threading.Thread(target=lambda: codes.append(lib.mfb_paged_decode_attention_tc(*args[1])))
+    other.start()
+    other.join()
+    torch.cuda.synchronize()
+    assert codes == [0, 0], lib.mfb_last_error()
+    assert outs[0].any() and torch.equal(outs[0], outs[1])
