@@ -1057,6 +1057,7 @@ def _split3(x: torch.Tensor, across: bool, parts: int) -> torch.Tensor:
 # Up to this many rows the gate runs on the CUDA cores, weight by weight (``gate_rows_kernel``); more are a library product in fp32.
 _GATE_ROWS = 192
 _GATE_CHUNK = 256            # rows that a tensor-core sum of the weight's gradient spans
+_GATE_BYTES = 512 << 20      # of such sums at a time; more rows take turns
 
 
 class _GateFn(torch.autograd.Function):
@@ -1091,15 +1092,21 @@ class _GateFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             if 3 * E % 128:                                           # not whole tiles
                 return dx, torch.matmul(dy.t(), x.float())
-            lib, groups = _lib.get_lib(), -(-T // _GATE_CHUNK)
-            parts = torch.empty((groups * 3 * E, H), dtype=torch.float32, device=x.device)
-            rc = lib.mfb_gemm_bf16(d.data_ptr(), x.data_ptr(), parts.data_ptr(), 3 * E, H, _GATE_CHUNK, d.stride(0), x.stride(0), H, 1, 1, 1, 2,
-                                   groups, 0, 0, 0, T, _lib.status_word(x.device).data_ptr(), 0, _lib.stream_ptr())
-            _lib.check(rc, "mfb_gemm_bf16[gate]")
-            dw = torch.empty((E, H), dtype=torch.float32, device=x.device)
-            rc = lib.mfb_sum3(parts.data_ptr(), dw.data_ptr(), E, H, H, E * H, groups, 3 * E * H, _lib.stream_ptr())
-            _lib.check(rc, "mfb_sum3")
-            _lib.count_launch(2)
+            lib = _lib.get_lib()
+            rows = max(1, _GATE_BYTES // (12 * E * H)) * _GATE_CHUNK
+            parts = torch.empty((-(-min(T, rows) // _GATE_CHUNK) * 3 * E, H), dtype=torch.float32, device=x.device)
+            for t in range(0, T, rows):
+                n = min(rows, T - t)
+                groups = -(-n // _GATE_CHUNK)
+                rc = lib.mfb_gemm_bf16(d.data_ptr() + 2 * t * d.stride(0), x.data_ptr() + 2 * t * x.stride(0), parts.data_ptr(), 3 * E, H,
+                                       _GATE_CHUNK, d.stride(0), x.stride(0), H, 1, 1, 1, 2, groups, 0, 0, 0, n,
+                                       _lib.status_word(x.device).data_ptr(), 0, _lib.stream_ptr())
+                _lib.check(rc, "mfb_gemm_bf16[gate]")
+                part = torch.empty((E, H), dtype=torch.float32, device=x.device)
+                rc = lib.mfb_sum3(parts.data_ptr(), part.data_ptr(), E, H, H, E * H, groups, 3 * E * H, _lib.stream_ptr())
+                _lib.check(rc, "mfb_sum3")
+                _lib.count_launch(2)
+                dw = part if dw is None else dw.add_(part)
         return dx, dw
 
 

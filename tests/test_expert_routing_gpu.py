@@ -152,3 +152,25 @@ def test_gate_on_views():
     plain = torch.nn.functional.linear(row.float(), w)
     for a, b in zip((logits, *grads), (plain, *torch.autograd.grad(plain, (row, w), dy))):
         assert (a.float() - b.float()).norm() / b.float().norm() < 8e-3          # bf16 gradients, at most 2^-8 on either side
+
+
+def test_gate_gradient_in_turns(monkeypatch):
+    """The sums of blocks of rows that the weight's gradient is made of stay within their bytes, whatever the number of rows."""
+    from mindformers_b200.ops import functional as Fn
+    torch.manual_seed(0)
+    T, E, H = 5000, 128, 512
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, H, device=DEV) * 0.02).requires_grad_()
+    dy = torch.randn(T, E, device=DEV)
+    want = dy.double().t() @ x.double()
+    taken = []
+    for limit in (Fn._GATE_BYTES, 3 * 12 * E * H):                        # three blocks of 256 rows at a time
+        monkeypatch.setattr(Fn, "_GATE_BYTES", limit, raising=False)
+        y = Fn.gate_logits(x, w)
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        got = torch.autograd.grad(y, w, dy)[0]
+        taken.append(torch.cuda.max_memory_allocated() - before)
+        assert float((got.double() - want).norm() / want.norm()) < 1.4e-6         # as in test_gate
+    assert taken[1] < taken[0] - 16 * 12 * E * H
+    assert Fn._lib.read_status() == 0
