@@ -330,9 +330,9 @@ _PERSISTENT_UP_TO = 8.0
 
 class _PrefillPlan:
     """What the prefill kernels need to know about a step: per query tile ``(sequence, first row of q, rows, position of the first
-    row)``, longest first, for the sequences whose keys are all new (``fresh``) and for those with cached ones (``past``), or for both
-    (``all``, caches of latents); the first row of every sequence in q (``cu``), and in a gathered copy of the cached rows that the sequences
-    with history see (``past_rows``) or all that have new rows (``all_rows``). ``ok`` False: a step that
+    row)``, longest first, for the sequences whose keys are all new (``fresh``) and for those with cached ones (``past``; of a cache of
+    latents, all that have new rows); the first row of every sequence in q (``cu``), and in a gathered copy of the cached rows that the
+    sequences of ``past`` see (``past_rows``). ``ok`` False: a step that
     these kernels do not take (a sequence longer than its block table or without one, rows that are not there, tables of another form)."""
 
     def __init__(self, cache, rows: int, lens: list, latent: bool):
@@ -357,14 +357,10 @@ class _PrefillPlan:
         at = len(flat)
         dev, = _to_device([np.asarray(flat + list(cu) + first, np.int32)], tables.device)
         (a, n, p), (b, m, s) = spans
-        works = (dev[a:a + 4 * n], n, p), (dev[b:b + 4 * m], m, s)
-        cu_dev, rows_dev = dev[at:at + B + 1], dev[at + B + 1:]
-        if latent:
-            self.all, self.all_rows, self.n_all_rows, self.forms = works[1], rows_dev, first[-1], {}
-            self.new_and_seen = [(n, m) for n, m in zip(news, lens) if n]
-        else:
-            (self.fresh, self.past), self.cu, self.past_rows, self.n_past_rows = works, cu_dev, rows_dev, first[-1]
-            self.past_host, self.groups = (seeing, first), {}
+        self.fresh, self.past = (dev[a:a + 4 * n], n, p), (dev[b:b + 4 * m], m, s)
+        self.cu, self.past_rows, self.n_past_rows = dev[at:at + B + 1], dev[at + B + 1:], first[-1]
+        self.past_host, self.groups, self.forms = (seeing, first), {}, {}
+        self.new_and_seen = [(n, m) for n, m in zip(news, lens) if n] if latent else None
 
     def expands(self, heads: int) -> bool:
         """Whether multi-latent attention of ``heads`` heads expands the cached latents (one product over all rows that the step sees, whatever
@@ -373,7 +369,7 @@ class _PrefillPlan:
         of 8000 rows, 1 / 4 / 16 new ones each 29.8 / 30.1 / 29.9 and 9.5 / 15.8 / 35.2 ms; 1 sequence 0.97 / 0.99 / 0.96 and 0.41 / 0.56 / 1.19 ms;
         32 of 2300 rows 8.5 / 8.5 / 8.8 and 8.5 / 9.1 / 14.2 ms; 16 heads, 4 of 2300 rows, 1 / 200 new ones 0.26 / 0.28 and 1.15 / 2.5 ms."""
         if heads not in self.forms:
-            expanded = 110 + 0.9e-3 * self.n_all_rows * heads
+            expanded = 110 + 0.9e-3 * self.n_past_rows * heads
             absorbed = sum(max(265, 90 + m * (0.005 + 0.0002 * heads) + 0.056e-3 * n * m * heads) for n, m in self.new_and_seen)
             self.forms[heads] = expanded <= absorbed
         return self.forms[heads]
@@ -663,30 +659,32 @@ def _latent_prefill(attn, q_nope, q_pe, cache, layer: int):
             and rank % 8 == 0 and T and w.is_contiguous() and rows.is_contiguous() and Fn.get_gemm_backend() == "tcgen05") or _needs_graph(q_nope, q_pe, w):
         return None
     plan = _prefill_plan(cache, T, latent=True)
-    n = plan.n_all_rows if plan.ok else 0
-    if not plan.ok or n >= 1 << 31 or plan.longest * (rank + rope_d) >= 1 << 34 or not plan.expands(nh):
+    if not plan.ok or plan.n_past_rows >= 1 << 31 or plan.longest * (rank + rope_d) >= 1 << 34 or not plan.expands(nh):
         return None
     q_pe = q_pe.reshape(T, nh, rope_d)
     q_nope, q_pe = _strided(q_nope), _strided(q_pe)
     lib, dev = _lib.get_lib(), q_nope.device
-    latent = torch.empty((n, rank + rope_d), dtype=torch.bfloat16, device=dev)
-    _gather_rows(cache, [latent], [rows], [None], plan.all_rows, plan.longest)
     out = torch.empty((plan.rows, nh * vd), dtype=torch.bfloat16, device=dev)
-    step = max(1, min(nh, _EXPANDED_BYTES // (n * 256 * 8)))
-    for h in range(0, nh, step):
-        heads = min(step, nh - h)
-        kv = Fn.gemm(latent[:, :rank], w[h * 256:(h + heads) * 256], out_dtype=torch.float32)
-        parts = torch.empty((2,) + kv.shape, dtype=torch.bfloat16, device=dev)
-        hi, lo = parts.data_ptr(), parts.data_ptr() + 2 * kv.numel()
-        rc = lib.mfb_split_f32(kv.data_ptr(), hi, lo, kv.numel(), _lib.stream_ptr())
-        _lib.check(rc, "mfb_split_f32")
-        rc = lib.mfb_latent_prefill_tc(
-            q_nope.data_ptr() + 2 * h * q_nope.stride(1), q_nope.stride(0), q_nope.stride(1), q_pe.data_ptr() + 2 * h * q_pe.stride(1),
-            q_pe.stride(0), q_pe.stride(1), hi, lo, latent.data_ptr() + 2 * rank, rank + rope_d, n,
-            plan.all_rows.data_ptr(), plan.all[0].data_ptr(), plan.all[1], out.data_ptr() + 2 * h * vd, out.stride(0), T, heads,
-            float(attn.scale), _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
-        _lib.check(rc, "mfb_latent_prefill_tc")
-        _lib.count_launch(2)
+    groups = plan.copied(max(1, _COPIED_BYTES // (2 * (rank + rope_d))))
+    latent = torch.empty((max(g[2] for g in groups), rank + rope_d), dtype=torch.bfloat16, device=dev)
+    for work, first, n in groups:
+        _gather_rows(cache, [latent], [rows], [None], first, plan.longest)
+        step = max(1, min(nh, _EXPANDED_BYTES // (n * 256 * 8)))
+        for h in range(0, nh, step):
+            heads = min(step, nh - h)
+            kv = Fn.gemm(latent[:n, :rank], w[h * 256:(h + heads) * 256], out_dtype=torch.float32)
+            parts = torch.empty((2,) + kv.shape, dtype=torch.bfloat16, device=dev)
+            hi, lo = parts.data_ptr(), parts.data_ptr() + 2 * kv.numel()
+            rc = lib.mfb_split_f32(kv.data_ptr(), hi, lo, kv.numel(), _lib.stream_ptr())
+            _lib.check(rc, "mfb_split_f32")
+            rc = lib.mfb_latent_prefill_tc(
+                q_nope.data_ptr() + 2 * h * q_nope.stride(1), q_nope.stride(0), q_nope.stride(1), q_pe.data_ptr() + 2 * h * q_pe.stride(1),
+                q_pe.stride(0), q_pe.stride(1), hi, lo, latent.data_ptr() + 2 * rank, rank + rope_d, n, first.data_ptr(),
+                work[0].data_ptr(), work[1], out.data_ptr() + 2 * h * vd, out.stride(0), T, heads, float(attn.scale),
+                _lib.status_word(dev).data_ptr(), _lib.stream_ptr())
+            _lib.check(rc, "mfb_latent_prefill_tc")
+            _lib.count_launch(2)
+            del kv, parts                # before the next ones are allocated
     return out
 
 

@@ -652,3 +652,40 @@ def test_decode_kernel_first_in_a_thread():
     torch.cuda.synchronize()
     assert codes == [0, 0], lib.mfb_last_error()
     assert outs[0].any() and torch.equal(outs[0], outs[1])
+
+
+def test_latents_copied_in_turns(monkeypatch):
+    """A multi-latent step whose sequences see more cached rows than may be copied out at a time."""
+    from mindformers_b200.inference import paged_attention as pa
+    torch.manual_seed(0)
+    heads, block, lens, news = 2, 64, [2900, 2700, 64, 3000, 20], [700, 5, 64, 130, 0]
+    tables, blocks = _tables(lens, block)
+    ctx = pa.KVCacheContext(1, blocks, block, 1, 0, torch.bfloat16, DEV, mla_latent_dim=576)
+    ctx.key_cache[0].normal_()
+    w = (torch.randn(heads * 256, 512, device=DEV) * 512 ** -0.5).to(torch.bfloat16)
+    attn = types.SimpleNamespace(nh=heads, nope=128, rope_d=64, vd=128, kv_rank=512, layer_number=1, scale=192 ** -0.5,
+                                 linear_kvb=types.SimpleNamespace(weight=w))
+    T = sum(news)
+    q = torch.randn(T, heads, 192, device=DEV).to(torch.bfloat16)
+    new = torch.randn(T, 576, device=DEV).to(torch.bfloat16)
+    taken = []
+    for budget in (pa._COPIED_BYTES, 1):
+        monkeypatch.setattr(pa, "_COPIED_BYTES", budget)
+        _set(ctx, tables, block, lens, news)
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        with torch.no_grad():
+            got = pa.mla_paged_attention_forward(attn, q[..., :128], q[..., 128:].clone(), new[:, :512], new[:, 512:],
+                                                 types.SimpleNamespace(cache=ctx))
+        taken.append(torch.cuda.max_memory_allocated() - before)
+        at = 0
+        for b, (n, m) in enumerate(zip(news, lens)):
+            rows, at = slice(at, at + n), at + n
+            if not n:
+                continue
+            lt = _cached(ctx.key_cache[0][:, :, 0], tables, b, m, block).double()
+            kv = (lt[:, :512] @ w.double().t()).view(m, heads, 256)
+            want = _attend(q[rows], torch.cat((kv[..., :128], lt[:, None, 512:].expand(m, heads, 64)), -1), kv[..., 128:], attn.scale)
+            assert (got[rows].double() - want).norm() / want.norm() < 2e-3           # rounding of the result alone
+    row = 576 * 2 + heads * 256 * 8
+    assert taken[1] < taken[0] - 5000 * row                 # at most 3000 rows at a time instead of 8664
