@@ -109,8 +109,9 @@ __device__ __forceinline__ Tile get_tile(const GemmArgs& g, int tile, int mb_tot
 // and stored, and those past ROWS hold whatever lies behind them in shared memory (rows of a product do not touch each other). An
 // expert's 128-row block is 128 / ROWS tiles, of which those without a row in use are skipped, so weights are read once per ROWS rows in
 // use. The bytes that count are then the weights'; with whole blocks a quarter as much again went for padding rows in and out (24 tokens, 8
-// of 128 experts each, 109 of them hit, 2048 x 1536 and 768 x 2048: both products 212 us for 1.03 GB of weights, 204 us so, 0.77 of the rate of a
-// copy; tiles of 128 columns, whose boxes are 256 contiguous bytes of a weight row instead of 512, give that back).
+// of 128 experts each, 109 of them hit, 2048 x 1536 and 768 x 2048: both products with their launches 212 us for 1.03 GB of weights, 204 us so; the
+// kernels alone 186 us, 0.85 of the rate of a copy; tiles of 128 columns, whose boxes are 256 contiguous bytes of a weight row instead of 512,
+// give that back).
 template <int BN, int STAGES, bool A_MN, bool B_MN, int OUT_MODE, int ROWS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
