@@ -165,7 +165,8 @@ class KVCacheContext:
         if copied is not None:
             rc = _lib.get_lib().mfb_event_done(copied[0].cuda_event, 1)
             _lib.check(rc, "mfb_event_done")
-            self._copied = None
+            if self._copied is copied:           # and not the next step's, of another thread
+                self._copied = None
 
     def _in_order(self):
         """Before kernels on the current stream read the step's tensors: on the stream that copies them there is nothing to wait for."""
