@@ -148,7 +148,7 @@ class KVCacheContext:
         self.carry = torch.zeros((num_layers, slots, carry_width), dtype=torch.float32, device=device) if carry_width else None
         self.carry_before = torch.zeros_like(self.carry) if carry_width else None
         self.is_prefill = True
-        self._copied = None           # (event behind the copy of the step's tensors, its stream) while it may be under way
+        self._copied = None           # (event behind the copy of the step's tensors, its stream, asked before) while it may be under way
         self._event = None            # (the event, its device)
         self.block_tables = self.slot_mapping = self.context_lens = self.q_seq_lens = self.last_token_index = None
         self.cu_q = None              # python list of cumulative q lengths
@@ -175,8 +175,10 @@ class KVCacheContext:
             return
         if copied[1] != _lib.stream_ptr() or torch.cuda.is_current_stream_capturing():
             self._await_copy()
-        elif not self.is_prefill and _lib.get_lib().mfb_event_done(copied[0].cuda_event, 0) == 0:
-            self._copied = None              # the short layers of a decode step need not ask again
+        elif not self.is_prefill:
+            # the short layers of a decode step need not ask again once it is done; the first one would mostly find it under way
+            done = copied[2] and _lib.get_lib().mfb_event_done(copied[0].cuda_event, 0) == 0
+            self._copied = None if done else copied[:2] + (True,)
 
     def _mark_copy(self, index: Optional[int]):
         """Behind the copy of the step's tensors on the current stream of a device."""
@@ -188,7 +190,7 @@ class KVCacheContext:
             self._event[0].record(torch.cuda.current_stream(index))
         else:                                # (a stream object costs more host time than this)
             _lib.check(_lib.get_lib().mfb_event_record(self._event[0].cuda_event, stream), "mfb_event_record")
-        self._copied = (self._event[0], stream)
+        self._copied = (self._event[0], stream, False)
 
     def __getstate__(self):
         self._await_copy()
